@@ -10,6 +10,7 @@
 #include <cctype>
 #include <atomic>
 #include <mutex>
+#include <set>
 #include <string>
 #include <vector>
 
@@ -246,6 +247,19 @@ static bool flow_thresholds(double k, float thr[256]) {
     return true;
 }
 
+// "AIR, or not SOLID and less dense" as an order: 0 for AIR, 255 for SOLID, the others
+// 1 + the number of different densities below theirs (at most 254 of them, as the table
+// always holds an AIR and a SOLID material). A NaN compares with nothing: nothing sinks
+// into it (255), and as sand it sinks into AIR alone (the colour pass's cw_sink).
+uint32_t density_rank(const HostMat &m) {
+    if (m.type == T_AIR) return 0u;
+    if (m.type == T_SOLID || std::isnan(m.density)) return 255u;
+    std::set<float> below;
+    for (const HostMat &o : g_mats)
+        if (o.type != T_AIR && o.type != T_SOLID && o.density < m.density) below.insert(o.density);
+    return 1u + (uint32_t)below.size();
+}
+
 void build_table(MatTable &t) {
     memset(&t, 0, sizeof(t));
     t.n = (int)g_mats.size();
@@ -266,7 +280,8 @@ void build_table(MatTable &t) {
         int slip = std::min(std::max(m.slip, 0), 255);
         t.a[i] = (uint32_t)m.type | ((uint32_t)iters << 8) | ((uint32_t)slip << 16) |
                  ((uint32_t)max_stability(m.slip) << 24);
-        t.density[i] = m.density;
+        t.word[i] = (uint32_t)i | ((uint32_t)m.type << MW_TYPE_SHIFT) | (i == t.id_fire ? MW_FIRE : 0u) |
+                    (m.n_react > 0 ? MW_REACT : 0u) | (density_rank(m) << MW_RANK_SHIFT);
         t.f_base[i] = m.f_base;
         t.f_pack[i] = (uint32_t)(m.f_shift & 0xFF) | ((uint32_t)(m.f_lo & 0xFFF) << 8) | ((uint32_t)(m.f_mod & 0xFFF) << 20);
         t.f_scalar[i] = m.f_scalar;

@@ -18,7 +18,17 @@ constexpr int CP_THREADS = 1024;  // colour-pass CTA: >= the largest sweep-A sub
 constexpr uint8_t MOVED = 0x80;
 constexpr uint8_t VISITED = 0x40;  // shared-memory copy only; never stored to HBM
 constexpr uint8_t SETTLE_MASK = 0x3F;
-constexpr uint16_t DIRTY = 0x8000;  // shared-memory copy only: cell must be written back
+
+// MatTable::word: what a cell of the colour pass's tile takes from its material. Bits
+// 0-7 the id, 16-18 the type, 21 FIRE, 22 has reactions, 24-31 the density rank
+// (0 AIR, 255 SOLID or no comparable density, the others 1.. by increasing density,
+// equal densities alike); the colour pass keeps its own marks in the other bits
+constexpr int MW_TYPE_SHIFT = 16;
+constexpr uint32_t MW_TYPE = 7u << MW_TYPE_SHIFT;
+constexpr uint32_t MW_FIRE = 1u << 21;
+constexpr uint32_t MW_REACT = 1u << 22;
+constexpr int MW_RANK_SHIFT = 24;
+constexpr uint32_t MW_RANK = 0xFFu << MW_RANK_SHIFT;
 
 // FLUID_* (source/engine/core/const.h:23-34) in Q16.16
 constexpr int32_t Q_MAXV = 32768;
@@ -69,13 +79,13 @@ __host__ __device__ __forceinline__ uint32_t draw_k(uint32_t ck, uint32_t k) {
 
 // --------------------------------------------------------- material table
 // Packed per-material word A: type | iterations << 8 | slip << 16 | max_stab << 24,
-// word B: density bits. Factory: base colour, (shift | lo << 8 | mod << 20), scalar.
+// word: the cell word of the colour pass (MW_*). Factory: base colour, (shift | lo << 8 | mod << 20), scalar.
 struct MatTable {
     int n;
     int id_air, id_solid, id_fire, id_water, id_lava, id_steam, id_obsidian;
     int has_inter;
     uint32_t a[MAXMAT];
-    float density[MAXMAT];
+    uint32_t word[MAXMAT];
     uint32_t f_base[MAXMAT];
     uint32_t f_pack[MAXMAT];
     int32_t f_scalar[MAXMAT];

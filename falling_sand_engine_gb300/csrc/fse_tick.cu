@@ -25,6 +25,8 @@
 // no trace of that plane. fse_tick_temp.cu compiles the TEMP instantiation as a
 // translation unit of its own (including this file with FSE_TICK_TEMP_TU), so the
 // two build in parallel.
+#include <algorithm>
+
 #include "fse_internal.cuh"
 
 // Optional per-phase cycle counters of the colour pass (build with
@@ -76,16 +78,48 @@ __device__ __forceinline__ void divmod_small(int e, int n, float rn, int &q, int
     r = e - q * n;
 }
 
+// ------------------------------------------------------------- cell words
+// A cell of the shared-memory tile is one 32-bit word beside its scalar and colour
+// planes: the material id, the flags byte, what the rules ask of the material (its
+// type, whether it is updated in this iteration, whether it burns or reacts) and its
+// density rank. One load then answers every question a rule asks of a neighbour;
+// with id and flags in planes of their own and the material's type and density looked
+// up in tables, each question was a chain of two or three dependent shared loads, and
+// those chains set the length of a sub-phase.
+//
+// Ranks order the materials by density: AIR 0, SOLID 255 and the others by increasing
+// density from 1, equal densities equal ranks (MatTable::word, built on the host), so
+// that "AIR, or not SOLID and less dense" is one unsigned comparison (can_sink).
+constexpr uint32_t CW_ID = 0xFFu;
+constexpr uint32_t CW_FLAGS = 0xFF00u;  // the flags byte: MOVED, VISITED, settle count
+constexpr uint32_t CW_SETTLE = (uint32_t)SETTLE_MASK << 8;
+constexpr uint32_t CW_VIS = (uint32_t)VISITED << 8;
+constexpr uint32_t CW_MOVED = (uint32_t)MOVED << 8;
+constexpr uint32_t CW_TYPE = MW_TYPE;
+constexpr uint32_t CW_LIVE = 1u << 19;   // the material's iterations exceed this pass's
+constexpr uint32_t CW_DIRTY = 1u << 20;  // the cell must be written back
+constexpr uint32_t CW_FIRE = MW_FIRE;
+constexpr uint32_t CW_REACT = MW_REACT;
+constexpr uint32_t CW_RANK = MW_RANK;
+// the bits a cell takes from its material
+constexpr uint32_t CW_MAT = ~(CW_FLAGS | CW_DIRTY);
+
+__device__ __forceinline__ int cw_id(uint32_t w) { return (int)(w & CW_ID); }
+__device__ __forceinline__ bool cw_is(uint32_t w, int type) { return (w & CW_TYPE) == (uint32_t)type << MW_TYPE_SHIFT; }
+__device__ __forceinline__ bool cw_air(uint32_t w) { return (w & CW_TYPE) == 0; }
+__device__ __forceinline__ bool cw_same(uint32_t a, uint32_t b) { return ((a ^ b) & CW_ID) == 0; }
+// cells that sand `w` sinks into have words below this: AIR, or not SOLID and less
+// dense (a SAND of rank 255 has no density to compare, a NaN: only AIR is below it)
+__device__ __forceinline__ uint32_t cw_sink(uint32_t w) { return w >= CW_RANK ? 1u << 24 : w & CW_RANK; }
+
 struct Cell {
-    uint16_t id;
-    uint8_t fl;
+    uint32_t w;  // its word; the VISITED and DIRTY bits mean nothing here
     int32_t sc;
     uint32_t col;
     int32_t df;
 };
 
 struct SpawnEv {
-    int n;     // particles to emit (0 = none)
     int kind;  // 1 sand, 2 soup, 3 fire
     int x, y;
     uint16_t id;
@@ -98,37 +132,41 @@ struct SpawnEv {
 };
 
 // ------------------------------------------------------- shared-memory tile
-// Region: x in [cx - HALO, cx + C + HALO), full state for y in
-// [cy - HALO, cy + C + HALO), material ids only down to y < cy + C + 10 (the
-// deepest read, the friction pillar of world.cpp:1619-1627).
+// Region: x in [cx - 2, cx + C + HALO), full state for y in [cy - 2, cy + C + HALO),
+// words only down to y < cy + C + 10 (the deepest read, the friction pillar of
+// world.cpp:1619-1627).
 //
 // Every access of the rules stays inside the tile: relative to the active cell
-// they reach x +- 2 (fire), y - 2 .. y + 2 in the full planes, ids down to y + 4
-// (sand and liquid free fall), and the interaction boxes, whose |offset| + radius
-// <= 5 is enforced at registration and which run with HALO = 5; the sweep-B pillar
-// reads ids down to cy + C + 9. So the tile needs no bounds checks. EDGE selects
-// the world bounds policy of world.cpp:999-1008 (outside reads GENERIC_SOLID,
-// outside writes dropped); it is needed only when the tile crosses the world edge.
+// they reach x +- 2 (fire), y - 2 .. y + 2 in the full planes, words down to y + 4
+// (sand and liquid free fall), and the interaction boxes, which lie right of and
+// below the cell (a box with a negative corner is not visited) with offset + radius
+// <= 5 enforced at registration and run with HALO = 5; the sweep-B pillar reads
+// words down to cy + C + 9. So the tile needs no bounds checks. Where the tile
+// crosses the world edge it holds GENERIC_SOLID, which is what world.cpp:999-1002
+// reads there; the only writes that can reach such cells are those of fire and
+// interactions, which check the world bounds themselves (world.cpp:1003-1008 drops
+// them).
+constexpr int HALO_LO = 2;  // cells staged left of and above the chunk
+
 struct TileData {
-    uint16_t *s_id;
-    uint8_t *s_fl;
+    uint32_t *s_w;
     int32_t *s_sc;
     uint32_t *s_col;
+    const uint32_t *mw;  // material id -> word of a new cell (flags clear)
     const uint32_t *ma;  // material word A in shared memory
-    const float *md;     // density in shared memory
     int32_t *df;         // HBM diff plane
     int16_t *tp;         // HBM temperature plane of SOUP cells (NULL: not kept)
     int x0, y0, RW, RHF, RHI;
     int W, H;
-    int id_solid, id_air;
+    int id_air;
     // sweep-B pillar snapshot: AIR bits of columns ax0.., rows ay0.., 5 words per column
     const uint32_t *s_air;
     int ax0, ay0, aw;
     // a chunk split over a CTA pair: the partner's copy of the planes (shared::cluster
-    // addresses) and the world row of its first tile row; both copies have RW, RHF
-    // and RHI of this one
-    uint32_t p_id, p_fl, p_sc, p_col;
-    int py0;
+    // addresses); cell i of this tile is cell i + pd of the partner's, both of RW
+    // columns and RHF, RHI rows
+    uint32_t p_w, p_sc, p_col;
+    int pd;
 };
 
 // --------------------------------------------------- CTA-pair (cluster) helpers
@@ -138,12 +176,6 @@ __device__ __forceinline__ uint32_t mapa_rank(uint32_t a, uint32_t r) {
     uint32_t o;
     asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(o) : "r"(a), "r"(r));
     return o;
-}
-__device__ __forceinline__ void st_cluster_u8(uint32_t a, uint8_t v) {
-    asm volatile("st.shared::cluster.u8 [%0], %1;" ::"r"(a), "h"((unsigned short)v) : "memory");
-}
-__device__ __forceinline__ void st_cluster_u16(uint32_t a, uint16_t v) {
-    asm volatile("st.shared::cluster.u16 [%0], %1;" ::"r"(a), "h"(v) : "memory");
 }
 __device__ __forceinline__ void st_cluster_u32(uint32_t a, uint32_t v) {
     asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(a), "r"(v) : "memory");
@@ -214,50 +246,59 @@ constexpr unsigned long long FUSED_WAIT_NS = 2000000000ull;  // a dependency wai
 // holds is made in both copies (reads are always local), so both copies of the
 // shared rows stay equal; at the end of a sub-phase the cluster barrier makes them
 // visible.
-template <bool EDGE, bool TEMP, bool LIVE = false, bool F32 = false, bool PAIR = false>
+//
+// Cells are named by their tile index i (neighbours i +- 1, i +- RW) and, for the
+// planes in HBM, their world index g (neighbours g +- 1, g +- W).
+template <bool TEMP, bool LIVE = false, bool F32 = false, bool PAIR = false>
 struct Tile : TileData {
     static constexpr bool kTemp = TEMP;
     static constexpr bool kF32 = F32;
     __device__ __forceinline__ explicit Tile(const TileData &d) : TileData(d) {}
 
-    // the partner's index of cell (x, y): -1 outside its tile; *full: a full-state row
-    __device__ __forceinline__ int pli(int x, int y, bool *full) const {
-        const int r = y - py0;
-        if (r < 0 || r >= RHI) return -1;
-        *full = r < RHF;
-        return r * RW + (x - x0);
+    __device__ __forceinline__ int li(int x, int y) const { return (y - y0) * RW + (x - x0); }
+    __device__ __forceinline__ int gi(int x, int y) const { return y * W + x; }
+    __device__ __forceinline__ uint32_t at(int i) const { return s_w[i]; }
+    __device__ __forceinline__ bool air(int i) const { return cw_air(s_w[i]); }
+    // inside the world: the writes of fire and interactions can reach cells outside it,
+    // where world.cpp:1003-1008 drops them
+    __device__ __forceinline__ bool in_world(int x, int y) const {
+        return (unsigned)x < (unsigned)W && (unsigned)y < (unsigned)H;
     }
-    // the same bytes as the local copy of cell i, in the partner's copy of (x, y)
-    __device__ __forceinline__ void mirror(int x, int y, int i) const {
+
+    // store a cell's word, and its planes, in both copies of a pair
+    __device__ __forceinline__ void set_word(int i, uint32_t w) const {
+        s_w[i] = w;
         if constexpr (PAIR) {
-            bool full;
-            const int j = pli(x, y, &full);
-            if (j < 0) return;
-            st_cluster_u16(p_id + 2u * (uint32_t)j, s_id[i]);
-            if (full) {
-                st_cluster_u8(p_fl + (uint32_t)j, s_fl[i]);
-                st_cluster_u32(p_sc + 4u * (uint32_t)j, (uint32_t)s_sc[i]);
-                st_cluster_u32(p_col + 4u * (uint32_t)j, s_col[i]);
+            const int j = i + pd;
+            if (j >= 0 && j < RW * RHI) st_cluster_u32(p_w + 4u * (uint32_t)j, w);
+        }
+    }
+    __device__ __forceinline__ void set_planes(int i, int32_t sc, uint32_t col) const {
+        s_sc[i] = sc;
+        s_col[i] = col;
+        if constexpr (PAIR) {
+            const int j = i + pd;
+            if (j >= 0 && j < RW * RHF) {
+                st_cluster_u32(p_sc + 4u * (uint32_t)j, (uint32_t)sc);
+                st_cluster_u32(p_col + 4u * (uint32_t)j, col);
             }
         }
     }
-    __device__ __forceinline__ void mirror_idfl(int x, int y, int i) const {
+    __device__ __forceinline__ void set_sc(int i, int32_t sc) const {
+        s_sc[i] = sc;
         if constexpr (PAIR) {
-            bool full;
-            const int j = pli(x, y, &full);
-            if (j < 0) return;
-            st_cluster_u16(p_id + 2u * (uint32_t)j, s_id[i]);
-            if (full) st_cluster_u8(p_fl + (uint32_t)j, s_fl[i]);
+            const int j = i + pd;
+            if (j >= 0 && j < RW * RHF) st_cluster_u32(p_sc + 4u * (uint32_t)j, (uint32_t)sc);
         }
     }
 
-    // 10 AIR bits of column x starting at row y: from the snapshot (0 outside it), or
-    // live
-    __device__ __forceinline__ uint32_t air10(int x, int y) const {
+    // 10 AIR bits of the column of cell i (at (x, y)) starting at it: from the snapshot
+    // (0 outside it), or live
+    __device__ __forceinline__ uint32_t air10(int i, int x, int y) const {
         if constexpr (LIVE) {
             uint32_t bits = 0;
             for (int k = 0; k < 10; k++)
-                if (type(x, y + k) == T_AIR) bits |= 1u << k;
+                if (air(i + k * RW)) bits |= 1u << k;
             return bits;
         }
         int sx = x - ax0, sy = y - ay0;
@@ -269,159 +310,63 @@ struct Tile : TileData {
         return (uint32_t)(v >> b) & 0x3FFu;
     }
 
-    // inside the world (always true away from the world edge)
-    __device__ __forceinline__ bool inw(int x, int y) const {
-        return !EDGE || ((unsigned)x < (unsigned)W && (unsigned)y < (unsigned)H);
+    __device__ __forceinline__ int32_t df_load(int g) const { return df[g]; }
+    // the pending diff of cell i (0 where it is not SOUP)
+    __device__ __forceinline__ int32_t df_of(int i, int g) const { return cw_is(s_w[i], T_SOUP) ? df[g] : 0; }
+    // cell i becomes `c`; the visited mark stays with the position
+    __device__ __forceinline__ void put(int i, int g, const Cell &c) const {
+        set_word(i, (c.w & ~CW_VIS) | CW_DIRTY | (s_w[i] & CW_VIS));
+        set_planes(i, c.sc, c.col);
+        if (cw_is(c.w, T_SOUP)) df[g] = c.df;
     }
-    // inside the world whatever EDGE: the writes of fire and interactions can reach
-    // cells outside the world, where world.cpp:1003-1008 drops them
-    __device__ __forceinline__ bool in_world(int x, int y) const {
-        return (unsigned)x < (unsigned)W && (unsigned)y < (unsigned)H;
+    // the same, for a cell known not to be SOUP
+    __device__ __forceinline__ void put_dry(int i, uint32_t w, int32_t sc, uint32_t col) const {
+        set_word(i, (w & ~CW_VIS) | CW_DIRTY | (s_w[i] & CW_VIS));
+        set_planes(i, sc, col);
     }
-    __device__ __forceinline__ int li(int x, int y) const { return (y - y0) * RW + (x - x0); }
-
-    // world.cpp:999-1002: outside the world reads Tiles_TEST_SOLID
-    __device__ __forceinline__ int id(int x, int y) const {
-        if (!inw(x, y)) return id_solid;
-        return s_id[li(x, y)] & 0x7FFF;
-    }
-    __device__ __forceinline__ int type(int x, int y) const { return mt_type(ma[id(x, y)]); }
-    __device__ __forceinline__ int32_t sc(int x, int y) const {
-        if (!inw(x, y)) return 0;
-        return s_sc[li(x, y)];
-    }
-    __device__ __forceinline__ int32_t df_of(int x, int y) const {
-        if (!inw(x, y) || mt_type(ma[id(x, y)]) != T_SOUP) return 0;
-        return df[y * W + x];
-    }
-    // The active cell. Its df field starts at 0 and collects the change of its
-    // pending diff (put_delta applies it with a reduction); the stored diff is
-    // loaded only where a rule needs the value itself (df_load).
-    __device__ __forceinline__ Cell get_active(int x, int y) const {
-        Cell c;
-        int i = li(x, y);
-        c.id = s_id[i] & 0x7FFF;
-        c.fl = s_fl[i] & (uint8_t)~VISITED;
-        c.sc = s_sc[i];
-        c.col = s_col[i];
-        c.df = 0;
-        return c;
-    }
-    __device__ __forceinline__ int32_t df_load(int x, int y) const { return df[y * W + x]; }
-    // write the active cell back at its own position, adding its diff change
-    __device__ __forceinline__ void put_delta(int x, int y, const Cell &c) const {
-        int i = li(x, y);
-        s_id[i] = c.id | DIRTY;
-        s_fl[i] = (uint8_t)((c.fl & (uint8_t)~VISITED) | (s_fl[i] & VISITED));
-        s_sc[i] = c.sc;
-        s_col[i] = c.col;
-        mirror(x, y, i);
-        if (c.df != 0) atomicAdd(&df[y * W + x], c.df);  // no return value: a fire-and-forget reduction
-    }
-    // world.cpp:1004-1008: outside the world writes are dropped
-    __device__ __forceinline__ void put(int x, int y, const Cell &c) const {
-        if (!inw(x, y)) return;
-        int i = li(x, y);
-        s_id[i] = c.id | DIRTY;
-        s_fl[i] = (uint8_t)((c.fl & (uint8_t)~VISITED) | (s_fl[i] & VISITED));
-        s_sc[i] = c.sc;
-        s_col[i] = c.col;
-        mirror(x, y, i);
-        if (mt_type(ma[c.id]) == T_SOUP) df[y * W + x] = c.df;
-    }
-    __device__ __forceinline__ void set_nothing(int x, int y) const {
-        Cell c;
-        c.id = (uint16_t)id_air;
-        c.fl = 0;
-        c.sc = 0;
-        c.col = 0;
-        c.df = 0;
-        put(x, y, c);
-    }
-    // write the cell at (sx, sy) over (dx, dy); the visited mark stays with the position
-    __device__ __forceinline__ void move(int dx, int dy, int sx, int sy) const {
-        if (!inw(dx, dy)) return;
-        int d = li(dx, dy);
-        if (!inw(sx, sy)) {
-            s_id[d] = (uint16_t)id_solid | DIRTY;
-            s_fl[d] = (uint8_t)(s_fl[d] & VISITED);
-            s_sc[d] = 0;
-            s_col[d] = 0xff0000u;
-            mirror(dx, dy, d);
-            return;
-        }
-        int s = li(sx, sy);
-        uint16_t v = s_id[s] & 0x7FFF;
-        s_id[d] = v | DIRTY;
-        s_fl[d] = (uint8_t)((s_fl[s] & (uint8_t)~VISITED) | (s_fl[d] & VISITED));
-        s_sc[d] = s_sc[s];
-        s_col[d] = s_col[s];
-        mirror(dx, dy, d);
-        if (mt_type(ma[v]) == T_SOUP) {
-            df[dy * W + dx] = df[sy * W + sx];
-            if (TEMP && tp) tp[dy * W + dx] = tp[sy * W + sx];
+    __device__ __forceinline__ void set_nothing(int i) const { put_dry(i, mw[id_air], 0, 0); }
+    // write the cell at s over d; the visited mark stays with the position
+    __device__ __forceinline__ void move(int d, int dg, int s, int sg) const {
+        const uint32_t v = s_w[s];
+        set_word(d, (v & ~CW_VIS) | CW_DIRTY | (s_w[d] & CW_VIS));
+        set_planes(d, s_sc[s], s_col[s]);
+        if (cw_is(v, T_SOUP)) {
+            df[dg] = df[sg];
+            if (TEMP && tp) tp[dg] = tp[sg];
         }
     }
     // Temperatures of SOUP cells live in HBM beside the diff; the tile's scalar is
     // their amount. They move only where a SOUP cell moves or is made, so the
     // rules touch them at those few places and nowhere else.
-    __device__ __forceinline__ int16_t tp_load(int x, int y) const {
-        return (TEMP && tp) ? tp[y * W + x] : (int16_t)0;
-    }
-    __device__ __forceinline__ void tp_store(int x, int y, int16_t v) const {
-        if (TEMP && tp && inw(x, y)) tp[y * W + x] = v;
+    __device__ __forceinline__ int16_t tp_load(int g) const { return (TEMP && tp) ? tp[g] : (int16_t)0; }
+    __device__ __forceinline__ void tp_store(int g, int16_t v) const {
+        if (TEMP && tp) tp[g] = v;
     }
     // put a tile just made by a factory (TilesCreate): a SOUP tile takes the
     // factory temperature, or `keep` (a reaction keeps the old temperature)
-    __device__ __forceinline__ void put_new(int x, int y, const Cell &c, const MatTable *mt, bool keep = false,
+    __device__ __forceinline__ void put_new(int i, int g, const Cell &c, const MatTable *mt, bool keep = false,
                                             int32_t keep_t = 0) const {
-        put(x, y, c);
-        if (TEMP && tp && mt_type(ma[c.id]) == T_SOUP)
-            tp_store(x, y, keep ? (int16_t)keep_t : (int16_t)__ldg(&mt->f_temp[c.id]));
+        put(i, g, c);
+        if (TEMP && tp && cw_is(c.w, T_SOUP)) tp[g] = keep ? (int16_t)keep_t : (int16_t)__ldg(&mt->f_temp[cw_id(c.w)]);
     }
     // only a change marks the cell for write-back (settled sand clears an already
-    // clear flag every pass)
-    __device__ __forceinline__ void set_moved(int x, int y, bool on) const {
-        if (!inw(x, y)) return;
-        int i = li(x, y);
-        const uint8_t f = s_fl[i];
-        const uint8_t nf = on ? (uint8_t)(f | MOVED) : (uint8_t)(f & (uint8_t)~MOVED);
-        if (nf != f) {
-            s_fl[i] = nf;
-            s_id[i] |= DIRTY;
-            mirror_idfl(x, y, i);
-        }
+    // clear flag every pass); w: the cell's word
+    __device__ __forceinline__ void set_moved_w(int i, uint32_t w, bool on) const {
+        const uint32_t n = on ? w | CW_MOVED : w & ~CW_MOVED;
+        if (n != w) set_word(i, n | CW_DIRTY);
     }
-    __device__ __forceinline__ void add_diff(int x, int y, int32_t v) const {
-        if (!inw(x, y)) return;
-        atomicAdd(&df[y * W + x], v);  // fire-and-forget reduction: the thread does not wait
+    __device__ __forceinline__ void set_moved(int i, bool on) const { set_moved_w(i, s_w[i], on); }
+    __device__ __forceinline__ void add_diff(int g, int32_t v) const {
+        atomicAdd(&df[g], v);  // fire-and-forget reduction: the thread does not wait
     }
     // f32 worlds: fluidAmountDiff += v as the reference's float add. No other cell of
     // the sub-phase (or wavefront step) touches this diff, and the ones that touched
     // it before did so in the reference's order, so a plain read-modify-write adds in
     // that order.
-    __device__ __forceinline__ void add_diff_f(int x, int y, float v) const {
-        if (!inw(x, y)) return;
-        int32_t *p = &df[y * W + x];
-        *p = __float_as_int(__fadd_rn(__int_as_float(*p), v));
+    __device__ __forceinline__ void add_diff_f(int g, float v) const {
+        df[g] = __float_as_int(__fadd_rn(__int_as_float(df[g]), v));
     }
-    // write the active cell back at its own position with its diff (f32 worlds)
-    __device__ __forceinline__ void put_df(int x, int y, const Cell &c, float dfv) const {
-        int i = li(x, y);
-        s_id[i] = c.id | DIRTY;
-        s_fl[i] = (uint8_t)((c.fl & (uint8_t)~VISITED) | (s_fl[i] & VISITED));
-        s_sc[i] = c.sc;
-        s_col[i] = c.col;
-        mirror(x, y, i);
-        df[y * W + x] = __float_as_int(dfv);
-    }
-    __device__ __forceinline__ bool vis(int x, int y) const { return (s_fl[li(x, y)] & VISITED) != 0; }
-    __device__ __forceinline__ void setvis(int x, int y) const {
-        if (!inw(x, y)) return;
-        const int i = li(x, y);
-        s_fl[i] |= VISITED;
-        mirror_idfl(x, y, i);
-    }
+    __device__ __forceinline__ void setvis(int i) const { set_word(i, s_w[i] | CW_VIS); }
 };
 
 // ------------------------------------------------------------- rule context
@@ -433,13 +378,13 @@ struct Ctx {
     int id_fire, id_water, id_lava, id_steam, id_obsidian, has_inter;
     bool f32;  // f32 liquid amounts: the ledger keeps no fluid rows (a compile-time constant)
     const MatTable *mt;
-    long long *led_s;      // shared ledger [LED_ROWS][64]
+    int32_t *led_s;        // shared ledger [LED_ROWS][64] of the chunk-pass
     long long *led_g;      // global ledger [LED_ROWS][MAXMAT]
-    const uint32_t *ma;
-    const uint8_t *mreact;  // reactions per material (shared)
+    const uint32_t *mw;    // material words (shared)
     // the cell's spawn event, a local of its own: emit_spawns takes its address, and a
     // member whose address escapes keeps the whole context in local memory
     SpawnEv *ev;
+    int ev_n;  // particles the cell emits (0: none)
     // start the draws of the cell at (x, y); most cells never draw, so the key
     // (two hash rounds) is computed only when the first draw needs it
     __device__ __forceinline__ void at(int x, int y) {
@@ -458,42 +403,45 @@ struct Ctx {
     __device__ __forceinline__ uint32_t D() { return draw_k(key(), k++); }
 };
 
-__device__ __forceinline__ void led_add(Ctx &c, int row, int mat, long long v) {
-    if (v == 0 || mt_type(c.ma[mat]) == T_AIR) return;
-    if (mat < 64 && v > -(1LL << 24) && v < (1LL << 24)) {
-        // lanes of a warp mostly hit the same counter: sum them first, one atomic per group
-        const unsigned act = __activemask();
-        const unsigned grp = __match_any_sync(act, row * 64 + mat);
-        const int sum = __reduce_add_sync(grp, (int)v);
-        if ((threadIdx.x & 31) == __ffs(grp) - 1)
-            atomicAdd((unsigned long long *)&c.led_s[row * 64 + mat], (unsigned long long)(long long)sum);
-    } else if (mat < 64) {
-        atomicAdd((unsigned long long *)&c.led_s[row * 64 + mat], (unsigned long long)v);
-    } else {
-        atomicAdd((unsigned long long *)&c.led_g[row * MAXMAT + mat], (unsigned long long)v);
-    }
+// Ledger counts of one chunk-pass are 32-bit shared counters (native shared atomics;
+// 64-bit ones are compare-and-swap loops), added to the world's 64-bit ledger when the
+// chunk-pass ends. A counter takes amounts below 1024 only, so that a chunk-pass, with
+// at most 3 sweeps x 16384 cells and a few dozen entries a cell, cannot overflow it;
+// larger ones go to the world's ledger at once.
+__device__ __forceinline__ void led_add(Ctx &c, int row, uint32_t w, int32_t v) {
+    if (v == 0 || cw_air(w)) return;
+    const int mat = cw_id(w);
+    if (mat < 64 && v > -1024 && v < 1024)
+        atomicAdd(&c.led_s[row * 64 + mat], v);
+    else
+        atomicAdd((unsigned long long *)&c.led_g[row * MAXMAT + mat], (unsigned long long)(long long)v);
+}
+__device__ __forceinline__ void led_add64(Ctx &c, int row, uint32_t w, long long v) {
+    if (v > -1024 && v < 1024)
+        led_add(c, row, w, (int32_t)v);
+    else if (!cw_air(w))
+        atomicAdd((unsigned long long *)&c.led_g[row * MAXMAT + cw_id(w)], (unsigned long long)v);
 }
 // a conversion (not a move) of the content old -> nw
-__device__ __forceinline__ void led_swap(Ctx &c, int old_id, long long old_fluid, int new_id, long long new_fluid) {
-    led_add(c, LED_DN, old_id, 1);
-    if (!c.f32 && mt_type(c.ma[old_id]) == T_SOUP) led_add(c, LED_DF, old_id, old_fluid);
-    led_add(c, LED_CN, new_id, 1);
-    if (!c.f32 && mt_type(c.ma[new_id]) == T_SOUP) led_add(c, LED_CF, new_id, new_fluid);
+__device__ __forceinline__ void led_swap(Ctx &c, uint32_t old_w, long long old_fluid, uint32_t new_w,
+                                         long long new_fluid) {
+    led_add(c, LED_DN, old_w, 1);
+    if (!c.f32 && cw_is(old_w, T_SOUP)) led_add64(c, LED_DF, old_w, old_fluid);
+    led_add(c, LED_CN, new_w, 1);
+    if (!c.f32 && cw_is(new_w, T_SOUP)) led_add64(c, LED_CF, new_w, new_fluid);
 }
-// conversion of whatever is at (x, y) into nw
+// conversion of whatever is at cell i into nw
 template <class TL>
-__device__ __forceinline__ void led_replace_at(const TL &T, Ctx &c, int x, int y, const Cell &nw) {
-    if (!T.inw(x, y)) return;
-    int oid = T.id(x, y);
-    long long of = (!c.f32 && mt_type(c.ma[oid]) == T_SOUP) ? (long long)T.sc(x, y) + T.df_of(x, y) : 0;
-    led_swap(c, oid, of, nw.id, (long long)nw.sc + nw.df);
+__device__ __forceinline__ void led_replace_at(const TL &T, Ctx &c, int i, int g, const Cell &nw) {
+    const uint32_t o = T.at(i);
+    const long long of = (!c.f32 && cw_is(o, T_SOUP)) ? (long long)T.s_sc[i] + T.df_of(i, g) : 0;
+    led_swap(c, o, of, nw.w, (long long)nw.sc + nw.df);
 }
 
 // TilesCreate(id, x, y), game_datastruct.cpp:494-574
 __device__ __forceinline__ Cell create_tile(Ctx &c, int mid) {
     Cell t;
-    t.id = (uint16_t)mid;
-    t.fl = 0;
+    t.w = c.mw[mid];
     t.df = 0;
     t.sc = soup_scalar(c.mt, mid, c.f32);  // a temperature, or a SOUP tile's amount
     t.col = __ldg(&c.mt->f_base[mid]);
@@ -543,651 +491,653 @@ __device__ __forceinline__ bool can_sink(const uint32_t *ma, const float *md, in
     return t == T_AIR || (t != T_SOLID && md[other] < md[self]);
 }
 
-// the world of the CTA's current chunk (copied per chunk by thread 0)
+// the world of the CTA's current chunk
 __shared__ WorldDev s_w;
 
-// one SOUP flow from (x, y) towards (x + dx, y + dy), shared by the four directions
-// of world.cpp:1309-1460; a rendering world also adds it to the flow of (x, y)
-// (flowX -= / += flow for left / right, flowY += / -= for down / up,
-// world.cpp:1334,1374,1402,1432), a reduction no other cell of the sub-phase makes
-template <class TL>
-__device__ __forceinline__ void soup_flow(const TL &T, Ctx &c, Cell &t, int32_t &rem, int32_t flow, int nT, int x,
-                                          int y, int dx, int dy) {
-    if (flow == 0) return;
-    const int nx = x + dx, ny = y + dy;
-    int32_t *fw = s_w.flow;
-    if (fw) atomicAdd(&fw[2 * ((size_t)y * T.W + x) + (dx != 0 ? 0 : 1)], (dx + dy) * flow);
-    rem -= flow;
-    t.df -= flow;
-    if (nT == T_AIR) {
-        Cell nt;
-        nt.id = t.id;
-        nt.fl = 0;
-        nt.sc = 0;
-        nt.col = t.col;
-        nt.df = flow;
-        T.put(nx, ny, nt);
-        T.tp_store(nx, ny, T.tp_load(x, y));  // MaterialInstance(tile.mat, tile.color, tile.temperature)
-        led_add(c, LED_CN, t.id, 1);
-    } else {
-        T.add_diff(nx, ny, flow);
-    }
+// a liquid cell's flow in a rendering world, added to the flow of its cell (flowX -= /
+// += flow for left / right, flowY += / -= for down / up, world.cpp:1334,1374,1402,1432):
+// a reduction no other cell of the sub-phase makes
+__device__ __forceinline__ void render_flow(int32_t *fw, int g, int axis, int32_t v) {
+    atomicAdd(&fw[2 * (size_t)g + axis], v);
+}
+__device__ __forceinline__ void render_flow_f(int32_t *fw, int g, int axis, float v, bool add) {
+    float *q = reinterpret_cast<float *>(fw) + 2 * (size_t)g + axis;
+    *q = add ? __fadd_rn(*q, v) : __fsub_rn(*q, v);
 }
 
-// f32 worlds: one flow of world.cpp:1309-1460 from (x, y) towards (x + dx, y + dy);
-// dfv is the active cell's fluidAmountDiff, updated in the reference's order
+// the cell a liquid `w0` of colour `col` makes where it flows into the AIR cell n
+// (word wn): MaterialInstance(tile.mat, tile.color, tile.temperature) with amount 0 and
+// the flow as its pending diff
 template <class TL>
-__device__ __forceinline__ void soup_flow_f(const TL &T, Ctx &c, const Cell &t, float &rem, float &dfv, float flow,
-                                            int nT, int x, int y, int dx, int dy) {
-    if (flow == 0.0f) return;
-    const int nx = x + dx, ny = y + dy;
-    float *fw = reinterpret_cast<float *>(s_w.flow);
-    if (fw) {
-        // flowX / flowY of (x, y) (world.cpp:1334,1374,1402,1432): only this cell adds to them
-        float *q = &fw[2 * ((size_t)y * T.W + x) + (dx != 0 ? 0 : 1)];
-        *q = (dx + dy) > 0 ? __fadd_rn(*q, flow) : __fsub_rn(*q, flow);
-    }
-    rem = __fsub_rn(rem, flow);
-    dfv = __fsub_rn(dfv, flow);
-    if (nT == T_AIR) {
-        // MaterialInstance(tile.mat, tile.color, tile.temperature), fluidAmount 0,
-        // then fluidAmountDiff (0) += flow
-        Cell nt;
-        nt.id = t.id;
-        nt.fl = 0;
-        nt.sc = __float_as_int(0.0f);
-        nt.col = t.col;
-        nt.df = __float_as_int(__fadd_rn(0.0f, flow));
-        T.put(nx, ny, nt);
-        T.tp_store(nx, ny, T.tp_load(x, y));
-        led_add(c, LED_CN, t.id, 1);
-    } else {
-        T.add_diff_f(nx, ny, flow);
-    }
+__device__ __forceinline__ void flow_into_air(const TL &T, uint32_t w0, uint32_t col, int n, uint32_t wn, int gn,
+                                              int32_t diff, int g) {
+    T.set_word(n, (w0 & CW_MAT) | CW_DIRTY | (wn & CW_VIS));
+    T.set_planes(n, 0, col);
+    T.df[gn] = diff;
+    T.tp_store(gn, T.tp_load(g));
 }
 
-__device__ __forceinline__ void spawn_one(Ctx &c, int kind, int x, int y, const Cell &t, float vx, float vy) {
-    c.ev->n = 1;
+// the active liquid trades places with its liquid neighbour n (world.cpp:1341-1350,
+// 1439-1448), carrying its whole pending diff
+template <class TL>
+__device__ __forceinline__ void swap_liquid(const TL &T, uint32_t w0, int32_t sc, uint32_t col, int32_t diff, int i,
+                                            int g, int n, int gn) {
+    const int16_t tv = T.tp_load(g);
+    T.move(i, g, n, gn);
+    Cell t;
+    t.w = w0;
+    t.sc = sc;
+    t.col = col;
+    t.df = diff;
+    T.put(n, gn, t);
+    T.tp_store(gn, tv);
+}
+
+// WATER on LAVA, world.cpp:1519-1537; old_fluid: the water's amount and diff
+template <class TL>
+__device__ __forceinline__ void water_on_lava(const TL &T, Ctx &c, uint32_t w0, long long old_fluid, int i, int g) {
+    const MatTable *mt = c.mt;
+    Cell st = create_tile(c, c.id_steam);
+    led_swap(c, w0, old_fluid, st.w, c.f32 ? 0 : (long long)st.sc);
+    T.put_new(i, g, st, mt);
+    const int n = i + T.RW, gn = g + T.W;
+    Cell ob = create_tile(c, c.id_obsidian);
+    led_replace_at(T, c, n, gn, ob);
+    T.put_new(n, gn, ob, mt);
+    T.setvis(n);
+    for (int xx = -1; xx <= 1; xx++)
+        for (int yy = 0; yy <= 2; yy++) {
+            const int m = i + yy * T.RW + xx, gm = g + yy * T.W + xx;
+            if (cw_id(T.at(m)) == c.id_lava) {
+                Cell o2 = create_tile(c, c.id_obsidian);
+                led_replace_at(T, c, m, gm, o2);
+                T.put_new(m, gm, o2, mt);
+                T.setvis(m);
+            }
+        }
+}
+
+__device__ __forceinline__ void spawn_one(Ctx &c, int kind, int x, int y, uint32_t w, int32_t sc, uint32_t col,
+                                          float vx, float vy) {
+    c.ev_n = 1;
     c.ev->kind = kind;
     c.ev->x = x;
     c.ev->y = y;
-    c.ev->id = t.id;
-    c.ev->fl = t.fl;
-    c.ev->col = t.col;
-    c.ev->sc = t.sc;
+    c.ev->id = (uint16_t)cw_id(w);
+    c.ev->fl = (uint8_t)((w & (CW_FLAGS & ~CW_VIS)) >> 8);
+    c.ev->col = col;
+    c.ev->sc = sc;
     c.ev->vx = vx;
     c.ev->vy = vy;
 }
 
-// ------------------------------------------------- sweep A, f32 liquids
-// world.cpp:1269-1567 with the reference's own float amounts (FSE_CFG_F32_FLUID):
-// the same branches as the Q16.16 rule, in f32 with every operation rounded on its
-// own; the cell's fluidAmountDiff is read when its turn begins (it already holds the
-// flows of the cells updated before it) and written back with its own flows
-// subtracted in order, as the reference's copy of the tile does.
+// a liquid cell in free fall becomes n particles (world.cpp:1283-1305)
 template <class TL>
-__device__ __forceinline__ void rule_a_soup_f32(const TL &T, Ctx &c, Cell &t, int x, int y) {
-    const uint32_t *ma = T.ma;
-    const float amount = __int_as_float(t.sc);
+__device__ __forceinline__ void free_fall(const TL &T, Ctx &c, uint32_t w0, int32_t sc, uint32_t col, int n, int i,
+                                          int g, int x, int y) {
+    T.set_nothing(i);
+    if (n < 1) n = 1;
+    led_add(c, LED_CN, w0, n - 1);
+    c.ev_n = n;
+    c.ev->kind = 2;
+    c.ev->x = x;
+    c.ev->y = y + 1;
+    c.ev->id = (uint16_t)cw_id(w0);
+    c.ev->fl = 0;
+    c.ev->col = col;
+    c.ev->sc = sc;
+    if (TL::kTemp) c.ev->tp = T.tp_load(g);
+    c.ev->ck = c.key();
+    c.ev->k0 = c.k;
+    c.k += 2 * n;
+}
+
+// settle counts and the moved flags around a liquid that has had its turn
+// (world.cpp:1472-1483): unchanged amounts count, flows wake the liquid neighbours
+__device__ __forceinline__ uint32_t settle_word(uint32_t w0) {
+    uint32_t s = w0 & CW_SETTLE;
+    if (s < CW_SETTLE) s += 0x100u;
+    uint32_t w = (w0 & ~CW_SETTLE) | s;
+    if (s >= 10u << 8) w |= CW_MOVED;
+    return w;
+}
+
+// ------------------------------------------------- sweep A, liquids
+// world.cpp:1269-1567. The neighbours are read first, all together (nothing the cell
+// writes before it reads them is among them: a flow writes only the cell it enters).
+// Q16.16 amounts, or with F32 the reference's own float amounts: the same branches
+// in f32 with every operation rounded on its own, and the cell's fluidAmountDiff read
+// when its turn begins (it already holds the flows of the cells updated before it) and
+// written back with its own flows subtracted in order, as the reference's copy of the
+// tile does.
+template <class TL>
+__device__ __forceinline__ void rule_a_soup(const TL &T, Ctx &c, uint32_t w0, int i, int x, int y) {
+    const int32_t sc = T.s_sc[i];
+    if (sc == 0) return;
+    if (sc < Q_MINV) {
+        led_add64(c, LED_DF, w0, sc);
+        T.set_word(i, w0 | CW_DIRTY);
+        T.set_sc(i, 0);
+        return;
+    }
+    const int RW = T.RW;
+    const uint32_t col = T.s_col[i];
+    const uint32_t wb = T.at(i + RW);
+    const bool airBelow = cw_air(wb);
+    const int g = T.gi(x, y);
+    if (airBelow && sc > Q_FREEFALL) {
+        const uint32_t w2 = T.at(i + 2 * RW), w3 = T.at(i + 3 * RW), w4 = T.at(i + 4 * RW);
+        if (cw_air(w2) && cw_air(w3) && cw_air(w4)) {
+            led_add64(c, LED_DF, w0, T.df_load(g));
+            free_fall(T, c, w0, sc, col, sc >> 18, i, g, x, y);
+            return;
+        }
+    }
+    if (w0 & CW_MOVED) return;
+    const uint32_t wl = T.at(i - 1), wr = T.at(i + 1), wt = T.at(i - RW);
+    const int32_t sb = T.s_sc[i + RW], sl = T.s_sc[i - 1], sr = T.s_sc[i + 1], su = T.s_sc[i - RW];
+    int32_t rem = sc, down = 0, left = 0, right = 0, up = 0;
+    bool gone = false;
+    if ((airBelow && c.iter <= 2) || cw_same(wb, w0)) {
+        const int32_t dst = airBelow ? 0 : sb;
+        down = clampflow(vflow(sc, dst) - dst, sc);
+        rem -= down;
+    } else if (c.iter == 0 && cw_is(wb, T_SOUP)) {
+        if (c.D() % 10 == 0) {
+            swap_liquid(T, w0, sc, col, T.df_load(g), i, g, i + RW, g + T.W);
+            return;
+        }
+    }
+    const bool canL = (cw_air(wl) || cw_same(wl, w0)) && !airBelow;
+    const bool canR = (cw_air(wr) || cw_same(wr, w0)) && !airBelow;
+    gone = rem < Q_MINV;
+    if (!gone && canL) {
+        const int32_t d = rem - (cw_air(wl) ? 0 : sl);
+        left = clampflow(canR ? d / 3 : d / 2, rem);
+        rem -= left;
+        gone = rem < Q_MINV;
+    }
+    if (!gone && canR) {
+        const int32_t d = rem - (cw_air(wr) ? 0 : sr);
+        right = clampflow(d / 2, rem);
+        rem -= right;
+        gone = rem < Q_MINV;
+    }
+    bool swap_up = false;
+    if (!gone) {
+        if (cw_air(wt) || cw_same(wt, w0)) {
+            const int32_t dst = cw_air(wt) ? 0 : su;
+            up = clampflow(rem - vflow(rem, dst), rem);
+            rem -= up;
+            gone = rem < Q_MINV;
+        } else if (c.iter == 0 && cw_is(wt, T_SOUP)) {
+            swap_up = c.D() % 10 == 0;
+        }
+    }
+    // the flows: a new cell in AIR, else a pending diff
+    int made = 0;
+    int32_t *fw = s_w.flow;
+    if (down != 0) {
+        if (fw) render_flow(fw, g, 1, down);
+        if (airBelow) {
+            flow_into_air(T, w0, col, i + RW, wb, g + T.W, down, g);
+            made++;
+        } else {
+            T.add_diff(g + T.W, down);
+        }
+    }
+    if (left != 0) {
+        if (fw) render_flow(fw, g, 0, -left);
+        if (cw_air(wl)) {
+            flow_into_air(T, w0, col, i - 1, wl, g - 1, left, g);
+            made++;
+        } else {
+            T.add_diff(g - 1, left);
+        }
+    }
+    if (right != 0) {
+        if (fw) render_flow(fw, g, 0, right);
+        if (cw_air(wr)) {
+            flow_into_air(T, w0, col, i + 1, wr, g + 1, right, g);
+            made++;
+        } else {
+            T.add_diff(g + 1, right);
+        }
+    }
+    if (up != 0) {
+        if (fw) render_flow(fw, g, 1, -up);
+        if (cw_air(wt)) {
+            flow_into_air(T, w0, col, i - RW, wt, g - T.W, up, g);
+            made++;
+        } else {
+            T.add_diff(g - T.W, up);
+        }
+    }
+    led_add(c, LED_CN, w0, made);
+    const int32_t dd = rem - sc;  // the change of its own pending diff
+    if (swap_up) {
+        swap_liquid(T, w0, sc, col, dd + T.df_load(g), i, g, i - RW, g - T.W);
+        return;
+    }
+    if (gone) {  // the remainder evaporates
+        led_add64(c, LED_DF, w0, rem);
+        T.set_word(i, w0 | CW_DIRTY);
+        if (sc != 0) T.add_diff(g, -sc);
+        return;
+    }
+    uint32_t wn = w0;
+    if (dd == 0) {
+        wn = settle_word(w0);
+    } else {
+        if (cw_is(wt, T_SOUP)) T.set_moved_w(i - RW, wt, false);
+        if (cw_is(wb, T_SOUP)) T.set_moved_w(i + RW, wb, false);
+        if (cw_is(wl, T_SOUP)) T.set_moved_w(i - 1, wl, false);
+        if (cw_is(wr, T_SOUP)) T.set_moved_w(i + 1, wr, false);
+        T.add_diff(g, dd);
+    }
+    T.set_word(i, wn | CW_DIRTY);
+    if (cw_id(w0) == c.id_water && cw_id(wb) == c.id_lava)
+        water_on_lava(T, c, wn, (long long)sc + T.df_load(g), i, g);
+}
+
+template <class TL>
+__device__ __forceinline__ void rule_a_soup_f32(const TL &T, Ctx &c, uint32_t w0, int i, int x, int y) {
+    const int32_t sc = T.s_sc[i];
+    const float amount = __int_as_float(sc);
     if (amount == 0.0f) return;
     if (amount < F_MINV) {
-        t.sc = __float_as_int(0.0f);
-        T.put_delta(x, y, t);  // t.df is 0: the diff stays as it is
+        T.set_word(i, w0 | CW_DIRTY);  // the diff stays as it is
+        T.set_sc(i, __float_as_int(0.0f));
         return;
     }
+    const int RW = T.RW;
+    const uint32_t col = T.s_col[i];
+    const uint32_t wb = T.at(i + RW);
+    const bool airBelow = cw_air(wb);
+    const int g = T.gi(x, y);
     // tile.fluidAmount > 0.005 compares in double (0.005 is a double literal)
-    if ((double)amount > 0.005 && T.type(x, y + 1) == T_AIR && T.type(x, y + 2) == T_AIR &&
-        T.type(x, y + 3) == T_AIR && T.type(x, y + 4) == T_AIR) {  // world.cpp:1283-1305
-        T.set_nothing(x, y);
-        int n = (int)__fdiv_rn(amount, 4.0f);  // int n = tile.fluidAmount / 4
-        if (n < 1) n = 1;
-        led_add(c, LED_CN, t.id, n - 1);
-        c.ev->n = n;
-        c.ev->kind = 2;
-        c.ev->x = x;
-        c.ev->y = y + 1;
-        c.ev->id = t.id;
-        c.ev->fl = 0;
-        c.ev->col = t.col;
-        c.ev->sc = t.sc;
-        if (TL::kTemp) c.ev->tp = T.tp_load(x, y);
-        c.ev->ck = c.key();
-        c.ev->k0 = c.k;
-        c.k += 2 * n;
-        return;
+    if (airBelow && (double)amount > 0.005) {
+        const uint32_t w2 = T.at(i + 2 * RW), w3 = T.at(i + 3 * RW), w4 = T.at(i + 4 * RW);
+        if (cw_air(w2) && cw_air(w3) && cw_air(w4)) {
+            free_fall(T, c, w0, sc, col, (int)__fdiv_rn(amount, 4.0f), i, g, x, y);  // int n = tile.fluidAmount / 4
+            return;
+        }
     }
-    if (t.fl & MOVED) return;
+    if (w0 & CW_MOVED) return;
+    float dfv = __int_as_float(T.df_load(g));
+    const uint32_t wl = T.at(i - 1), wr = T.at(i + 1), wt = T.at(i - RW);
+    const float sb = __int_as_float(T.s_sc[i + RW]), sl = __int_as_float(T.s_sc[i - 1]);
+    const float sr = __int_as_float(T.s_sc[i + 1]), su = __int_as_float(T.s_sc[i - RW]);
     const float start = amount;
     float rem = amount;
-    float dfv = __int_as_float(T.df_load(x, y));
-    const int bid = T.id(x, y + 1);
-    const int bT = mt_type(ma[bid]);
-    const bool airBelow = bT == T_AIR;
-    if ((airBelow && c.iter <= 2) || bid == (int)t.id) {
-        const float dst = (bT == T_SOUP) ? __int_as_float(T.sc(x, y + 1)) : 0.0f;
-        soup_flow_f(T, c, t, rem, dfv, clampflow_f(__fsub_rn(vflow_f(start, dst), dst), start), bT, x, y, 0, 1);
-    } else if (c.iter == 0 && bT == T_SOUP && bid != (int)t.id) {
-        if (c.D() % 10 == 0) {
-            t.df = __float_as_int(dfv);  // the cell leaves its position with its diff
-            const int16_t tv = T.tp_load(x, y);
-            T.move(x, y, x, y + 1);
-            T.put(x, y + 1, t);
-            T.tp_store(x, y + 1, tv);
+    int made = 0;
+    int32_t *fw = s_w.flow;
+    // one flow (world.cpp:1309-1460) into neighbour n
+    auto flow_to = [&](float flow, int n, uint32_t wn, int gn, int axis, bool add) {
+        if (flow == 0.0f) return;
+        if (fw) render_flow_f(fw, g, axis, flow, add);
+        rem = __fsub_rn(rem, flow);
+        dfv = __fsub_rn(dfv, flow);
+        if (cw_air(wn)) {
+            // fluidAmount 0, then fluidAmountDiff (0) += flow
+            flow_into_air(T, w0, col, n, wn, gn, __float_as_int(__fadd_rn(0.0f, flow)), g);
+            made++;
+        } else {
+            T.add_diff_f(gn, flow);
+        }
+    };
+    bool done = false;  // the remainder evaporates
+    if ((airBelow && c.iter <= 2) || cw_same(wb, w0)) {
+        const float dst = airBelow ? 0.0f : sb;
+        flow_to(clampflow_f(__fsub_rn(vflow_f(start, dst), dst), start), i + RW, wb, g + T.W, 1, true);
+    } else if (c.iter == 0 && cw_is(wb, T_SOUP)) {
+        if (c.D() % 10 == 0) {  // the cell leaves its position with its diff
+            swap_liquid(T, w0, sc, col, __float_as_int(dfv), i, g, i + RW, g + T.W);
             return;
         }
     }
-    if (rem < F_MINV) {
-        T.put_df(x, y, t, __fsub_rn(dfv, rem));
-        return;
+    const bool canL = (cw_air(wl) || cw_same(wl, w0)) && !airBelow;
+    const bool canR = (cw_air(wr) || cw_same(wr, w0)) && !airBelow;
+    done = rem < F_MINV;
+    if (!done && canL) {
+        const float dst = cw_air(wl) ? 0.0f : sl;
+        flow_to(clampflow_f(__fdiv_rn(__fsub_rn(rem, dst), canR ? 3.0f : 2.0f), rem), i - 1, wl, g - 1, 0, false);
+        done = rem < F_MINV;
     }
-    const int lid = T.id(x - 1, y);
-    const int lT = mt_type(ma[lid]);
-    const bool canL = (lT == T_AIR || lid == (int)t.id) && !airBelow;
-    const int rid = T.id(x + 1, y);
-    const int rT = mt_type(ma[rid]);
-    const bool canR = (rT == T_AIR || rid == (int)t.id) && !airBelow;
-    if (canL) {
-        const float dst = (lT == T_SOUP) ? __int_as_float(T.sc(x - 1, y)) : 0.0f;
-        soup_flow_f(T, c, t, rem, dfv, clampflow_f(__fdiv_rn(__fsub_rn(rem, dst), canR ? 3.0f : 2.0f), rem), lT, x,
-                    y, -1, 0);
+    if (!done && canR) {
+        const float dst = cw_air(wr) ? 0.0f : sr;
+        flow_to(clampflow_f(__fdiv_rn(__fsub_rn(rem, dst), 2.0f), rem), i + 1, wr, g + 1, 0, true);
+        done = rem < F_MINV;
     }
-    if (rem < F_MINV) {
-        T.put_df(x, y, t, __fsub_rn(dfv, rem));
-        return;
-    }
-    if (canR) {
-        const float dst = (rT == T_SOUP) ? __int_as_float(T.sc(x + 1, y)) : 0.0f;
-        soup_flow_f(T, c, t, rem, dfv, clampflow_f(__fdiv_rn(__fsub_rn(rem, dst), 2.0f), rem), rT, x, y, 1, 0);
-    }
-    if (rem < F_MINV) {
-        T.put_df(x, y, t, __fsub_rn(dfv, rem));
-        return;
-    }
-    const int tid = T.id(x, y - 1);
-    const int tT = mt_type(ma[tid]);
-    if (tT == T_AIR || tid == (int)t.id) {
-        const float dst = (tT == T_SOUP) ? __int_as_float(T.sc(x, y - 1)) : 0.0f;
-        soup_flow_f(T, c, t, rem, dfv, clampflow_f(__fsub_rn(rem, vflow_f(rem, dst)), rem), tT, x, y, 0, -1);
-    } else if (c.iter == 0 && tT == T_SOUP && tid != (int)t.id) {
-        if (c.D() % 10 == 0) {
-            t.df = __float_as_int(dfv);
-            const int16_t tv = T.tp_load(x, y);
-            T.move(x, y, x, y - 1);
-            T.put(x, y - 1, t);
-            T.tp_store(x, y - 1, tv);
-            return;
+    bool swap_up = false;
+    if (!done) {
+        if (cw_air(wt) || cw_same(wt, w0)) {
+            const float dst = cw_air(wt) ? 0.0f : su;
+            flow_to(clampflow_f(__fsub_rn(rem, vflow_f(rem, dst)), rem), i - RW, wt, g - T.W, 1, false);
+            done = rem < F_MINV;
+        } else if (c.iter == 0 && cw_is(wt, T_SOUP)) {
+            swap_up = c.D() % 10 == 0;
         }
     }
-    if (rem < F_MINV) {
-        T.put_df(x, y, t, __fsub_rn(dfv, rem));
+    led_add(c, LED_CN, w0, made);
+    if (swap_up) {
+        swap_liquid(T, w0, sc, col, __float_as_int(dfv), i, g, i - RW, g - T.W);
         return;
     }
-    if (start == rem) {  // world.cpp:1472-1483
-        uint8_t s = t.fl & SETTLE_MASK;
-        if (s < SETTLE_MASK) s++;
-        t.fl = (uint8_t)((t.fl & ~SETTLE_MASK) | s);
-        if (s >= 10) t.fl |= MOVED;
+    uint32_t wn = w0;
+    if (done) {
+        dfv = __fsub_rn(dfv, rem);
+    } else if (start == rem) {
+        wn = settle_word(w0);
     } else {
-        if (tT == T_SOUP) T.set_moved(x, y - 1, false);
-        if (bT == T_SOUP) T.set_moved(x, y + 1, false);
-        if (lT == T_SOUP) T.set_moved(x - 1, y, false);
-        if (rT == T_SOUP) T.set_moved(x + 1, y, false);
+        if (cw_is(wt, T_SOUP)) T.set_moved_w(i - RW, wt, false);
+        if (cw_is(wb, T_SOUP)) T.set_moved_w(i + RW, wb, false);
+        if (cw_is(wl, T_SOUP)) T.set_moved_w(i - 1, wl, false);
+        if (cw_is(wr, T_SOUP)) T.set_moved_w(i + 1, wr, false);
     }
-    T.put_df(x, y, t, dfv);
-    // WATER on LAVA, world.cpp:1519-1537
-    if ((int)t.id == c.id_water && T.id(x, y + 1) == c.id_lava) {
-        const MatTable *mt = c.mt;
-        Cell st = create_tile(c, c.id_steam);
-        led_swap(c, t.id, 0, st.id, 0);
-        T.put_new(x, y, st, mt);
-        Cell ob = create_tile(c, c.id_obsidian);
-        led_replace_at(T, c, x, y + 1, ob);
-        T.put_new(x, y + 1, ob, mt);
-        T.setvis(x, y + 1);
-        for (int xx = -1; xx <= 1; xx++)
-            for (int yy = 0; yy <= 2; yy++) {
-                if (T.id(x + xx, y + yy) == c.id_lava) {
-                    Cell o2 = create_tile(c, c.id_obsidian);
-                    led_replace_at(T, c, x + xx, y + yy, o2);
-                    T.put_new(x + xx, y + yy, o2, mt);
-                    T.setvis(x + xx, y + yy);
+    T.set_word(i, wn | CW_DIRTY);
+    T.df[g] = __float_as_int(dfv);
+    if (!done && cw_id(w0) == c.id_water && cw_id(wb) == c.id_lava) water_on_lava(T, c, wn, 0, i, g);
+}
+
+// fire, world.cpp:1101-1146. Returns false where the cell burnt out (the sweep goes on
+// to its material's own rule either way, which for FIRE is none)
+template <class TL>
+__device__ __forceinline__ void rule_a_fire(const TL &T, Ctx &c, uint32_t w0, int i, int x, int y) {
+    const MatTable *mt = c.mt;
+    const int g = T.gi(x, y);
+    const int32_t sc = T.s_sc[i];
+    uint32_t col = T.s_col[i];
+    if (c.D() % 10 == 0) col = (255u << 16) | ((uint32_t)(100 + (int)(c.D() % 50)) << 8) | 50u;
+    if (c.D() % 10 == 0) {
+        float vx = (float)((int)(c.D() % 10) - 5) / 20.0f;
+        float vy = -((float)(int)(c.D() % 10) / 10.0f) / 3.0f + -0.5f;
+        spawn_one(c, 3, x, y - 1, w0, sc, col, vx, vy);
+        led_add(c, LED_CN, w0, 1);
+    }
+    if (c.D() % 150 == 0) {
+        led_swap(c, w0, (long long)sc, T.mw[T.id_air], 0);
+        T.set_nothing(i);
+        T.setvis(i);
+    } else {
+        bool found = false;
+        for (int xx = -2; xx <= 2; xx++)
+            for (int yy = -2; yy <= 2; yy++) {
+                const int n = i + yy * T.RW + xx;
+                if (cw_is(T.at(n), T_SOLID)) {
+                    found = true;
+                    if (c.D() % 500 == 0) {
+                        Cell f = create_tile(c, c.id_fire);
+                        if (T.in_world(x + xx, y + yy)) {
+                            const int gn = g + yy * T.W + xx;
+                            led_replace_at(T, c, n, gn, f);
+                            T.put_new(n, gn, f, mt);
+                            T.setvis(n);
+                        }
+                    }
                 }
             }
+        if (!found && c.D() % 120 == 0) {
+            led_swap(c, w0, (long long)sc, T.mw[T.id_air], 0);
+            T.set_nothing(i);
+            T.setvis(i);
+        }
     }
 }
 
-// ----------------------------------------------------------------- sweep A
+// interactions of sand with the cell below it, world.cpp:1153-1179: true where the
+// pair of materials has any (the sand's turn then ends)
 template <class TL>
-__device__ __forceinline__ void rule_a(const TL &T, Ctx &c, int x, int y) {
-    if (T.vis(x, y)) return;  // world.cpp:1091
-    const uint32_t *ma = T.ma;
-    const float *md = T.md;
-    const int sid = T.id(x, y);
-    const uint32_t a = ma[sid];
-    if (c.iter >= mt_iter(a)) {  // world.cpp:1093-1096
-        T.setvis(x, y);
+__device__ __forceinline__ bool rule_a_inter(const TL &T, Ctx &c, uint32_t w0, int bid, int i, int x, int y) {
+    const MatTable *mt = c.mt;
+    const int sid = cw_id(w0), g = T.gi(x, y);
+    int hit = -1;
+    for (int k = 0; k < mt->n_inter; k++)
+        if (mt->inter[k][0] == sid && mt->inter[k][1] == bid) hit = k;
+    if (hit < 0) return false;
+    for (int k = 0; k < mt->n_inter; k++) {
+        if (mt->inter[k][0] != sid || mt->inter[k][1] != bid) continue;
+        int kind = mt->inter[k][2], d1 = mt->inter[k][3], d2 = mt->inter[k][4];
+        int ox = mt->inter[k][5], oy = mt->inter[k][6];
+        // the radius is a u32 in the reference, so its loops compare
+        // unsigned: a box whose low corner is negative is not visited
+        if (ox - d2 < 0 || oy - d2 < 0) continue;
+        for (int xx = ox - d2; xx <= ox + d2; xx++)
+            for (int yy = oy - d2; yy <= oy + d2; yy++) {
+                const int n = i + yy * T.RW + xx;
+                const int nid = cw_id(T.at(n));
+                bool doit = (kind == INTER_TRANSFORM) ? (nid == bid) : ((xx == 0 && yy == 0) || nid == T.id_air);
+                if (doit) {
+                    Cell nt = create_tile(c, d1);
+                    if (T.in_world(x + xx, y + yy)) {
+                        const int gn = g + yy * T.W + xx;
+                        led_replace_at(T, c, n, gn, nt);
+                        T.put_new(n, gn, nt, mt);
+                        T.setvis(n);
+                    }
+                }
+            }
+    }
+    return true;
+}
+
+// temperature reactions of a SAND cell, world.cpp:1181-1204: true where one happened
+template <class TL>
+__device__ __forceinline__ bool rule_a_react(const TL &T, Ctx &c, uint32_t w0, int i, int x, int y) {
+    const MatTable *mt = c.mt;
+    const int sid = cw_id(w0), g = T.gi(x, y);
+    const int32_t sc = T.s_sc[i];
+    const int nr = mt->n_react[sid];
+    bool react = false;
+    for (int k = 0; k < nr; k++) {
+        int kind = mt->react[sid][k][0], temp = mt->react[sid][k][1], res = mt->react[sid][k][2];
+        bool hit = (kind == REACT_BELOW) ? (sc < temp) : (sc > temp);
+        if (hit) {
+            Cell nt = create_tile(c, res);
+            // the temperature is kept (world.cpp:1188,1196): in the scalar,
+            // or beside the amount of a SOUP result
+            if (!cw_is(nt.w, T_SOUP)) nt.sc = sc;
+            led_replace_at(T, c, i, g, nt);
+            T.put_new(i, g, nt, mt, true, sc);
+            T.setvis(i);
+            react = true;
+        }
+    }
+    return react;
+}
+
+// ----------------------------------------------------------------- sweep A
+// c.ev_n: the particles the cell emits (its event in *c.ev)
+template <class TL>
+__device__ __forceinline__ void rule_a(const TL &T, Ctx &c, int i, int x, int y) {
+    const uint32_t w0 = T.at(i);
+    if (w0 & CW_VIS) return;  // world.cpp:1091
+    if (!(w0 & CW_LIVE)) {    // world.cpp:1093-1096
+        T.set_word(i, w0 | CW_VIS);
         return;
     }
-    const int type = mt_type(a);
-    if (type != T_SAND && type != T_SOUP && type != T_GAS && sid != c.id_fire) return;
-    if (sid != c.id_fire) {
-        // the common no-op cases, decided before the cell is loaded: sand that
-        // cannot sink (world.cpp:1206, without interactions or reactions) and gas
-        // with no AIR above (world.cpp:1573)
-        if (type == T_SAND && !c.has_inter && c.mreact[sid] == 0 && !can_sink(ma, md, T.id(x, y + 1), sid)) return;
-        if (type == T_GAS && T.type(x, y - 1) != T_AIR) return;
-    }
-    Cell t = T.get_active(x, y);
     c.at(x, y);
-    const MatTable *mt = c.mt;
-
-    if (sid == c.id_fire) {  // world.cpp:1101-1146
-        if (c.D() % 10 == 0) t.col = (255u << 16) | ((uint32_t)(100 + (int)(c.D() % 50)) << 8) | 50u;
-        if (c.D() % 10 == 0) {
-            float vx = (float)((int)(c.D() % 10) - 5) / 20.0f;
-            float vy = -((float)(int)(c.D() % 10) / 10.0f) / 3.0f + -0.5f;
-            spawn_one(c, 3, x, y - 1, t, vx, vy);
-            led_add(c, LED_CN, t.id, 1);
-        }
-        if (c.D() % 150 == 0) {
-            led_swap(c, t.id, (long long)t.sc + t.df, T.id_air, 0);
-            T.set_nothing(x, y);
-            T.setvis(x, y);
-        } else {
-            bool found = false;
-            for (int xx = -2; xx <= 2; xx++)
-                for (int yy = -2; yy <= 2; yy++) {
-                    if (T.type(x + xx, y + yy) == T_SOLID) {
-                        found = true;
-                        if (c.D() % 500 == 0) {
-                            Cell f = create_tile(c, c.id_fire);
-                            if (T.in_world(x + xx, y + yy)) {
-                                led_replace_at(T, c, x + xx, y + yy, f);
-                                T.put_new(x + xx, y + yy, f, mt);
-                                T.setvis(x + xx, y + yy);
-                            }
-                        }
-                    }
-                }
-            if (!found && c.D() % 120 == 0) {
-                led_swap(c, t.id, (long long)t.sc + t.df, T.id_air, 0);
-                T.set_nothing(x, y);
-                T.setvis(x, y);
-            }
-        }
-    }
-
-    if (type == T_SAND) {
-        const int bid = T.id(x, y + 1);  // world.cpp:1150
-        const int bt = mt_type(ma[bid]);
-        if (c.has_inter) {  // world.cpp:1153-1179
-            int hit = -1;
-            for (int i = 0; i < mt->n_inter; i++)
-                if (mt->inter[i][0] == (int)t.id && mt->inter[i][1] == bid) hit = i;
-            if (hit >= 0) {
-                for (int i = 0; i < mt->n_inter; i++) {
-                    if (mt->inter[i][0] != (int)t.id || mt->inter[i][1] != bid) continue;
-                    int kind = mt->inter[i][2], d1 = mt->inter[i][3], d2 = mt->inter[i][4];
-                    int ox = mt->inter[i][5], oy = mt->inter[i][6];
-                    // the radius is a u32 in the reference, so its loops compare
-                    // unsigned: a box whose low corner is negative is not visited
-                    if (ox - d2 < 0 || oy - d2 < 0) continue;
-                    for (int xx = ox - d2; xx <= ox + d2; xx++)
-                        for (int yy = oy - d2; yy <= oy + d2; yy++) {
-                            bool doit = (kind == INTER_TRANSFORM)
-                                            ? (T.id(x + xx, y + yy) == bid)
-                                            : ((xx == 0 && yy == 0) || T.id(x + xx, y + yy) == T.id_air);
-                            if (doit) {
-                                Cell nt = create_tile(c, d1);
-                                if (T.in_world(x + xx, y + yy)) {
-                                    led_replace_at(T, c, x + xx, y + yy, nt);
-                                    T.put_new(x + xx, y + yy, nt, mt);
-                                    T.setvis(x + xx, y + yy);
-                                }
-                            }
-                        }
-                }
-                return;
-            }
-        }
-        const int nr = c.mreact[t.id];
-        if (nr > 0) {  // world.cpp:1181-1204
-            bool react = false;
-            for (int i = 0; i < nr; i++) {
-                int kind = mt->react[t.id][i][0], temp = mt->react[t.id][i][1], res = mt->react[t.id][i][2];
-                bool hit = (kind == REACT_BELOW) ? (t.sc < temp) : (t.sc > temp);
-                if (hit) {
-                    Cell nt = create_tile(c, res);
-                    // the temperature is kept (world.cpp:1188,1196): in the scalar,
-                    // or beside the amount of a SOUP result
-                    if (mt_type(ma[nt.id]) != T_SOUP) nt.sc = t.sc;
-                    led_replace_at(T, c, x, y, nt);
-                    T.put_new(x, y, nt, mt, true, t.sc);
-                    T.setvis(x, y);
-                    react = true;
-                }
-            }
-            if (react) return;
-        }
+    if (w0 & CW_FIRE) rule_a_fire(T, c, w0, i, x, y);
+    if (cw_is(w0, T_SAND)) {
+        const uint32_t wb = T.at(i + T.RW);  // world.cpp:1150
+        const uint32_t lim = cw_sink(w0);
+        if (c.has_inter && rule_a_inter(T, c, w0, cw_id(wb), i, x, y)) return;
+        if ((w0 & CW_REACT) && rule_a_react(T, c, w0, i, x, y)) return;
         // world.cpp:1206-1267
-        if (!can_sink(ma, md, bid, t.id)) return;
-        const bool canL = can_sink(ma, md, T.id(x - 1, y + 1), t.id);
-        const bool canR = can_sink(ma, md, T.id(x + 1, y + 1), t.id);
+        if (!(wb < lim)) return;
+        const bool canL = T.at(i + T.RW - 1) < lim, canR = T.at(i + T.RW + 1) < lim;
         if (!((canL || canR) && c.D() % 20 == 0)) {
-            if (bt == T_AIR && T.type(x, y + 2) == T_AIR && T.type(x, y + 3) == T_AIR && T.type(x, y + 4) == T_AIR) {
-                T.move(x, y, x, y + 1);
+            const int g = T.gi(x, y), n = i + T.RW;
+            const int32_t sc = T.s_sc[i];
+            const uint32_t col = T.s_col[i];
+            bool falls = cw_air(wb);
+            if (falls) {
+                const uint32_t w2 = T.at(i + 2 * T.RW), w3 = T.at(i + 3 * T.RW), w4 = T.at(i + 4 * T.RW);
+                falls = cw_air(w2) && cw_air(w3) && cw_air(w4);
+            }
+            T.move(i, g, n, g + T.W);
+            if (falls) {
                 float vx = (float)((int)(c.D() % 10) - 5) / 20.0f;
                 float vy = (float)(-((int)(c.D() % 2) + 3)) / 10.0f + 1.5f;
-                spawn_one(c, 1, x, y + 1, t, vx, vy);
+                spawn_one(c, 1, x, y + 1, w0, sc, col, vx, vy);
             } else {
-                T.move(x, y, x, y + 1);
-                if (c.D() % 2 == 0) t.fl |= MOVED;
-                T.put(x, y + 1, t);
-                T.setvis(x, y + 1);
+                const uint32_t t = c.D() % 2 == 0 ? w0 | CW_MOVED : w0;
+                T.set_word(n, t | CW_DIRTY | CW_VIS);
+                T.set_planes(n, sc, col);
             }
             if (c.D() % 2 == 0) {
-                if (x > 0 && T.type(x - 1, y + 1) == T_SAND) {
-                    if (c.D() % 2 == 0) T.set_moved(x - 1, y + 1, true);
+                if (x > 0 && cw_is(T.at(n - 1), T_SAND)) {
+                    if (c.D() % 2 == 0) T.set_moved(n - 1, true);
                 }
-                if (x < T.W - 1 && T.type(x + 1, y + 1) == T_SAND) {
-                    if (c.D() % 2 == 0) T.set_moved(x + 1, y + 1, true);
+                if (x < T.W - 1 && cw_is(T.at(n + 1), T_SAND)) {
+                    if (c.D() % 2 == 0) T.set_moved(n + 1, true);
                 }
             }
         }
-    } else if (TL::kF32 && type == T_SOUP) {
-        rule_a_soup_f32(T, c, t, x, y);
-    } else if (type == T_SOUP) {  // world.cpp:1269-1567
-        if (t.sc == 0) return;
-        if (t.sc < Q_MINV) {
-            led_add(c, LED_DF, t.id, t.sc);
-            t.sc = 0;
-            T.put_delta(x, y, t);
-            return;
-        }
-        if (t.sc > Q_FREEFALL && T.type(x, y + 1) == T_AIR && T.type(x, y + 2) == T_AIR &&
-            T.type(x, y + 3) == T_AIR && T.type(x, y + 4) == T_AIR) {  // world.cpp:1283-1305
-            led_add(c, LED_DF, t.id, T.df_load(x, y));
-            T.set_nothing(x, y);
-            int n = t.sc >> 18;
-            if (n < 1) n = 1;
-            led_add(c, LED_CN, t.id, n - 1);
-            c.ev->n = n;
-            c.ev->kind = 2;
-            c.ev->x = x;
-            c.ev->y = y + 1;
-            c.ev->id = t.id;
-            c.ev->fl = 0;
-            c.ev->col = t.col;
-            c.ev->sc = t.sc;
-            if (TL::kTemp) c.ev->tp = T.tp_load(x, y);
-            c.ev->ck = c.key();
-            c.ev->k0 = c.k;
-            c.k += 2 * n;
-            return;
-        }
-        if (t.fl & MOVED) return;
-        const int32_t start = t.sc;
-        int32_t rem = t.sc;
-        const int bid = T.id(x, y + 1);
-        const int bT = mt_type(ma[bid]);
-        const bool airBelow = bT == T_AIR;
-        if ((airBelow && c.iter <= 2) || bid == (int)t.id) {
-            int32_t dst = (bT == T_SOUP) ? T.sc(x, y + 1) : 0;
-            soup_flow(T, c, t, rem, clampflow(vflow(start, dst) - dst, start), bT, x, y, 0, 1);
-        } else if (c.iter == 0 && bT == T_SOUP && bid != (int)t.id) {
-            if (c.D() % 10 == 0) {
-                t.df += T.df_load(x, y);  // the cell leaves its position: carry the whole diff
-                const int16_t tv = T.tp_load(x, y);
-                T.move(x, y, x, y + 1);
-                T.put(x, y + 1, t);
-                T.tp_store(x, y + 1, tv);
-                return;
-            }
-        }
-        if (rem < Q_MINV) {
-            t.df -= rem;
-            led_add(c, LED_DF, t.id, rem);
-            T.put_delta(x, y, t);
-            return;
-        }
-        const int lid = T.id(x - 1, y);
-        const int lT = mt_type(ma[lid]);
-        const bool canL = (lT == T_AIR || lid == (int)t.id) && !airBelow;
-        const int rid = T.id(x + 1, y);
-        const int rT = mt_type(ma[rid]);
-        const bool canR = (rT == T_AIR || rid == (int)t.id) && !airBelow;
-        if (canL) {
-            int32_t dst = (lT == T_SOUP) ? T.sc(x - 1, y) : 0;
-            soup_flow(T, c, t, rem, clampflow(canR ? (rem - dst) / 3 : (rem - dst) / 2, rem), lT, x, y, -1, 0);
-        }
-        if (rem < Q_MINV) {
-            t.df -= rem;
-            led_add(c, LED_DF, t.id, rem);
-            T.put_delta(x, y, t);
-            return;
-        }
-        if (canR) {
-            int32_t dst = (rT == T_SOUP) ? T.sc(x + 1, y) : 0;
-            soup_flow(T, c, t, rem, clampflow((rem - dst) / 2, rem), rT, x, y, 1, 0);
-        }
-        if (rem < Q_MINV) {
-            t.df -= rem;
-            led_add(c, LED_DF, t.id, rem);
-            T.put_delta(x, y, t);
-            return;
-        }
-        const int tid = T.id(x, y - 1);
-        const int tT = mt_type(ma[tid]);
-        if (tT == T_AIR || tid == (int)t.id) {
-            int32_t dst = (tT == T_SOUP) ? T.sc(x, y - 1) : 0;
-            soup_flow(T, c, t, rem, clampflow(rem - vflow(rem, dst), rem), tT, x, y, 0, -1);
-        } else if (c.iter == 0 && tT == T_SOUP && tid != (int)t.id) {
-            if (c.D() % 10 == 0) {
-                t.df += T.df_load(x, y);
-                const int16_t tv = T.tp_load(x, y);
-                T.move(x, y, x, y - 1);
-                T.put(x, y - 1, t);
-                T.tp_store(x, y - 1, tv);
-                return;
-            }
-        }
-        if (rem < Q_MINV) {
-            t.df -= rem;
-            led_add(c, LED_DF, t.id, rem);
-            T.put_delta(x, y, t);
-            return;
-        }
-        if (start == rem) {  // world.cpp:1472-1483
-            uint8_t s = t.fl & SETTLE_MASK;
-            if (s < SETTLE_MASK) s++;
-            t.fl = (uint8_t)((t.fl & ~SETTLE_MASK) | s);
-            if (s >= 10) t.fl |= MOVED;
-        } else {
-            if (tT == T_SOUP) T.set_moved(x, y - 1, false);
-            if (bT == T_SOUP) T.set_moved(x, y + 1, false);
-            if (lT == T_SOUP) T.set_moved(x - 1, y, false);
-            if (rT == T_SOUP) T.set_moved(x + 1, y, false);
-        }
-        T.put_delta(x, y, t);
-        // WATER on LAVA, world.cpp:1519-1537
-        if ((int)t.id == c.id_water && T.id(x, y + 1) == c.id_lava) {
-            Cell st = create_tile(c, c.id_steam);
-            led_swap(c, t.id, (long long)t.sc + T.df_load(x, y), st.id, (long long)st.sc);
-            T.put_new(x, y, st, mt);
-            Cell ob = create_tile(c, c.id_obsidian);
-            led_replace_at(T, c, x, y + 1, ob);
-            T.put_new(x, y + 1, ob, mt);
-            T.setvis(x, y + 1);
-            for (int xx = -1; xx <= 1; xx++)
-                for (int yy = 0; yy <= 2; yy++) {
-                    if (T.id(x + xx, y + yy) == c.id_lava) {
-                        Cell o2 = create_tile(c, c.id_obsidian);
-                        led_replace_at(T, c, x + xx, y + yy, o2);
-                        T.put_new(x + xx, y + yy, o2, mt);
-                        T.setvis(x + xx, y + yy);
-                    }
-                }
-            return;
-        }
-    } else if (type == T_GAS) {  // world.cpp:1569-1585
-        const int above = T.type(x, y - 1);
-        const int aboveL = T.type(x - 1, y - 1);
-        const int aboveR = T.type(x + 1, y - 1);
-        if (above == T_AIR && !((aboveL == T_AIR || aboveR == T_AIR) && c.D() % 2 == 0)) {
-            T.move(x, y, x, y - 1);
-            T.put(x, y - 1, t);
-            T.setvis(x, y - 1);
+    } else if (cw_is(w0, T_SOUP)) {
+        if constexpr (TL::kF32)
+            rule_a_soup_f32(T, c, w0, i, x, y);
+        else
+            rule_a_soup(T, c, w0, i, x, y);
+    } else if (cw_is(w0, T_GAS)) {  // world.cpp:1569-1585
+        const int n = i - T.RW;
+        const uint32_t above = T.at(n), aboveL = T.at(n - 1), aboveR = T.at(n + 1);
+        if (cw_air(above) && !((cw_air(aboveL) || cw_air(aboveR)) && c.D() % 2 == 0)) {
+            const int32_t sc = T.s_sc[i];
+            const uint32_t col = T.s_col[i];
+            // the AIR cell above and the gas trade places
+            T.put_dry(i, above, T.s_sc[n], T.s_col[n]);
+            T.set_word(n, w0 | CW_DIRTY | CW_VIS);
+            T.set_planes(n, sc, col);
         }
     }
 }
 
 // ----------------------------------------------------------------- sweep B
-// dfv: the cell's pending fluid diff, read when the sub-phase began (no other cell
-// of the sub-phase writes it)
+// w0: the cell's word; dfv: a SOUP cell's pending fluid diff, read when the sub-phase
+// began (no other cell of the sub-phase writes it)
 template <class TL>
-__device__ __forceinline__ void rule_b(const TL &T, Ctx &c, int x, int y, int32_t dfv) {
-    if (T.vis(x, y)) return;  // world.cpp:1597
-    const uint32_t *ma = T.ma;
-    const float *md = T.md;
-    const int sid = T.id(x, y);
-    const uint32_t a = ma[sid];
-    const int type = mt_type(a);
-    if (type != T_SAND && type != T_SOUP && type != T_GAS) return;
-    c.at(x, y);
-    if (type == T_SAND) {  // world.cpp:1602-1727
-        const int i = T.li(x, y);
-        const uint8_t fl0 = T.s_fl[i] & (uint8_t)~VISITED;
-        const bool canL = can_sink(ma, md, T.id(x - 1, y + 1), sid);
-        const bool canR = can_sink(ma, md, T.id(x + 1, y + 1), sid);
-        bool stopped = !(fl0 & MOVED);
-        const int slip = mt_slip(a);
+__device__ __forceinline__ void rule_b(const TL &T, Ctx &c, uint32_t w0, int i, int x, int y, int32_t dfv) {
+    if (w0 & CW_VIS) return;  // world.cpp:1597
+    if (cw_is(w0, T_SAND)) {  // world.cpp:1602-1727
+        const int RW = T.RW;
+        const uint32_t lim = cw_sink(w0);
+        const bool canL = T.at(i + RW - 1) < lim;
+        const bool canR = T.at(i + RW + 1) < lim;
+        bool stopped = !(w0 & CW_MOVED);
+        c.at(x, y);
+        const uint32_t a = T.ma[cw_id(w0)];
         if (stopped) {
             // world.cpp:1619-1627 over the AIR snapshot taken when sweep B began
-            const int drop = __popc(T.air10(x - 1, y + 1) | T.air10(x + 1, y + 1));
+            const int drop = __popc(T.air10(i + RW - 1, x - 1, y + 1) | T.air10(i + RW + 1, x + 1, y + 1));
             int d = drop + 1 - mt_stab(a);
             if (d > 0) {
                 int chance = 1000 / d;
                 if (chance < 1000) {
                     if (c.D() % (uint32_t)chance == 0) {
                         stopped = false;
-                        T.set_moved(x, y, true);
+                        T.set_moved_w(i, w0, true);
                     }
                 }
             }
         }
         if (stopped || !(canL || canR)) {
-            T.set_moved(x, y, false);
+            T.set_moved(i, false);
             return;
         }
         // the moving cell as it was when its turn began
-        Cell t;
-        t.id = (uint16_t)sid;
-        t.fl = fl0;
-        t.sc = T.s_sc[i];
-        t.col = T.s_col[i];
-        t.df = 0;
+        uint32_t t = w0;
+        const int g = T.gi(x, y);
+        const int32_t sc = T.s_sc[i];
+        const uint32_t col = T.s_col[i];
+        const int slip = mt_slip(a);
         const bool shouldMove = (slip > 0) ? (c.D() % (uint32_t)(2 * slip) != 0) : true;
         if (shouldMove && (canL || canR)) {
             if (c.D() % 2 == 0) {
-                if (T.type(x, y + 1) == T_SAND) {
-                    if (c.D() % 2 == 0) T.set_moved(x, y + 1, true);
+                if (cw_is(T.at(i + RW), T_SAND)) {
+                    if (c.D() % 2 == 0) T.set_moved(i + RW, true);
                 }
             }
         }
-        if (shouldMove && canL && (!canR || c.D() % 2 == 0)) {
-            if (T.type(x - 1, y) == T_AIR) {
-                T.move(x - 1, y, x - 1, y + 1);
-                T.setvis(x - 1, y);
-                T.set_nothing(x, y);
-            } else {
-                T.move(x, y, x - 1, y + 1);
-                T.setvis(x, y);
-            }
-            if (slip > 0 && c.D() % (uint32_t)(20 * slip) == 0) t.fl &= (uint8_t)~MOVED;
-            T.put(x - 1, y + 1, t);
-            T.setvis(x - 1, y + 1);
-        } else if (shouldMove && canR) {
-            if (T.type(x + 1, y) == T_AIR) {
-                T.move(x + 1, y, x + 1, y + 1);
-                T.set_nothing(x, y);
-            } else {
-                T.move(x, y, x + 1, y + 1);
-                T.setvis(x, y);
-            }
-            if (slip > 0 && c.D() % (uint32_t)(20 * slip) == 0) t.fl &= (uint8_t)~MOVED;
-            T.put(x + 1, y + 1, t);
-            T.setvis(x + 1, y + 1);
+        const bool goL = shouldMove && canL && (!canR || c.D() % 2 == 0);
+        if (!goL && !(shouldMove && canR)) {
+            T.set_moved(i, false);
+            return;
+        }
+        const int o = goL ? -1 : 1;  // towards the left or the right
+        const int s = i + o, d = i + RW + o, gd = g + T.W + o;
+        if (T.air(s)) {
+            T.move(s, g + o, d, gd);
+            if (goL) T.setvis(s);
+            T.set_nothing(i);
         } else {
-            T.set_moved(x, y, false);
+            T.move(i, g, d, gd);
+            T.setvis(i);
         }
-    } else if (TL::kF32 && type == T_SOUP) {  // world.cpp:1728-1745 in f32
-        Cell t = T.get_active(x, y);
-        const float a = __fadd_rn(__int_as_float(t.sc), __int_as_float(dfv));
-        t.sc = __float_as_int(a);
-        t.df = __float_as_int(0.0f);
-        if (a < F_MINV) {
-            led_add(c, LED_DN, t.id, 1);
-            T.set_nothing(x, y);
-            T.setvis(x, y);
+        if (slip > 0 && c.D() % (uint32_t)(20 * slip) == 0) t &= ~CW_MOVED;
+        T.set_word(d, t | CW_DIRTY | CW_VIS);
+        T.set_planes(d, sc, col);
+    } else if (cw_is(w0, T_SOUP)) {  // world.cpp:1728-1745
+        const int g = T.gi(x, y);
+        int32_t a;
+        bool dry;
+        if constexpr (TL::kF32) {
+            const float f = __fadd_rn(__int_as_float(T.s_sc[i]), __int_as_float(dfv));
+            a = __float_as_int(f);
+            dry = f < F_MINV;
         } else {
-            T.put(x, y, t);
-            T.setvis(x, y);
+            a = T.s_sc[i] + dfv;
+            dry = a < Q_MINV;
         }
-    } else if (type == T_SOUP) {  // world.cpp:1728-1745
-        Cell t = T.get_active(x, y);
-        t.sc += dfv;
-        t.df = 0;
-        if (t.sc < Q_MINV) {
-            led_add(c, LED_DN, t.id, 1);
-            led_add(c, LED_DF, t.id, t.sc);
-            T.set_nothing(x, y);
-            T.setvis(x, y);
+        if (dry) {
+            led_add(c, LED_DN, w0, 1);
+            if constexpr (!TL::kF32) led_add64(c, LED_DF, w0, a);
+            T.set_word(i, T.mw[T.id_air] | CW_DIRTY | CW_VIS);
+            T.set_planes(i, 0, 0);
         } else {
-            T.put(x, y, t);
-            T.setvis(x, y);
+            T.set_word(i, w0 | CW_DIRTY | CW_VIS);
+            T.set_sc(i, a);
+            if (dfv != 0) T.df[g] = 0;
         }
-    } else {  // GAS, world.cpp:1799-1818
-        const int aboveL = T.type(x - 1, y - 1);
-        const int aboveR = T.type(x + 1, y - 1);
-        if (aboveL != T_AIR && aboveR != T_AIR) return;
-        const Cell t = T.get_active(x, y);
-        if (aboveL == T_AIR && !(aboveR == T_AIR && c.D() % 2 == 0)) {
-            T.move(x, y, x - 1, y - 1);
-            T.put(x - 1, y - 1, t);
-            T.setvis(x - 1, y - 1);
-        } else if (aboveR == T_AIR) {
-            T.move(x, y, x + 1, y - 1);
-            T.put(x + 1, y - 1, t);
-            T.setvis(x + 1, y - 1);
-        }
+    } else if (cw_is(w0, T_GAS)) {  // world.cpp:1799-1818
+        const int n = i - T.RW;
+        const bool aboveL = T.air(n - 1), aboveR = T.air(n + 1);
+        if (!aboveL && !aboveR) return;
+        c.at(x, y);
+        const int32_t sc = T.s_sc[i];
+        const uint32_t col = T.s_col[i];
+        const bool goL = aboveL && !(aboveR && c.D() % 2 == 0);
+        if (!goL && !aboveR) return;
+        const int d = goL ? n - 1 : n + 1;  // the AIR cell and the gas trade places
+        T.put_dry(i, T.at(d), T.s_sc[d], T.s_col[d]);
+        T.set_word(d, w0 | CW_DIRTY | CW_VIS);
+        T.set_planes(d, sc, col);
     }
 }
 
 // ----------------------------------------------------------------- sweep C
 template <class TL>
-__device__ __forceinline__ void rule_c(const TL &T, Ctx &c, int x, int y) {
-    if (T.vis(x, y)) return;  // world.cpp:1831
-    const int sid = T.id(x, y);
-    if (mt_type(T.ma[sid]) != T_GAS) return;
-    c.at(x, y);
+__device__ __forceinline__ void rule_c(const TL &T, Ctx &c, int i, int x, int y) {
+    const uint32_t w0 = T.at(i);
+    if ((w0 & CW_VIS) || !cw_is(w0, T_GAS)) return;  // world.cpp:1831
     // world.cpp:1862-1889
-    const int l = T.type(x - 1, y);
-    const int r = T.type(x + 1, y);
-    if (l != T_AIR && r != T_AIR && sid != c.id_steam) return;
-    const Cell t = T.get_active(x, y);
-    if (l == T_AIR && !(r == T_AIR && c.D() % 2 == 0)) {
-        T.move(x, y, x - 1, y);
-        T.put(x - 1, y, t);
-        T.setvis(x - 1, y);
-    } else if (r == T_AIR) {
-        T.move(x, y, x + 1, y);
-        T.put(x + 1, y, t);
-        T.setvis(x + 1, y);
-    } else if (sid == c.id_steam) {
+    const bool l = T.air(i - 1), r = T.air(i + 1), steam = cw_id(w0) == c.id_steam;
+    if (!l && !r && !steam) return;
+    c.at(x, y);
+    const bool goL = l && !(r && c.D() % 2 == 0);
+    if (goL || r) {
+        const int d = goL ? i - 1 : i + 1;  // the AIR cell and the gas trade places
+        const int32_t sc = T.s_sc[i];
+        const uint32_t col = T.s_col[i];
+        T.put_dry(i, T.at(d), T.s_sc[d], T.s_col[d]);
+        T.set_word(d, w0 | CW_DIRTY | CW_VIS);
+        T.set_planes(d, sc, col);
+    } else if (steam) {
         if (c.D() % 10 == 0) {
+            const int g = T.gi(x, y);
             Cell wt = create_tile(c, c.id_water);
-            led_swap(c, t.id, 0, wt.id, (long long)wt.sc);
-            T.put_new(x, y, wt, c.mt);
+            led_swap(c, w0, 0, wt.w, (long long)wt.sc);
+            T.put_new(i, g, wt, c.mt);
         }
     }
 }
@@ -1246,19 +1196,19 @@ __device__ __forceinline__ int block_excl_scan(int v, int *scratch, int *total) 
 
 // write the particles of one spawn event (world.cpp:1110-1119,1222,1298)
 template <bool TEMP, bool F32>
-static __device__ __noinline__ void emit_spawns(const WorldDev &w, const SpawnEv &ev, uint32_t cp, uint32_t rank0,
-                                                int base) {
+static __device__ __noinline__ void emit_spawns(const WorldDev &w, const SpawnEv &ev, int n, uint32_t cp,
+                                                uint32_t rank0, int base) {
     int32_t base_amt = 0, extra = 0;
     if (ev.kind == 2) {
         if (F32) {
             // f32 amt = tile.fluidAmount / n for every particle (world.cpp:1292)
-            base_amt = __float_as_int(__fdiv_rn(__int_as_float(ev.sc), (float)ev.n));
+            base_amt = __float_as_int(__fdiv_rn(__int_as_float(ev.sc), (float)n));
         } else {
-            base_amt = ev.sc / ev.n;
-            extra = ev.sc % ev.n;
+            base_amt = ev.sc / n;
+            extra = ev.sc % n;
         }
     }
-    for (int i = 0; i < ev.n; i++) {
+    for (int i = 0; i < n; i++) {
         int slot = base + i;
         if (slot >= w.stage_cap) {
             atomicOr(w.err, ERR_SPAWN_CAP);
@@ -1308,21 +1258,31 @@ static __device__ __noinline__ void emit_spawns(const WorldDev &w, const SpawnEv
 
 // -------------------------------------------------------------- the kernel
 // shared memory besides the tile planes
-template <int NT>
+template <int NT, bool PAIR>
 struct SmemHeadT {
-    uint32_t ma[MAXMAT];
-    float md[MAXMAT];
-    long long led[LED_ROWS * 64];
+    uint32_t ma[MAXMAT];  // material word A
+    uint32_t mw[MAXMAT];  // material -> cell word of this iteration
+    int32_t led[LED_ROWS * 64];   // the chunk-pass's ledger counts
     int scan[40];
-    uint8_t mreact[MAXMAT];
-    int cnt[NT];  // sweep-A spawns per enumeration index, then their ranks
+    int cnt[PAIR ? NT : 1];       // CTA pair: sweep-A spawns per enumeration index
     uint32_t air[(128 + 2) * 5];  // sweep-B pillar snapshot (chunk edge <= 128)
     // CTA pair: what the partner wrote here: [0..1] its chunk flags, [2..3] its spawn
     // count of a sweep-A sub-phase (alternate slots)
     uint32_t xch[4];
     uint32_t vote[32];  // each warp's activity (bit 0) and fire (bit 1) votes of the chunk-pass
 };
-using SmemHead = SmemHeadT<CP_THREADS>;
+
+// Dynamic shared memory of a CTA that updates `own` rows of a chunk of edge C: the
+// head, up to 128 bytes of padding (the planes start on a 128-byte boundary of the
+// window) and the planes of the largest tile
+template <int NT, bool PAIR>
+static size_t tile_smem(int C, int own, int halo, int width) {
+    const size_t RW = (size_t)std::max(width, C + HALO_LO + halo), RHF = (size_t)own + HALO_LO + halo;
+    const size_t RHI = (size_t)own + HALO_LO + 10;
+    const size_t head = (sizeof(SmemHeadT<NT, PAIR>) + 127) & ~(size_t)127;
+    const size_t plane = (RW * RHF + 31) & ~(size_t)31;
+    return 128 + head + (2 * plane + RW * RHI) * 4;
+}
 
 // items: (world << 20) | chunk slot within the colour; iter, tk select the pass.
 // FUSED: every pass of the tick in one launch (iter, tk, items and n_items unused;
@@ -1351,7 +1311,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
     static_assert(!(PAIR && SEQ), "the reference order runs a chunk in one CTA");
     static_assert(!(FUSED && (PAIR || SEQ)), "the fused tick runs partitioned chunk-passes in one CTA each");
     constexpr int T = PAIR ? CP_THREADS / 2 : CP_THREADS;
-    using Head = SmemHeadT<T>;
+    using Head = SmemHeadT<T, PAIR>;
     extern __shared__ __align__(16) unsigned char smem[];
     Head &S = *reinterpret_cast<Head *>(smem);
     // the planes start on a 128-byte boundary of the shared window (TMA destinations)
@@ -1366,11 +1326,8 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
     const int tid = threadIdx.x;
     const int rank = PAIR ? (int)cluster_rank() : 0;
     int npass = 0;  // chunks taken so far (the same count in both CTAs of a pair)
-    for (int i = tid; i < MAXMAT; i += T) {
-        S.ma[i] = (i < mt->n) ? mt->a[i] : 0u;
-        S.md[i] = (i < mt->n) ? mt->density[i] : 0.f;
-        S.mreact[i] = (uint8_t)((i < mt->n) ? mt->n_react[i] : 0);
-    }
+    for (int i = tid; i < MAXMAT; i += T) S.ma[i] = (i < mt->n) ? mt->a[i] : 0u;
+    int mw_iter = -1;  // the iteration S.mw was built for
     for (int i = tid; i < LED_ROWS * 64; i += T) S.led[i] = 0;
     Ctx c;
     SpawnEv ev_store;  // outside the context (see Ctx::ev)
@@ -1378,8 +1335,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
     c.iter = iter_arg;
     c.mt = mt;
     c.led_s = S.led;
-    c.ma = S.ma;
-    c.mreact = S.mreact;
+    c.mw = S.mw;
     c.id_fire = mt->id_fire;
     c.id_water = mt->id_water;
     c.id_lava = mt->id_lava;
@@ -1388,13 +1344,12 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
     // interactions exist exactly when the launch runs the 5-cell halo (tick_halo)
     c.has_inter = HALO == 5;
     c.f32 = F32;
-    const int id_solid = mt->id_solid, id_air = mt->id_air;
+    const int id_air = mt->id_air, id_solid = mt->id_solid;
     if (kTma && tid == 0) mbar_init(&s_tma_bar, 1);
     FSE_PT_DECL
     __syncthreads();
 
     int iter = iter_arg, tk = tk_arg;
-    long long *led_g_last = nullptr;
 
     const int wstart = PAIR ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
     const int wstride = PAIR ? (int)(gridDim.x >> 1) : (int)gridDim.x;
@@ -1459,6 +1414,12 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                 reinterpret_cast<uint2 *>(&s_w)[tid] =
                     __ldg(reinterpret_cast<const uint2 *>(&worlds[item >> 20]) + tid);
         }
+        if (iter != mw_iter) {
+            // the cell words of this iteration's materials
+            mw_iter = iter;
+            for (int i = tid; i < MAXMAT; i += T)
+                S.mw[i] = i < mt->n ? mt->word[i] | (iter < mt_iter(S.ma[i]) ? CW_LIVE : 0u) : (uint32_t)i;
+        }
         __syncthreads();
         FSE_PT(0)
         const WorldDev &w = s_w;
@@ -1498,16 +1459,6 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
             }
             __syncthreads();
         }
-        if (led_g_last != w.ledger && led_g_last != nullptr) {
-            // flush the shared ledger before switching worlds
-            for (int i = tid; i < LED_ROWS * 64; i += T) {
-                long long v = S.led[i];
-                if (v) atomicAdd((unsigned long long *)&led_g_last[(i / 64) * MAXMAT + (i % 64)], (unsigned long long)v);
-                S.led[i] = 0;
-            }
-            __syncthreads();
-        }
-        led_g_last = w.ledger;
         if (iter >= w.cell_iter) {
             __syncthreads();
             continue;
@@ -1524,36 +1475,33 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
         TileData Tl;
         const bool tma = kTma && w.tmap != nullptr;
         // with TMA the rows start on a 16-byte boundary and are tma_tile_width wide
-        Tl.RW = tma ? tma_tile_width(C) : C + 2 * HALO;
-        Tl.RHF = own + 2 * HALO;
-        Tl.RHI = own + HALO + 10;
-        Tl.x0 = tma ? ((cx - HALO) & ~3) : cx - HALO;
-        Tl.y0 = cy + o0 - HALO;
+        Tl.RW = tma ? tma_tile_width(C) : C + HALO_LO + HALO;
+        Tl.RHF = own + HALO_LO + HALO;
+        Tl.RHI = own + HALO_LO + 10;
+        Tl.x0 = tma ? ((cx - HALO_LO) & ~3) : cx - HALO_LO;
+        Tl.y0 = cy + o0 - HALO_LO;
         Tl.W = W;
         Tl.H = H;
         Tl.ma = S.ma;
-        Tl.md = S.md;
+        Tl.mw = S.mw;
         Tl.df = w.df;
         Tl.tp = w.tp;
-        Tl.id_solid = id_solid;
         Tl.id_air = id_air;
         Tl.s_air = S.air;
         Tl.ax0 = cx - 1;
         Tl.ay0 = cy + o0 + 1;
         Tl.aw = C + 2;
-        const int nid = Tl.RW * Tl.RHI, nfull = Tl.RW * Tl.RHF;
+        const int nfull = Tl.RW * Tl.RHF, plane = (nfull + 31) & ~31;  // 128-byte aligned planes
         Tl.s_sc = (int32_t *)planes;
-        Tl.s_col = (uint32_t *)(Tl.s_sc + ((nfull + 31) & ~31));  // 128-byte aligned
-        Tl.s_id = (uint16_t *)(Tl.s_col + nfull);
-        Tl.s_fl = (uint8_t *)(Tl.s_id + ((nid + 1) & ~1));
+        Tl.s_col = (uint32_t *)(Tl.s_sc + plane);
+        Tl.s_w = Tl.s_col + plane;
         if constexpr (PAIR) {
             // the partner's planes lie at the same offsets of its shared memory
             const uint32_t pr = (uint32_t)(rank ^ 1);
-            Tl.p_id = mapa_rank(smem_addr(Tl.s_id), pr);
-            Tl.p_fl = mapa_rank(smem_addr(Tl.s_fl), pr);
+            Tl.p_w = mapa_rank(smem_addr(Tl.s_w), pr);
             Tl.p_sc = mapa_rank(smem_addr(Tl.s_sc), pr);
             Tl.p_col = mapa_rank(smem_addr(Tl.s_col), pr);
-            Tl.py0 = cy + (rank ? 0 : half) - HALO;
+            Tl.pd = (rank ? half : -half) * Tl.RW;
         }
 
         // ---- stage the tile, one warp per row. The 4-byte planes go straight to
@@ -1607,11 +1555,11 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                     const int lx = lane + 32 * k, gx = Tl.x0 + lx;
                     if (lx >= Tl.RW) continue;
                     const int i = r * Tl.RW + lx;
-                    Tl.s_id[i] = v[k];
-                    if (full) Tl.s_fl[i] = f[k];
+                    const uint32_t cw_ = S.mw[v[k] & CW_ID];
+                    Tl.s_w[i] = cw_ | ((uint32_t)(f[k] & (uint8_t)~VISITED) << 8);
                     if (gx >= cx && gx < cx + C && gy >= cy + o0 && gy < cy + o1 && rin && gx < W) {
-                        if (mt_iter(S.ma[v[k]]) > c.iter) active = 1;
-                        if ((int)v[k] == c.id_fire) fire = 1;
+                        if (cw_ & CW_LIVE) active = 1;
+                        if (cw_ & CW_FIRE) fire = 1;
                     }
                 }
             }
@@ -1695,20 +1643,21 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                 for (int t = 0; t < steps; t++) {
                     const int dx = t - s * k;
                     if (row && dx >= 0 && dx < cw) {
-                        const int x = cx + dx, y = cy + dy;
+                        const int x = cx + dx, y = cy + dy, i = Tl.li(x, y);
                         if (sweep == 0) {
-                            c.ev->n = 0;
-                            rule_a(Tl, c, x, y);
-                            if (c.ev->n > 0) {
-                                const int base = atomicAdd(w.stage_count, c.ev->n);
-                                emit_spawns<TEMP, F32>(w, *c.ev, cp * (uint32_t)w.cp_rows + (uint32_t)k, (uint32_t)spawned,
-                                                  base);
-                                spawned += c.ev->n;
+                            c.ev_n = 0;
+                            rule_a(Tl, c, i, x, y);
+                            if (c.ev_n > 0) {
+                                const int base = atomicAdd(w.stage_count, c.ev_n);
+                                emit_spawns<TEMP, F32>(w, *c.ev, c.ev_n, cp * (uint32_t)w.cp_rows + (uint32_t)k,
+                                                       (uint32_t)spawned, base);
+                                spawned += c.ev_n;
                             }
                         } else if (sweep == 1) {
-                            rule_b(Tl, c, x, y, w.df[(size_t)y * W + x]);
+                            const uint32_t w0 = Tl.at(i);
+                            rule_b(Tl, c, w0, i, x, y, cw_is(w0, T_SOUP) ? w.df[Tl.gi(x, y)] : 0);
                         } else {
-                            rule_c(Tl, c, x, y);
+                            rule_c(Tl, c, i, x, y);
                         }
                     }
                     __syncthreads();
@@ -1721,17 +1670,15 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
             c.pk = pass_key(w.seed, *w.tick, (uint32_t)(c.iter * 3 + sweep));
             if (sweep == 1) {
                 // AIR snapshot for the friction pillar: columns cx-1..cx+C, rows cy+1..cy+C+9
+                // (consecutive threads take consecutive columns, which lie in different banks)
                 for (int task = tid; task < (C + 2) * 5; task += T) {
-                    const int sx = task / 5, wi = task - sx * 5;
+                    const int wi = task / (C + 2), sx = task - wi * (C + 2);
+                    const int rows = min(32, own + 9 - wi * 32);
+                    int i = Tl.li(cx - 1 + sx, Tl.ay0 + wi * 32);
                     uint32_t bits = 0;
-                    for (int b = 0; b < 32; b++) {
-                        const int sy = wi * 32 + b;
-                        if (sy < own + 9) {
-                            const int gx = cx - 1 + sx, gy = Tl.ay0 + sy;
-                            if (Tl.inw(gx, gy) && Tl.type(gx, gy) == T_AIR) bits |= 1u << b;
-                        }
-                    }
-                    S.air[task] = bits;
+                    for (int b = 0; b < rows; b++, i += Tl.RW)
+                        if (Tl.air(i)) bits |= 1u << b;
+                    S.air[sx * 5 + wi] = bits;
                 }
                 __syncthreads();
             }
@@ -1749,25 +1696,24 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                         // sweep A sub-phases have at most 43 x 22 <= T cells: one per thread,
                         // so every spawn event stays in its thread until it is ranked
                         const int e = tid;
-                        c.ev->n = 0;
-                        S.cnt[tid] = 0;
+                        c.ev_n = 0;
                         if (e < total) {
                             int q, r;
                             divmod_small(e, nx, rnx, q, r);
                             const int dy = dyb + q * py, dx = rx + r * px;
-                            if (dx < cw && dy < chh) rule_a(Tl, c, cx + dx, cy + dy);
+                            if (dx < cw && dy < chh) rule_a(Tl, c, Tl.li(cx + dx, cy + dy), cx + dx, cy + dy);
                         }
                         FSE_PT(3)
-                        // rank spawned particles in enumeration order. S.cnt[e] and the scan
-                        // scratch are next written after the next sub-phase's barrier, so no
-                        // barrier is needed after this block.
-                        if (c.ev->n > 0) S.cnt[e] = c.ev->n;
+                        // rank spawned particles in enumeration order. The scan scratch is
+                        // next written after the next sub-phase's barrier, so no barrier is
+                        // needed after this block.
                         if constexpr (PAIR) {
+                            S.cnt[tid] = c.ev_n;
                             // the sub-phase's enumeration runs through rank 0's rows first:
                             // each CTA ranks its own spawns, the partner's count of the
                             // sub-phase comes through the cluster barrier that ends it
                             int tot = 0, ex = 0;
-                            if (__syncthreads_or(c.ev->n > 0)) ex = block_excl_scan(S.cnt[tid], S.scan, &tot);
+                            if (__syncthreads_or(c.ev_n > 0)) ex = block_excl_scan(S.cnt[tid], S.scan, &tot);
                             const int slot_t = 2 + (nsub & 1);
                             if (tid == 0)
                                 st_cluster_u32(mapa_rank(smem_addr(&S.xch[slot_t]), (uint32_t)(rank ^ 1)),
@@ -1775,19 +1721,19 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                             cluster_sync();
                             const int tot_p = (int)S.xch[slot_t];
                             nsub++;
-                            if (c.ev->n > 0) {
-                                const int base = atomicAdd(w.stage_count, c.ev->n);
-                                emit_spawns<TEMP, F32>(w, *c.ev, cp, (uint32_t)(running + (rank ? tot_p : 0) + ex),
-                                                       base);
+                            if (c.ev_n > 0) {
+                                const int base = atomicAdd(w.stage_count, c.ev_n);
+                                emit_spawns<TEMP, F32>(w, *c.ev, c.ev_n, cp,
+                                                       (uint32_t)(running + (rank ? tot_p : 0) + ex), base);
                             }
                             running += tot + tot_p;
-                        } else if (__syncthreads_or(c.ev->n > 0)) {
+                        } else if (__syncthreads_or(c.ev_n > 0)) {
                             // ranks with one more barrier: each warp's total in shared
                             // memory, a thread's rank the totals of the warps before it plus
                             // its lanes' prefix (the scratch is next written after the next
                             // sub-phase's barrier)
                             const int lane = tid & 31, wid = tid >> 5;
-                            int inc = c.ev->n;
+                            int inc = c.ev_n;
 #pragma unroll
                             for (int o = 1; o < 32; o <<= 1) {
                                 const int t = __shfl_up_sync(0xffffffffu, inc, o);
@@ -1798,12 +1744,12 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                             const int ws = lane < T / 32 ? S.scan[lane] : 0;
                             const int tot = (int)__reduce_add_sync(0xffffffffu, (unsigned)ws);
                             const int ex = (int)__reduce_add_sync(0xffffffffu, lane < wid ? (unsigned)ws : 0u) + inc -
-                                           c.ev->n;
-                            if (c.ev->n > 0) {
+                                           c.ev_n;
+                            if (c.ev_n > 0) {
                                 // staging slots are taken in any order; the (chunk-pass, rank)
                                 // key orders the particles later
-                                const int base = atomicAdd(w.stage_count, c.ev->n);
-                                emit_spawns<TEMP, F32>(w, *c.ev, cp, (uint32_t)(running + ex), base);
+                                const int base = atomicAdd(w.stage_count, c.ev_n);
+                                emit_spawns<TEMP, F32>(w, *c.ev, c.ev_n, cp, (uint32_t)(running + ex), base);
                             }
                             running += tot;
                         }
@@ -1824,14 +1770,16 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                             const int dy1 = dyb + q1 * py, dx1 = rx + r1 * px;
                             const bool v0 = tid < total && dx0 < cw && dy0 < chh;
                             const bool v1 = tid + T < total && dx1 < cw && dy1 < chh;
-                            const int32_t df0 = v0 ? w.df[(size_t)(cy + dy0) * W + cx + dx0] : 0;
-                            const int32_t df1 = v1 ? w.df[(size_t)(cy + dy1) * W + cx + dx1] : 0;
-                            if (v0) rule_b(Tl, c, cx + dx0, cy + dy0, df0);
-                            if (v1) rule_b(Tl, c, cx + dx1, cy + dy1, df1);
+                            const int i0 = Tl.li(cx + dx0, cy + dy0), i1 = Tl.li(cx + dx1, cy + dy1);
+                            const uint32_t w0 = v0 ? Tl.at(i0) : CW_VIS, w1 = v1 ? Tl.at(i1) : CW_VIS;
+                            const int32_t df0 = cw_is(w0, T_SOUP) ? w.df[Tl.gi(cx + dx0, cy + dy0)] : 0;
+                            const int32_t df1 = cw_is(w1, T_SOUP) ? w.df[Tl.gi(cx + dx1, cy + dy1)] : 0;
+                            rule_b(Tl, c, w0, i0, cx + dx0, cy + dy0, df0);
+                            rule_b(Tl, c, w1, i1, cx + dx1, cy + dy1, df1);
                         } else {
                             for (int e = tid; e < total; e += T) {
                                 const int dy = dyb + q * py, dx = rx + r * px;
-                                if (dx < cw && dy < chh) rule_c(Tl, c, cx + dx, cy + dy);
+                                if (dx < cw && dy < chh) rule_c(Tl, c, Tl.li(cx + dx, cy + dy), cx + dx, cy + dy);
                                 q += dq;
                                 r += dr;
                                 if (r >= nx) {
@@ -1851,16 +1799,10 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
             }
         }
         };
-        // One instantiation of the sweeps for every chunk (a second one for the chunks
-        // at the world edge doubles the register pressure of the kernel, whose spills
-        // cost more than the checks they would save): the tile holds GENERIC_SOLID
-        // outside the world, which is what world.cpp:999-1002 reads there, and the only
-        // writes that can reach such cells (fire and interactions) check the world
-        // bounds themselves.
         if constexpr (SEQ)
-            sweeps_seq(Tile<false, TEMP, true, F32>(Tl));
+            sweeps_seq(Tile<TEMP, true, F32>(Tl));
         else
-            sweeps(Tile<false, TEMP, false, F32, PAIR>(Tl));
+            sweeps(Tile<TEMP, false, F32, PAIR>(Tl));
 
         // ---- write back the cells this CTA changed (full-state rows inside the world),
         // one warp per row
@@ -1878,10 +1820,10 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                     const int lx = lane + 32 * k, gx = Tl.x0 + lx;
                     if (lx >= Tl.RW || (unsigned)gx >= (unsigned)W) continue;
                     const int i = r * Tl.RW + lx;
-                    const uint16_t v = Tl.s_id[i];
-                    if (!(v & DIRTY)) continue;
-                    w.id[gb + gx] = (uint16_t)(v & 0x7FFF);
-                    w.fl[gb + gx] = (uint8_t)(Tl.s_fl[i] & (uint8_t)~VISITED);
+                    const uint32_t v = Tl.s_w[i];
+                    if (!(v & CW_DIRTY)) continue;
+                    w.id[gb + gx] = (uint16_t)cw_id(v);
+                    w.fl[gb + gx] = (uint8_t)((v & (CW_FLAGS & ~CW_VIS)) >> 8);
                     w.sc[gb + gx] = Tl.s_sc[i];
                     w.col[gb + gx] = Tl.s_col[i];
                     if (w.dirty) w.dirty[gb + gx] = 1;
@@ -1889,15 +1831,15 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
             }
         }
         if (!SEQ && tid == 0 && rank == 0) w.cp_count[cp] = running;
+        // the chunk-pass's ledger counts (the sweeps ended with a barrier)
+        for (int i = tid; i < LED_ROWS * 64; i += T) {
+            const int32_t v = S.led[i];
+            if (v == 0) continue;
+            S.led[i] = 0;
+            atomicAdd((unsigned long long *)&w.ledger[(i / 64) * MAXMAT + (i % 64)], (unsigned long long)(long long)v);
+        }
         __syncthreads();
         FSE_PT(9)
-    }
-    if (led_g_last) {
-        __syncthreads();
-        for (int i = tid; i < LED_ROWS * 64; i += T) {
-            long long v = S.led[i];
-            if (v) atomicAdd((unsigned long long *)&led_g_last[(i / 64) * MAXMAT + (i % 64)], (unsigned long long)v);
-        }
     }
     // a CTA of a pair leaves only when its partner no longer writes to it
     if constexpr (PAIR) cluster_sync();
@@ -1930,13 +1872,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
     !defined(FSE_TICK_PAIR_TU) && !defined(FSE_TICK_FUSED_TU)
 size_t colour_pass_smem(int C, int halo) {
     // a 2-cell halo leaves room for the TMA-staged tile's wider rows
-    size_t RW = (size_t)C + 2 * halo;
-    if (halo == 2) RW = std::max(RW, (size_t)tma_tile_width(C));
-    size_t RHF = (size_t)C + 2 * halo, RHI = (size_t)C + halo + 10;
-    size_t nid = RW * RHI, nfull = RW * RHF;
-    // the planes start on a 128-byte boundary of the window: up to 128 bytes of padding
-    size_t head = (sizeof(SmemHead) + 127) & ~(size_t)127;
-    return 128 + head + ((nfull + 31) & ~(size_t)31) * 4 + nfull * 4 + ((nid + 1) & ~(size_t)1) * 2 + nfull;
+    return tile_smem<CP_THREADS, false>(C, C, halo, halo == 2 ? tma_tile_width(C) : 0);
 }
 
 #endif
@@ -1971,13 +1907,7 @@ static cudaError_t launch_fused_t(const WorldDev *worlds, const FusedTick &ft, c
 }
 
 // shared memory of one CTA of a pair: half the chunk's rows plus the reach of its rules
-static size_t colour_pass_smem_pair(int C, int halo) {
-    const size_t own = (size_t)C / 2;
-    size_t RW = (size_t)C + 2 * halo, RHF = own + 2 * halo, RHI = own + halo + 10;
-    size_t nid = RW * RHI, nfull = RW * RHF;
-    size_t head = (sizeof(SmemHeadT<CP_THREADS / 2>) + 127) & ~(size_t)127;
-    return 128 + head + ((nfull + 31) & ~(size_t)31) * 4 + nfull * 4 + ((nid + 1) & ~(size_t)1) * 2 + nfull;
-}
+static size_t colour_pass_smem_pair(int C, int halo) { return tile_smem<CP_THREADS / 2, true>(C, C / 2, halo, 0); }
 
 // the chunks split over CTA pairs (thread-block clusters of two): `clusters` pairs
 template <int HALO, bool TEMP, bool F32>
