@@ -153,7 +153,6 @@ struct TileData {
     int32_t *s_sc;
     uint32_t *s_col;
     const uint32_t *mw;  // material id -> word of a new cell (flags clear)
-    const uint32_t *ma;  // material word A in shared memory
     int32_t *df;         // HBM diff plane
     int16_t *tp;         // HBM temperature plane of SOUP cells (NULL: not kept)
     int x0, y0, RW, RHF, RHI;
@@ -947,6 +946,34 @@ __device__ __forceinline__ bool rule_a_react(const TL &T, Ctx &c, uint32_t w0, i
 }
 
 // ----------------------------------------------------------------- sweep A
+// Whether sweep A may change cell i (a superset of the cells that its rule changes):
+// 0 no, 1 a liquid, 2 another cell. Cells whose material is not updated in this
+// iteration are marked visited here (world.cpp:1093-1096).
+template <class TL>
+__device__ __forceinline__ int class_a(const TL &T, const Ctx &c, int i) {
+    const uint32_t w0 = T.at(i);
+    if (w0 & CW_VIS) return 0;
+    if (!(w0 & CW_LIVE)) {
+        T.set_word(i, w0 | CW_VIS);
+        return 0;
+    }
+    const uint32_t wn = T.at(cw_is(w0, T_GAS) ? i - T.RW : i + T.RW);
+    if (cw_is(w0, T_SOUP)) {
+        const int32_t sc = T.s_sc[i];
+        // a settled liquid only falls or dries up
+        bool small;
+        if constexpr (TL::kF32)
+            small = __int_as_float(sc) < F_MINV;
+        else
+            small = sc < Q_MINV;
+        return sc != 0 && (!(w0 & CW_MOVED) || cw_air(wn) || small) ? 1 : 0;
+    }
+    bool act = (w0 & CW_FIRE) != 0;
+    if (cw_is(w0, T_SAND)) act = c.has_inter || (w0 & CW_REACT) || wn < cw_sink(w0);
+    if (cw_is(w0, T_GAS)) act = cw_air(wn);
+    return act ? 2 : 0;
+}
+
 // c.ev_n: the particles the cell emits (its event in *c.ev)
 template <class TL>
 __device__ __forceinline__ void rule_a(const TL &T, Ctx &c, int i, int x, int y) {
@@ -1014,11 +1041,51 @@ __device__ __forceinline__ void rule_a(const TL &T, Ctx &c, int i, int x, int y)
 }
 
 // ----------------------------------------------------------------- sweep B
-// w0: the cell's word; dfv: a SOUP cell's pending fluid diff, read when the sub-phase
-// began (no other cell of the sub-phase writes it)
+// a liquid takes its pending diff, world.cpp:1728-1745. w0: the cell's word; dfv: its
+// pending diff, read when the sub-phase began (no other cell of the sub-phase writes it)
 template <class TL>
-__device__ __forceinline__ void rule_b(const TL &T, Ctx &c, uint32_t w0, int i, int x, int y, int32_t dfv) {
-    if (w0 & CW_VIS) return;  // world.cpp:1597
+__device__ __forceinline__ void rule_b_soup(const TL &T, Ctx &c, uint32_t w0, int i, int g, int32_t dfv) {
+    int32_t a;
+    bool dry;
+    if constexpr (TL::kF32) {
+        const float f = __fadd_rn(__int_as_float(T.s_sc[i]), __int_as_float(dfv));
+        a = __float_as_int(f);
+        dry = f < F_MINV;
+    } else {
+        a = T.s_sc[i] + dfv;
+        dry = a < Q_MINV;
+    }
+    if (dry) {
+        led_add(c, LED_DN, w0, 1);
+        if constexpr (!TL::kF32) led_add64(c, LED_DF, w0, a);
+        T.set_word(i, T.mw[T.id_air] | CW_DIRTY | CW_VIS);
+        T.set_planes(i, 0, 0);
+    } else {
+        T.set_word(i, w0 | CW_DIRTY | CW_VIS);
+        T.set_sc(i, a);
+        if (dfv != 0) T.df[g] = 0;
+    }
+}
+
+// Whether sweep B may move cell i of word w0 (not SOUP; a superset). Sand that nothing
+// beside it lets slide only clears its moved flag, which happens here: the friction
+// draw of a stopped one could set the flag, but it is cleared again before the turn
+// ends, and leaves only the mark that the cell was written, which rendering worlds
+// (render: they count the written cells) keep exactly.
+template <class TL>
+__device__ __forceinline__ bool class_b(const TL &T, uint32_t w0, int i, bool render) {
+    const bool sand = cw_is(w0, T_SAND);
+    if (!sand && !cw_is(w0, T_GAS)) return false;
+    const int n = sand ? i + T.RW : i - T.RW;
+    const uint32_t lim = sand ? cw_sink(w0) : 1u << 24;  // gas rises into AIR
+    const bool slides = T.at(n - 1) < lim || T.at(n + 1) < lim;
+    if (sand && !slides && !render) T.set_moved_w(i, w0, false);
+    return slides || (sand && render);
+}
+
+// w0: the cell's word (sand or gas)
+template <class TL>
+__device__ __forceinline__ void rule_b(const TL &T, Ctx &c, uint32_t w0, int i, int x, int y) {
     if (cw_is(w0, T_SAND)) {  // world.cpp:1602-1727
         const int RW = T.RW;
         const uint32_t lim = cw_sink(w0);
@@ -1026,7 +1093,7 @@ __device__ __forceinline__ void rule_b(const TL &T, Ctx &c, uint32_t w0, int i, 
         const bool canR = T.at(i + RW + 1) < lim;
         bool stopped = !(w0 & CW_MOVED);
         c.at(x, y);
-        const uint32_t a = T.ma[cw_id(w0)];
+        const uint32_t a = __ldg(&c.mt->a[cw_id(w0)]);
         if (stopped) {
             // world.cpp:1619-1627 over the AIR snapshot taken when sweep B began
             const int drop = __popc(T.air10(i + RW - 1, x - 1, y + 1) | T.air10(i + RW + 1, x + 1, y + 1));
@@ -1077,28 +1144,6 @@ __device__ __forceinline__ void rule_b(const TL &T, Ctx &c, uint32_t w0, int i, 
         if (slip > 0 && c.D() % (uint32_t)(20 * slip) == 0) t &= ~CW_MOVED;
         T.set_word(d, t | CW_DIRTY | CW_VIS);
         T.set_planes(d, sc, col);
-    } else if (cw_is(w0, T_SOUP)) {  // world.cpp:1728-1745
-        const int g = T.gi(x, y);
-        int32_t a;
-        bool dry;
-        if constexpr (TL::kF32) {
-            const float f = __fadd_rn(__int_as_float(T.s_sc[i]), __int_as_float(dfv));
-            a = __float_as_int(f);
-            dry = f < F_MINV;
-        } else {
-            a = T.s_sc[i] + dfv;
-            dry = a < Q_MINV;
-        }
-        if (dry) {
-            led_add(c, LED_DN, w0, 1);
-            if constexpr (!TL::kF32) led_add64(c, LED_DF, w0, a);
-            T.set_word(i, T.mw[T.id_air] | CW_DIRTY | CW_VIS);
-            T.set_planes(i, 0, 0);
-        } else {
-            T.set_word(i, w0 | CW_DIRTY | CW_VIS);
-            T.set_sc(i, a);
-            if (dfv != 0) T.df[g] = 0;
-        }
     } else if (cw_is(w0, T_GAS)) {  // world.cpp:1799-1818
         const int n = i - T.RW;
         const bool aboveL = T.air(n - 1), aboveR = T.air(n + 1);
@@ -1166,34 +1211,6 @@ __device__ __forceinline__ void lattice(int sweep, int mode, int &px, int &py) {
     }
 }
 
-// block-wide exclusive scan of one int per thread; returns the exclusive prefix,
-// *total = block sum. scratch: >= 33 ints of shared memory.
-__device__ __forceinline__ int block_excl_scan(int v, int *scratch, int *total) {
-    int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-    int inc = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        int n = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += n;
-    }
-    if (lane == 31) scratch[wid] = inc;
-    __syncthreads();
-    if (wid == 0) {
-        int s = (lane < nw) ? scratch[lane] : 0;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            int n = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane >= o) s += n;
-        }
-        if (lane < nw) scratch[lane] = s;  // inclusive warp totals
-    }
-    __syncthreads();
-    int before = (wid > 0) ? scratch[wid - 1] : 0;
-    *total = scratch[nw - 1];
-    __syncthreads();
-    return before + inc - v;
-}
-
 // write the particles of one spawn event (world.cpp:1110-1119,1222,1298)
 template <bool TEMP, bool F32>
 static __device__ __noinline__ void emit_spawns(const WorldDev &w, const SpawnEv &ev, int n, uint32_t cp,
@@ -1258,14 +1275,24 @@ static __device__ __noinline__ void emit_spawns(const WorldDev &w, const SpawnEv
 
 // -------------------------------------------------------------- the kernel
 // shared memory besides the tile planes
-template <int NT, bool PAIR>
+template <int NT>
 struct SmemHeadT {
-    uint32_t ma[MAXMAT];  // material word A
     uint32_t mw[MAXMAT];  // material -> cell word of this iteration
     int32_t led[LED_ROWS * 64];   // the chunk-pass's ledger counts
-    int scan[40];
-    int cnt[PAIR ? NT : 1];       // CTA pair: sweep-A spawns per enumeration index
-    uint32_t air[(128 + 2) * 5];  // sweep-B pillar snapshot (chunk edge <= 128)
+    int scan[32];
+    // sweep A: the spawn counts of a sub-phase by enumeration index (zero between
+    // sub-phases); sweep B: the pillar snapshot (chunk edge <= 128)
+    union {
+        uint16_t cnt[NT];
+        uint32_t air[(128 + 2) * 5];
+    };
+    // the cells of a sub-phase that a rule may change (dx | dy << 8); after a sweep-A
+    // sub-phase that spawned, the ranks of its spawns by enumeration index
+    union {
+        uint16_t list[2 * NT];
+        uint32_t rank[NT];
+    };
+    uint32_t n_list[3];  // lengths of the lists of this sub-phase and of the next two, in turn
     // CTA pair: what the partner wrote here: [0..1] its chunk flags, [2..3] its spawn
     // count of a sweep-A sub-phase (alternate slots)
     uint32_t xch[4];
@@ -1275,11 +1302,11 @@ struct SmemHeadT {
 // Dynamic shared memory of a CTA that updates `own` rows of a chunk of edge C: the
 // head, up to 128 bytes of padding (the planes start on a 128-byte boundary of the
 // window) and the planes of the largest tile
-template <int NT, bool PAIR>
+template <int NT>
 static size_t tile_smem(int C, int own, int halo, int width) {
     const size_t RW = (size_t)std::max(width, C + HALO_LO + halo), RHF = (size_t)own + HALO_LO + halo;
     const size_t RHI = (size_t)own + HALO_LO + 10;
-    const size_t head = (sizeof(SmemHeadT<NT, PAIR>) + 127) & ~(size_t)127;
+    const size_t head = (sizeof(SmemHeadT<NT>) + 127) & ~(size_t)127;
     const size_t plane = (RW * RHF + 31) & ~(size_t)31;
     return 128 + head + (2 * plane + RW * RHI) * 4;
 }
@@ -1311,7 +1338,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
     static_assert(!(PAIR && SEQ), "the reference order runs a chunk in one CTA");
     static_assert(!(FUSED && (PAIR || SEQ)), "the fused tick runs partitioned chunk-passes in one CTA each");
     constexpr int T = PAIR ? CP_THREADS / 2 : CP_THREADS;
-    using Head = SmemHeadT<T, PAIR>;
+    using Head = SmemHeadT<T>;
     extern __shared__ __align__(16) unsigned char smem[];
     Head &S = *reinterpret_cast<Head *>(smem);
     // the planes start on a 128-byte boundary of the shared window (TMA destinations)
@@ -1326,9 +1353,10 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
     const int tid = threadIdx.x;
     const int rank = PAIR ? (int)cluster_rank() : 0;
     int npass = 0;  // chunks taken so far (the same count in both CTAs of a pair)
-    for (int i = tid; i < MAXMAT; i += T) S.ma[i] = (i < mt->n) ? mt->a[i] : 0u;
     int mw_iter = -1;  // the iteration S.mw was built for
     for (int i = tid; i < LED_ROWS * 64; i += T) S.led[i] = 0;
+    if (tid < 3) S.n_list[tid] = 0;
+    int nsub = 0;  // the list count of the next sub-phase of sweeps A and B
     Ctx c;
     SpawnEv ev_store;  // outside the context (see Ctx::ev)
     c.ev = &ev_store;
@@ -1418,7 +1446,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
             // the cell words of this iteration's materials
             mw_iter = iter;
             for (int i = tid; i < MAXMAT; i += T)
-                S.mw[i] = i < mt->n ? mt->word[i] | (iter < mt_iter(S.ma[i]) ? CW_LIVE : 0u) : (uint32_t)i;
+                S.mw[i] = i < mt->n ? mt->word[i] | (iter < mt_iter(mt->a[i]) ? CW_LIVE : 0u) : (uint32_t)i;
         }
         __syncthreads();
         FSE_PT(0)
@@ -1482,7 +1510,6 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
         Tl.y0 = cy + o0 - HALO_LO;
         Tl.W = W;
         Tl.H = H;
-        Tl.ma = S.ma;
         Tl.mw = S.mw;
         Tl.df = w.df;
         Tl.tp = w.tp;
@@ -1503,6 +1530,8 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
             Tl.p_col = mapa_rank(smem_addr(Tl.s_col), pr);
             Tl.pd = (rank ? half : -half) * Tl.RW;
         }
+
+        S.cnt[tid] = 0;
 
         // ---- stage the tile, one warp per row. The 4-byte planes go straight to
         // shared memory, as two tensor copies (TMA) or with cp.async; ids and flags
@@ -1622,7 +1651,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
         const int mode = c.has_inter ? 2 : (fire ? 1 : 0);
         const int cw = min(C, W - cx), chh = min(C, H - cy);
         int running = 0;  // spawns emitted so far by this chunk-pass
-        int nsub = 0;     // sweep-A sub-phases so far (CTA pair: alternate exchange slots)
+        int nsub_a = 0;   // CTA pair: the exchange slot of the sweep-A sub-phase
         c.led_g = w.ledger;
         // The reference's order as a wavefront: thread k updates chunk row k counted
         // from the bottom (the row world.cpp's loop takes k-th), cell dx at step
@@ -1655,7 +1684,12 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                             }
                         } else if (sweep == 1) {
                             const uint32_t w0 = Tl.at(i);
-                            rule_b(Tl, c, w0, i, x, y, cw_is(w0, T_SOUP) ? w.df[Tl.gi(x, y)] : 0);
+                            if (w0 & CW_VIS) {  // world.cpp:1597
+                            } else if (cw_is(w0, T_SOUP)) {
+                                rule_b_soup(Tl, c, w0, i, Tl.gi(x, y), w.df[Tl.gi(x, y)]);
+                            } else {
+                                rule_b(Tl, c, w0, i, x, y);
+                            }
                         } else {
                             rule_c(Tl, c, i, x, y);
                         }
@@ -1684,56 +1718,71 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
             }
             int px, py;
             lattice(sweep, mode, px, py);
+            // A sub-phase's cells are enumerated row by row, nxm to a row for every one of
+            // its columns (the last may lie beyond the chunk), so that the threads keep
+            // their places in the lattice for the whole sweep.
+            const int nxm = (C + px - 1) / px;
+            int q, r, dq, dr;
+            divmod_small(tid, nxm, __frcp_rn((float)nxm), q, r);
+            divmod_small(T, nxm, __frcp_rn((float)nxm), dq, dr);
+            const int q1 = q + dq + (r + dr >= nxm ? 1 : 0);  // and of index tid + T
+            const int r1 = r + dr - (r + dr >= nxm ? nxm : 0);
             for (int ry = py - 1; ry >= 0; ry--) {
                 // this CTA's rows of the sub-phase: dyb, dyb + py, ... below o1
                 const int dyb = ry + (o0 > ry ? (o0 - ry + py - 1) / py * py : 0);
-                const int ny = dyb < o1 ? (o1 - dyb + py - 1) / py : 0;
+                const int yend = min(o1, chh);
                 for (int rx = 0; rx < px; rx++) {
-                    const int nx = (C - rx + px - 1) / px;
-                    const int total = nx * ny;
-                    const float rnx = __frcp_rn((float)nx);
+                    const int dx = rx + r * px, dy = dyb + q * py;
+                    const bool v0 = dx < cw && dy < yend;
                     if (sweep == 0) {
-                        // sweep A sub-phases have at most 43 x 22 <= T cells: one per thread,
-                        // so every spawn event stays in its thread until it is ranked
-                        const int e = tid;
+                        // at most 43 x 22 <= T cells: one per thread
+                        const int cls = v0 ? class_a(Tl, c, Tl.li(cx + dx, cy + dy)) : 0;
+                        const unsigned ml = __ballot_sync(0xffffffffu, cls == 1);
+                        const unsigned mo = __ballot_sync(0xffffffffu, cls == 2);
+                        if (ml | mo) {
+                            const int lane = tid & 31;
+                            const unsigned lt = (1u << lane) - 1u;
+                            unsigned at = 0;
+                            if (lane == 0)
+                                at = atomicAdd(&S.n_list[nsub], (unsigned)__popc(ml) | ((unsigned)__popc(mo) << 16));
+                            at = __shfl_sync(0xffffffffu, at, 0);
+                            const uint16_t item = (uint16_t)(dx | (dy << 8));
+                            if (cls == 1) S.list[(at & 0xFFFF) + __popc(ml & lt)] = item;
+                            if (cls == 2) S.list[T - 1 - (at >> 16) - __popc(mo & lt)] = item;
+                        }
+                        __syncthreads();
+                        const unsigned nl = S.n_list[nsub];
+                        const int nnext = nsub == 2 ? 0 : nsub + 1;
+                        // last read before this sub-phase's barrier, next used after the next one's
+                        if (tid == 0) S.n_list[nnext == 2 ? 0 : nnext + 1] = 0;
+                        nsub = nnext;
+                        if constexpr (!PAIR) {
+                            if (nl == 0) continue;  // nothing to do, nothing written but visited marks
+                        }
+                        FSE_PT(2)
                         c.ev_n = 0;
-                        if (e < total) {
-                            int q, r;
-                            divmod_small(e, nx, rnx, q, r);
-                            const int dy = dyb + q * py, dx = rx + r * px;
-                            if (dx < cw && dy < chh) rule_a(Tl, c, Tl.li(cx + dx, cy + dy), cx + dx, cy + dy);
+                        int e = 0;
+                        if (tid < (int)(nl & 0xFFFF) || tid >= T - (int)(nl >> 16)) {
+                            const int item = S.list[tid];
+                            const int ix = item & 0xFF, iy = item >> 8;
+                            rule_a(Tl, c, Tl.li(cx + ix, cy + iy), cx + ix, cy + iy);
+                            if (c.ev_n > 0) {
+                                int qe, re, t_;
+                                divmod_small(iy - dyb, py, __frcp_rn((float)py), qe, t_);
+                                divmod_small(ix - rx, px, __frcp_rn((float)px), re, t_);
+                                e = qe * nxm + re;
+                                S.cnt[e] = (uint16_t)c.ev_n;  // at most 2^31 >> 18
+                            }
                         }
                         FSE_PT(3)
-                        // rank spawned particles in enumeration order. The scan scratch is
-                        // next written after the next sub-phase's barrier, so no barrier is
-                        // needed after this block.
-                        if constexpr (PAIR) {
-                            S.cnt[tid] = c.ev_n;
-                            // the sub-phase's enumeration runs through rank 0's rows first:
-                            // each CTA ranks its own spawns, the partner's count of the
-                            // sub-phase comes through the cluster barrier that ends it
-                            int tot = 0, ex = 0;
-                            if (__syncthreads_or(c.ev_n > 0)) ex = block_excl_scan(S.cnt[tid], S.scan, &tot);
-                            const int slot_t = 2 + (nsub & 1);
-                            if (tid == 0)
-                                st_cluster_u32(mapa_rank(smem_addr(&S.xch[slot_t]), (uint32_t)(rank ^ 1)),
-                                               (uint32_t)tot);
-                            cluster_sync();
-                            const int tot_p = (int)S.xch[slot_t];
-                            nsub++;
-                            if (c.ev_n > 0) {
-                                const int base = atomicAdd(w.stage_count, c.ev_n);
-                                emit_spawns<TEMP, F32>(w, *c.ev, c.ev_n, cp,
-                                                       (uint32_t)(running + (rank ? tot_p : 0) + ex), base);
-                            }
-                            running += tot + tot_p;
-                        } else if (__syncthreads_or(c.ev_n > 0)) {
-                            // ranks with one more barrier: each warp's total in shared
-                            // memory, a thread's rank the totals of the warps before it plus
-                            // its lanes' prefix (the scratch is next written after the next
-                            // sub-phase's barrier)
+                        // spawned particles are ranked in enumeration order
+                        const bool any = __syncthreads_or(c.ev_n > 0);
+                        int tot = 0, before = running;
+                        if (any) {
                             const int lane = tid & 31, wid = tid >> 5;
-                            int inc = c.ev_n;
+                            const int v = S.cnt[tid];
+                            S.cnt[tid] = 0;
+                            int inc = v;
 #pragma unroll
                             for (int o = 1; o < 32; o <<= 1) {
                                 const int t = __shfl_up_sync(0xffffffffu, inc, o);
@@ -1742,58 +1791,103 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                             if (lane == 31) S.scan[wid] = inc;
                             __syncthreads();
                             const int ws = lane < T / 32 ? S.scan[lane] : 0;
-                            const int tot = (int)__reduce_add_sync(0xffffffffu, (unsigned)ws);
-                            const int ex = (int)__reduce_add_sync(0xffffffffu, lane < wid ? (unsigned)ws : 0u) + inc -
-                                           c.ev_n;
+                            tot = (int)__reduce_add_sync(0xffffffffu, (unsigned)ws);
+                            S.rank[tid] = __reduce_add_sync(0xffffffffu, lane < wid ? (unsigned)ws : 0u) +
+                                          (unsigned)(inc - v);
+                            __syncthreads();
+                        }
+                        if constexpr (PAIR) {
+                            // the sub-phase's enumeration runs through rank 0's rows first:
+                            // each CTA ranks its own spawns, the partner's count of the
+                            // sub-phase comes through the cluster barrier that ends it
+                            const int slot_t = 2 + nsub_a;
+                            nsub_a ^= 1;
+                            if (tid == 0)
+                                st_cluster_u32(mapa_rank(smem_addr(&S.xch[slot_t]), (uint32_t)(rank ^ 1)),
+                                               (uint32_t)tot);
+                            cluster_sync();
+                            const int tot_p = (int)S.xch[slot_t];
+                            if (rank) before += tot_p;
+                            running += tot_p;
+                        }
+                        if (any) {
+                            // staging slots are taken in any order; the (chunk-pass, rank)
+                            // key orders the particles later
                             if (c.ev_n > 0) {
-                                // staging slots are taken in any order; the (chunk-pass, rank)
-                                // key orders the particles later
                                 const int base = atomicAdd(w.stage_count, c.ev_n);
-                                emit_spawns<TEMP, F32>(w, *c.ev, c.ev_n, cp, (uint32_t)(running + ex), base);
+                                emit_spawns<TEMP, F32>(w, *c.ev, c.ev_n, cp, (uint32_t)before + S.rank[e], base);
                             }
                             running += tot;
+                            __syncthreads();  // the ranks give way to the next list
                         }
                         FSE_PT(4)
-                    } else {
-                        // cells of one sub-phase never conflict: each thread takes all of its
-                        // cells in turn, one barrier per sub-phase
-                        int q, r;
-                        divmod_small(tid, nx, rnx, q, r);
-                        int dq, dr;
-                        divmod_small(T, nx, rnx, dq, dr);
-                        if (sweep == 1) {
-                            // at most 43 x 43 < 2 T cells: two per thread, their pending
-                            // diffs requested together before either is processed
-                            const int q1 = q + dq + (r + dr >= nx ? 1 : 0);
-                            const int r1 = r + dr - (r + dr >= nx ? nx : 0);
-                            const int dy0 = dyb + q * py, dx0 = rx + r * px;
-                            const int dy1 = dyb + q1 * py, dx1 = rx + r1 * px;
-                            const bool v0 = tid < total && dx0 < cw && dy0 < chh;
-                            const bool v1 = tid + T < total && dx1 < cw && dy1 < chh;
-                            const int i0 = Tl.li(cx + dx0, cy + dy0), i1 = Tl.li(cx + dx1, cy + dy1);
-                            const uint32_t w0 = v0 ? Tl.at(i0) : CW_VIS, w1 = v1 ? Tl.at(i1) : CW_VIS;
-                            const int32_t df0 = cw_is(w0, T_SOUP) ? w.df[Tl.gi(cx + dx0, cy + dy0)] : 0;
-                            const int32_t df1 = cw_is(w1, T_SOUP) ? w.df[Tl.gi(cx + dx1, cy + dy1)] : 0;
-                            rule_b(Tl, c, w0, i0, cx + dx0, cy + dy0, df0);
-                            rule_b(Tl, c, w1, i1, cx + dx1, cy + dy1, df1);
-                        } else {
-                            for (int e = tid; e < total; e += T) {
-                                const int dy = dyb + q * py, dx = rx + r * px;
-                                if (dx < cw && dy < chh) rule_c(Tl, c, Tl.li(cx + dx, cy + dy), cx + dx, cy + dy);
-                                q += dq;
-                                r += dr;
-                                if (r >= nx) {
-                                    r -= nx;
-                                    q++;
-                                }
-                            }
+                    } else if (sweep == 1) {
+                        // at most 43 x 43 < 2 T cells: two per thread. Liquids take their
+                        // pending diffs, requested together; sand and gas that may move are
+                        // listed and dealt to the threads
+                        const int dx1 = rx + r1 * px, dy1 = dyb + q1 * py;
+                        const bool v1 = dx1 < cw && dy1 < yend;
+                        const int i0 = Tl.li(cx + dx, cy + dy), i1 = Tl.li(cx + dx1, cy + dy1);
+                        const uint32_t w0 = v0 ? Tl.at(i0) : CW_VIS, w1 = v1 ? Tl.at(i1) : CW_VIS;
+                        const int g0 = Tl.gi(cx + dx, cy + dy), g1 = Tl.gi(cx + dx1, cy + dy1);
+                        const bool s0 = (w0 & (CW_TYPE | CW_VIS)) == (uint32_t)T_SOUP << MW_TYPE_SHIFT;
+                        const bool s1 = (w1 & (CW_TYPE | CW_VIS)) == (uint32_t)T_SOUP << MW_TYPE_SHIFT;
+                        const int32_t df0 = s0 ? w.df[g0] : 0, df1 = s1 ? w.df[g1] : 0;
+                        const bool a0 = !(w0 & CW_VIS) && class_b(Tl, w0, i0, w.dirty != nullptr);
+                        const bool a1 = !(w1 & CW_VIS) && class_b(Tl, w1, i1, w.dirty != nullptr);
+                        const unsigned m0 = __ballot_sync(0xffffffffu, a0), m1 = __ballot_sync(0xffffffffu, a1);
+                        if (m0 | m1) {
+                            const int lane = tid & 31;
+                            const unsigned lt = (1u << lane) - 1u;
+                            unsigned at = 0;
+                            if (lane == 0) at = atomicAdd(&S.n_list[nsub], (unsigned)(__popc(m0) + __popc(m1)));
+                            at = __shfl_sync(0xffffffffu, at, 0);
+                            if (a0) S.list[at + __popc(m0 & lt)] = (uint16_t)(dx | (dy << 8));
+                            if (a1) S.list[at + __popc(m0) + __popc(m1 & lt)] = (uint16_t)(dx1 | (dy1 << 8));
                         }
-                        FSE_PT(3 + 2 * sweep)
+                        if (s0) rule_b_soup(Tl, c, w0, i0, g0, df0);
+                        if (s1) rule_b_soup(Tl, c, w1, i1, g1, df1);
+                        FSE_PT(5)
+                        __syncthreads();
+                        const int nl = (int)S.n_list[nsub];
+                        const int nnext = nsub == 2 ? 0 : nsub + 1;
+                        if (tid == 0) S.n_list[nnext == 2 ? 0 : nnext + 1] = 0;
+                        nsub = nnext;
+                        if constexpr (!PAIR) {
+                            if (nl == 0) continue;
+                        }
+                        for (int k = tid; k < nl; k += T) {
+                            const int item = S.list[k];
+                            const int ix = item & 0xFF, iy = item >> 8;
+                            const int i = Tl.li(cx + ix, cy + iy);
+                            rule_b(Tl, c, Tl.at(i), i, cx + ix, cy + iy);
+                        }
                         if constexpr (PAIR)
                             cluster_sync();
                         else
                             __syncthreads();
-                        FSE_PT(4 + 2 * sweep)
+                        FSE_PT(6)
+                    } else {
+                        // every row of the chunk, its columns 3 apart: each thread takes all of
+                        // its cells in turn
+                        int qe = q, re = r;
+                        for (;;) {
+                            const int ex = rx + re * px, ey = dyb + qe * py;
+                            if (ey >= yend) break;
+                            if (ex < cw) rule_c(Tl, c, Tl.li(cx + ex, cy + ey), cx + ex, cy + ey);
+                            qe += dq;
+                            re += dr;
+                            if (re >= nxm) {
+                                re -= nxm;
+                                qe++;
+                            }
+                        }
+                        FSE_PT(7)
+                        if constexpr (PAIR)
+                            cluster_sync();
+                        else
+                            __syncthreads();
+                        FSE_PT(8)
                     }
                 }
             }
@@ -1872,7 +1966,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
     !defined(FSE_TICK_PAIR_TU) && !defined(FSE_TICK_FUSED_TU)
 size_t colour_pass_smem(int C, int halo) {
     // a 2-cell halo leaves room for the TMA-staged tile's wider rows
-    return tile_smem<CP_THREADS, false>(C, C, halo, halo == 2 ? tma_tile_width(C) : 0);
+    return tile_smem<CP_THREADS>(C, C, halo, halo == 2 ? tma_tile_width(C) : 0);
 }
 
 #endif
@@ -1907,7 +2001,7 @@ static cudaError_t launch_fused_t(const WorldDev *worlds, const FusedTick &ft, c
 }
 
 // shared memory of one CTA of a pair: half the chunk's rows plus the reach of its rules
-static size_t colour_pass_smem_pair(int C, int halo) { return tile_smem<CP_THREADS / 2, true>(C, C / 2, halo, 0); }
+static size_t colour_pass_smem_pair(int C, int halo) { return tile_smem<CP_THREADS / 2>(C, C / 2, halo, 0); }
 
 // the chunks split over CTA pairs (thread-block clusters of two): `clusters` pairs
 template <int HALO, bool TEMP, bool F32>
