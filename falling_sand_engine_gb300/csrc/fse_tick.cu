@@ -355,9 +355,6 @@ struct Tile : TileData {
         if (n != w) set_word(i, n | CW_DIRTY);
     }
     __device__ __forceinline__ void set_moved(int i, bool on) const { set_moved_w(i, s_w[i], on); }
-    __device__ __forceinline__ void add_diff(int g, int32_t v) const {
-        atomicAdd(&df[g], v);  // fire-and-forget reduction: the thread does not wait
-    }
     // f32 worlds: fluidAmountDiff += v as the reference's float add. No other cell of
     // the sub-phase (or wavefront step) touches this diff, and the ones that touched
     // it before did so in the reference's order, so a plain read-modify-write adds in
@@ -377,9 +374,10 @@ struct Ctx {
     int id_fire, id_water, id_lava, id_steam, id_obsidian, has_inter;
     bool f32;  // f32 liquid amounts: the ledger keeps no fluid rows (a compile-time constant)
     const MatTable *mt;
-    int32_t *led_s;        // shared ledger [LED_ROWS][64] of the chunk-pass
+    int32_t *led_s;        // shared ledger [LED_TICK][64] of the chunk-pass
     long long *led_g;      // global ledger [LED_ROWS][MAXMAT]
     const uint32_t *mw;    // material words (shared)
+    const uint16_t *fr;    // slipperiness | stability << 8 (shared)
     // the cell's spawn event, a local of its own: emit_spawns takes its address, and a
     // member whose address escapes keeps the whole context in local memory
     SpawnEv *ev;
@@ -407,11 +405,13 @@ struct Ctx {
 // chunk-pass ends. A counter takes amounts below 1024 only, so that a chunk-pass, with
 // at most 3 sweeps x 16384 cells and a few dozen entries a cell, cannot overflow it;
 // larger ones go to the world's ledger at once.
+constexpr int LED_TICK = 4;  // the rows the cell update counts in: all but LED_XN and LED_XF
+__host__ __device__ constexpr int led_slot(int row) { return row > LED_XN ? row - 1 : row; }
 __device__ __forceinline__ void led_add(Ctx &c, int row, uint32_t w, int32_t v) {
     if (v == 0 || cw_air(w)) return;
     const int mat = cw_id(w);
     if (mat < 64 && v > -1024 && v < 1024)
-        atomicAdd(&c.led_s[row * 64 + mat], v);
+        atomicAdd(&c.led_s[led_slot(row) * 64 + mat], v);
     else
         atomicAdd((unsigned long long *)&c.led_g[row * MAXMAT + mat], (unsigned long long)(long long)v);
 }
@@ -454,17 +454,18 @@ __device__ __forceinline__ Cell create_tile(Ctx &c, int mid) {
 }
 
 // CalculateVerticalFlowValue, world.cpp:1021-1034, Q16.16
+// rem > 0. The sum in 32 bits: unsigned it is exact for dst >= 0, and for dst < 0 it is
+// a signed number below 2^31.
 __device__ __forceinline__ int32_t vflow(int32_t rem, int32_t dst) {
-    long long sum = (long long)rem + dst;
-    if (sum <= Q_MAXV) return Q_MAXV;
-    if (sum < 2 * Q_MAXV + Q_MAXCOMP)  // here MAXV^2 + sum * MAXCOMP < 2^31: 32-bit unsigned is exact
-        return (int32_t)(((uint32_t)Q_MAXV * Q_MAXV + (uint32_t)sum * Q_MAXCOMP) / (uint32_t)(Q_MAXV + Q_MAXCOMP));
-    return (int32_t)((sum + Q_MAXCOMP) / 2);
+    const uint32_t sum = (uint32_t)rem + (uint32_t)dst;
+    if (sum <= (uint32_t)Q_MAXV || (dst < 0 && (int32_t)sum < 0)) return Q_MAXV;
+    // MAXV^2 + sum * MAXCOMP < 2^31 below the bound; MAXCOMP is even above it
+    if (sum < (uint32_t)(2 * Q_MAXV + Q_MAXCOMP))
+        return (int32_t)(((uint32_t)Q_MAXV * Q_MAXV + sum * Q_MAXCOMP) / (uint32_t)(Q_MAXV + Q_MAXCOMP));
+    return (int32_t)((sum >> 1) + Q_MAXCOMP / 2);
 }
 __device__ __forceinline__ int32_t clampflow(int32_t flow, int32_t rem) {
-    if (flow < 0) flow = 0;
-    int32_t lim = rem < Q_MAXFLOW ? rem : Q_MAXFLOW;
-    return flow > lim ? lim : flow;
+    return min(max(flow, 0), min(rem, Q_MAXFLOW));  // rem > 0
 }
 
 // CalculateVerticalFlowValue, world.cpp:1021-1034, in the reference's f32: every
@@ -673,46 +674,28 @@ __device__ __forceinline__ void rule_a_soup(const TL &T, Ctx &c, uint32_t w0, in
             swap_up = c.D() % 10 == 0;
         }
     }
-    // the flows: a new cell in AIR, else a pending diff
-    int made = 0;
-    int32_t *fw = s_w.flow;
-    if (down != 0) {
-        if (fw) render_flow(fw, g, 1, down);
-        if (airBelow) {
-            flow_into_air(T, w0, col, i + RW, wb, g + T.W, down, g);
-            made++;
-        } else {
-            T.add_diff(g + T.W, down);
-        }
+    int32_t *pd = T.df + g;
+    if (int32_t *fw = s_w.flow) {
+        if (down != 0) render_flow(fw, g, 1, down);
+        if (left != 0) render_flow(fw, g, 0, -left);
+        if (right != 0) render_flow(fw, g, 0, right);
+        if (up != 0) render_flow(fw, g, 1, -up);
     }
-    if (left != 0) {
-        if (fw) render_flow(fw, g, 0, -left);
-        if (cw_air(wl)) {
-            flow_into_air(T, w0, col, i - 1, wl, g - 1, left, g);
-            made++;
-        } else {
-            T.add_diff(g - 1, left);
-        }
+    // the flows: pending diffs (reductions, nothing waits for them), and where they enter
+    // AIR new cells, which few of a liquid's flows do
+    const bool mb = down != 0 && airBelow, ml = left != 0 && cw_air(wl), mr = right != 0 && cw_air(wr);
+    const bool mu = up != 0 && cw_air(wt);
+    if (down != 0 && !airBelow) atomicAdd(pd + T.W, down);
+    if (left != 0 && !ml) atomicAdd(pd - 1, left);
+    if (right != 0 && !mr) atomicAdd(pd + 1, right);
+    if (up != 0 && !mu) atomicAdd(pd - T.W, up);
+    if (mb || ml || mr || mu) {
+        if (mb) flow_into_air(T, w0, col, i + RW, wb, g + T.W, down, g);
+        if (ml) flow_into_air(T, w0, col, i - 1, wl, g - 1, left, g);
+        if (mr) flow_into_air(T, w0, col, i + 1, wr, g + 1, right, g);
+        if (mu) flow_into_air(T, w0, col, i - RW, wt, g - T.W, up, g);
+        led_add(c, LED_CN, w0, (int)mb + (int)ml + (int)mr + (int)mu);
     }
-    if (right != 0) {
-        if (fw) render_flow(fw, g, 0, right);
-        if (cw_air(wr)) {
-            flow_into_air(T, w0, col, i + 1, wr, g + 1, right, g);
-            made++;
-        } else {
-            T.add_diff(g + 1, right);
-        }
-    }
-    if (up != 0) {
-        if (fw) render_flow(fw, g, 1, -up);
-        if (cw_air(wt)) {
-            flow_into_air(T, w0, col, i - RW, wt, g - T.W, up, g);
-            made++;
-        } else {
-            T.add_diff(g - T.W, up);
-        }
-    }
-    led_add(c, LED_CN, w0, made);
     const int32_t dd = rem - sc;  // the change of its own pending diff
     if (swap_up) {
         swap_liquid(T, w0, sc, col, dd + T.df_load(g), i, g, i - RW, g - T.W);
@@ -721,7 +704,7 @@ __device__ __forceinline__ void rule_a_soup(const TL &T, Ctx &c, uint32_t w0, in
     if (gone) {  // the remainder evaporates
         led_add64(c, LED_DF, w0, rem);
         T.set_word(i, w0 | CW_DIRTY);
-        if (sc != 0) T.add_diff(g, -sc);
+        atomicAdd(pd, -sc);
         return;
     }
     uint32_t wn = w0;
@@ -732,7 +715,7 @@ __device__ __forceinline__ void rule_a_soup(const TL &T, Ctx &c, uint32_t w0, in
         if (cw_is(wb, T_SOUP)) T.set_moved_w(i + RW, wb, false);
         if (cw_is(wl, T_SOUP)) T.set_moved_w(i - 1, wl, false);
         if (cw_is(wr, T_SOUP)) T.set_moved_w(i + 1, wr, false);
-        T.add_diff(g, dd);
+        atomicAdd(pd, dd);
     }
     T.set_word(i, wn | CW_DIRTY);
     if (cw_id(w0) == c.id_water && cw_id(wb) == c.id_lava)
@@ -1093,11 +1076,11 @@ __device__ __forceinline__ void rule_b(const TL &T, Ctx &c, uint32_t w0, int i, 
         const bool canR = T.at(i + RW + 1) < lim;
         bool stopped = !(w0 & CW_MOVED);
         c.at(x, y);
-        const uint32_t a = __ldg(&c.mt->a[cw_id(w0)]);
+        const int a = c.fr[cw_id(w0)];
         if (stopped) {
             // world.cpp:1619-1627 over the AIR snapshot taken when sweep B began
             const int drop = __popc(T.air10(i + RW - 1, x - 1, y + 1) | T.air10(i + RW + 1, x + 1, y + 1));
-            int d = drop + 1 - mt_stab(a);
+            int d = drop + 1 - (a >> 8);
             if (d > 0) {
                 int chance = 1000 / d;
                 if (chance < 1000) {
@@ -1117,7 +1100,7 @@ __device__ __forceinline__ void rule_b(const TL &T, Ctx &c, uint32_t w0, int i, 
         const int g = T.gi(x, y);
         const int32_t sc = T.s_sc[i];
         const uint32_t col = T.s_col[i];
-        const int slip = mt_slip(a);
+        const int slip = a & 0xFF;
         const bool shouldMove = (slip > 0) ? (c.D() % (uint32_t)(2 * slip) != 0) : true;
         if (shouldMove && (canL || canR)) {
             if (c.D() % 2 == 0) {
@@ -1278,20 +1261,21 @@ static __device__ __noinline__ void emit_spawns(const WorldDev &w, const SpawnEv
 template <int NT>
 struct SmemHeadT {
     uint32_t mw[MAXMAT];  // material -> cell word of this iteration
-    int32_t led[LED_ROWS * 64];   // the chunk-pass's ledger counts
+    uint16_t fr[MAXMAT];  // slipperiness | stability << 8
+    int32_t led[LED_TICK * 64];   // the chunk-pass's ledger counts (led_slot)
     int scan[32];
-    // sweep A: the spawn counts of a sub-phase by enumeration index (zero between
-    // sub-phases); sweep B: the pillar snapshot (chunk edge <= 128)
-    union {
-        uint16_t cnt[NT];
-        uint32_t air[(128 + 2) * 5];
-    };
+    // the pillar snapshot of sweep B (chunk edge <= 128)
+    uint32_t air[(128 + 2) * 5];
     // the cells of a sub-phase that a rule may change (dx | dy << 8); after a sweep-A
-    // sub-phase that spawned, the ranks of its spawns by enumeration index
+    // sub-phase where a cell spawned several particles, the spawn counts, then ranks
     union {
         uint16_t list[2 * NT];
-        uint32_t rank[NT];
+        uint32_t cnt[NT];
     };
+    // which cells of a sweep-A sub-phase spawn, by enumeration index, in the same turn; and
+    // the last sub-phase in which a cell spawned more than one particle
+    uint32_t spawn_bits[3][NT / 32];
+    int many;
     uint32_t n_list[3];  // lengths of the lists of this sub-phase and of the next two, in turn
     // CTA pair: what the partner wrote here: [0..1] its chunk flags, [2..3] its spawn
     // count of a sweep-A sub-phase (alternate slots)
@@ -1354,8 +1338,14 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
     const int rank = PAIR ? (int)cluster_rank() : 0;
     int npass = 0;  // chunks taken so far (the same count in both CTAs of a pair)
     int mw_iter = -1;  // the iteration S.mw was built for
-    for (int i = tid; i < LED_ROWS * 64; i += T) S.led[i] = 0;
+    for (int i = tid; i < MAXMAT; i += T)
+        S.fr[i] = (uint16_t)(i < mt->n ? mt_slip(mt->a[i]) | (mt_stab(mt->a[i]) << 8) : 0);
+    for (int i = tid; i < LED_TICK * 64; i += T) S.led[i] = 0;
     if (tid < 3) S.n_list[tid] = 0;
+    if (tid < T / 32)
+        for (int k = 0; k < 3; k++) S.spawn_bits[k][tid] = 0;
+    if (tid == 0) S.many = 0;
+    int seq = 0;  // sub-phases of sweep A so far
     int nsub = 0;  // the list count of the next sub-phase of sweeps A and B
     Ctx c;
     SpawnEv ev_store;  // outside the context (see Ctx::ev)
@@ -1364,6 +1354,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
     c.mt = mt;
     c.led_s = S.led;
     c.mw = S.mw;
+    c.fr = S.fr;
     c.id_fire = mt->id_fire;
     c.id_water = mt->id_water;
     c.id_lava = mt->id_lava;
@@ -1531,8 +1522,6 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
             Tl.pd = (rank ? half : -half) * Tl.RW;
         }
 
-        S.cnt[tid] = 0;
-
         // ---- stage the tile, one warp per row. The 4-byte planes go straight to
         // shared memory, as two tensor copies (TMA) or with cp.async; ids and flags
         // are loaded a row at a time, all loads of a row in flight together. The
@@ -1544,7 +1533,59 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
             tma_load_2d(Tl.s_col, tm + 128, Tl.x0, Tl.y0, &s_tma_bar);
         }
         int active = 0, fire = 0;
-        {
+        if (tma) {
+            // ids and flags four cells at a time: a group starts on a multiple of four cells, so
+            // it lies wholly inside or outside a world that is a multiple of four cells wide.
+            // All of a thread's loads are in flight together: one round trip to memory where
+            // the row-by-row form below waits for five.
+            constexpr int NG = 5;  // 140 rows of 34 groups over 1024 threads
+            const int gpr = Tl.RW / 4, groups = gpr * Tl.RHI;
+            const float rgpr = __frcp_rn((float)gpr);
+            uint2 v[NG];
+            uint32_t f[NG];
+            int rows[NG];
+#pragma unroll
+            for (int k = 0; k < NG; k++) {
+                const int e = tid + k * T;
+                int r, q4;
+                divmod_small(e, gpr, rgpr, r, q4);
+                const int gx = Tl.x0 + 4 * q4, gy = Tl.y0 + r;
+                rows[k] = r;
+                const bool in = e < groups && (unsigned)gy < (unsigned)H && (unsigned)gx < (unsigned)W;
+                const uint32_t so = (uint32_t)id_solid * 0x10001u;
+                v[k] = make_uint2(so, so);
+                f[k] = 0;
+                if (in) {
+                    const size_t gi = (size_t)gy * W + gx;
+                    v[k] = *reinterpret_cast<const uint2 *>(&w.id[gi]);
+                    if (r < Tl.RHF) f[k] = *reinterpret_cast<const uint32_t *>(&w.fl[gi]);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < NG; k++) {
+                const int e = tid + k * T;
+                if (e >= groups) break;
+                const int q4 = e - rows[k] * gpr, gx = Tl.x0 + 4 * q4, gy = Tl.y0 + rows[k];
+                const uint32_t fl = f[k] & ~((uint32_t)VISITED * 0x01010101u);
+                uint4 o;
+                o.x = S.mw[v[k].x & CW_ID] | ((fl & 0xFFu) << 8);
+                o.y = S.mw[(v[k].x >> 16) & CW_ID] | (fl & 0xFF00u);
+                o.z = S.mw[v[k].y & CW_ID] | ((fl >> 8) & 0xFF00u);
+                o.w = S.mw[(v[k].y >> 16) & CW_ID] | ((fl >> 16) & 0xFF00u);
+                *reinterpret_cast<uint4 *>(&Tl.s_w[4 * e]) = o;
+                // the chunk's cells inside the world vote
+                if (gy >= cy && gy < cy + C && gy < H && gx < W) {
+                    const int l = cx - gx, u = cx + C - gx;  // cells l .. u - 1 of the group
+                    uint32_t any = 0;
+                    if (l <= 0 && u > 0) any |= o.x;
+                    if (l <= 1 && u > 1) any |= o.y;
+                    if (l <= 2 && u > 2) any |= o.z;
+                    if (l <= 3 && u > 3) any |= o.w;
+                    if (any & CW_LIVE) active = 1;
+                    if (any & CW_FIRE) fire = 1;
+                }
+            }
+        } else {
             const int lane = tid & 31, wid = tid >> 5;
             constexpr int NW = T / 32;
             for (int r = wid; r < Tl.RHI; r += NW) {
@@ -1700,6 +1741,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
             if (tid < w.cp_rows) w.cp_count[cp * w.cp_rows + tid] = spawned;
         };
         auto sweeps = [&](const auto &Tl) {
+#pragma unroll 1
         for (int sweep = 0; sweep < 3; sweep++) {
             c.pk = pass_key(w.seed, *w.tick, (uint32_t)(c.iter * 3 + sweep));
             if (sweep == 1) {
@@ -1727,10 +1769,12 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
             divmod_small(T, nxm, __frcp_rn((float)nxm), dq, dr);
             const int q1 = q + dq + (r + dr >= nxm ? 1 : 0);  // and of index tid + T
             const int r1 = r + dr - (r + dr >= nxm ? nxm : 0);
+#pragma unroll 1
             for (int ry = py - 1; ry >= 0; ry--) {
                 // this CTA's rows of the sub-phase: dyb, dyb + py, ... below o1
                 const int dyb = ry + (o0 > ry ? (o0 - ry + py - 1) / py * py : 0);
                 const int yend = min(o1, chh);
+#pragma unroll 1
                 for (int rx = 0; rx < px; rx++) {
                     const int dx = rx + r * px, dy = dyb + q * py;
                     const bool v0 = dx < cw && dy < yend;
@@ -1752,9 +1796,10 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                         }
                         __syncthreads();
                         const unsigned nl = S.n_list[nsub];
-                        const int nnext = nsub == 2 ? 0 : nsub + 1;
+                        const int sub = nsub, nnext = nsub == 2 ? 0 : nsub + 1;
                         // last read before this sub-phase's barrier, next used after the next one's
                         if (tid == 0) S.n_list[nnext == 2 ? 0 : nnext + 1] = 0;
+                        if (tid < T / 32) S.spawn_bits[nnext == 2 ? 0 : nnext + 1][tid] = 0;
                         nsub = nnext;
                         if constexpr (!PAIR) {
                             if (nl == 0) continue;  // nothing to do, nothing written but visited marks
@@ -1771,30 +1816,70 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                                 divmod_small(iy - dyb, py, __frcp_rn((float)py), qe, t_);
                                 divmod_small(ix - rx, px, __frcp_rn((float)px), re, t_);
                                 e = qe * nxm + re;
-                                S.cnt[e] = (uint16_t)c.ev_n;  // at most 2^31 >> 18
                             }
                         }
-                        FSE_PT(3)
-                        // spawned particles are ranked in enumeration order
-                        const bool any = __syncthreads_or(c.ev_n > 0);
-                        int tot = 0, before = running;
-                        if (any) {
-                            const int lane = tid & 31, wid = tid >> 5;
-                            const int v = S.cnt[tid];
-                            S.cnt[tid] = 0;
-                            int inc = v;
+                        // The spawns take staging slots a warp at a time, in any order; the atomic
+                        // returns while the sub-phase's barrier waits for other warps.
+                        __syncwarp();
+                        const int lane = tid & 31, wid = tid >> 5;
+                        const unsigned sp = __ballot_sync(0xffffffffu, c.ev_n > 0);
+                        int slot = 0;
+                        seq++;
+                        if (sp) {
+                            int inc = c.ev_n;
 #pragma unroll
                             for (int o = 1; o < 32; o <<= 1) {
                                 const int t = __shfl_up_sync(0xffffffffu, inc, o);
                                 if (lane >= o) inc += t;
                             }
-                            if (lane == 31) S.scan[wid] = inc;
-                            __syncthreads();
-                            const int ws = lane < T / 32 ? S.scan[lane] : 0;
-                            tot = (int)__reduce_add_sync(0xffffffffu, (unsigned)ws);
-                            S.rank[tid] = __reduce_add_sync(0xffffffffu, lane < wid ? (unsigned)ws : 0u) +
-                                          (unsigned)(inc - v);
-                            __syncthreads();
+                            if (lane == 31) slot = atomicAdd(w.stage_count, inc);
+                            slot = __shfl_sync(0xffffffffu, slot, 31) + inc - c.ev_n;
+                            if (c.ev_n > 0) atomicOr(&S.spawn_bits[sub][e >> 5], 1u << (e & 31));
+                            if (c.ev_n > 1) S.many = seq;
+                        }
+                        FSE_PT(3)
+                        // spawned particles are ranked in enumeration order: from the bits of the
+                        // spawning cells, a word per lane of every warp, without another barrier
+                        const bool any = __syncthreads_or(c.ev_n > 0);
+                        int tot = 0, before = running, rank_e = 0;
+                        bool slow = false;
+                        if (any) {
+                            slow = S.many == seq;
+                            if (!slow) {
+                                const uint32_t word = lane < T / 32 ? S.spawn_bits[sub][lane] : 0u;
+                                int inc = __popc(word);
+#pragma unroll
+                                for (int o = 1; o < 32; o <<= 1) {
+                                    const int t = __shfl_up_sync(0xffffffffu, inc, o);
+                                    if (lane >= o) inc += t;
+                                }
+                                tot = __shfl_sync(0xffffffffu, inc, 31);
+                                const uint32_t we = __shfl_sync(0xffffffffu, word, e >> 5);
+                                rank_e = __shfl_sync(0xffffffffu, inc - __popc(word), e >> 5) +
+                                         __popc(we & ((1u << (e & 31)) - 1u));
+                            } else {
+                                // some cell spawns several: a scan over their counts
+                                S.cnt[tid] = 0;
+                                __syncthreads();
+                                if (c.ev_n > 0) S.cnt[e] = (uint32_t)c.ev_n;
+                                __syncthreads();
+                                const int v = (int)S.cnt[tid];
+                                int inc = v;
+#pragma unroll
+                                for (int o = 1; o < 32; o <<= 1) {
+                                    const int t = __shfl_up_sync(0xffffffffu, inc, o);
+                                    if (lane >= o) inc += t;
+                                }
+                                if (lane == 31) S.scan[wid] = inc;
+                                __syncthreads();
+                                const int ws = lane < T / 32 ? S.scan[lane] : 0;
+                                tot = (int)__reduce_add_sync(0xffffffffu, (unsigned)ws);
+                                S.cnt[tid] = __reduce_add_sync(0xffffffffu, lane < wid ? (unsigned)ws : 0u) +
+                                             (unsigned)(inc - v);
+                                __syncthreads();
+                                rank_e = (int)S.cnt[e];
+                                __syncthreads();
+                            }
                         }
                         if constexpr (PAIR) {
                             // the sub-phase's enumeration runs through rank 0's rows first:
@@ -1810,16 +1895,9 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                             if (rank) before += tot_p;
                             running += tot_p;
                         }
-                        if (any) {
-                            // staging slots are taken in any order; the (chunk-pass, rank)
-                            // key orders the particles later
-                            if (c.ev_n > 0) {
-                                const int base = atomicAdd(w.stage_count, c.ev_n);
-                                emit_spawns<TEMP, F32>(w, *c.ev, c.ev_n, cp, (uint32_t)before + S.rank[e], base);
-                            }
-                            running += tot;
-                            __syncthreads();  // the ranks give way to the next list
-                        }
+                        // the (chunk-pass, rank) key orders the particles later
+                        if (c.ev_n > 0) emit_spawns<TEMP, F32>(w, *c.ev, c.ev_n, cp, (uint32_t)(before + rank_e), slot);
+                        running += tot;
                         FSE_PT(4)
                     } else if (sweep == 1) {
                         // at most 43 x 43 < 2 T cells: two per thread. Liquids take their
@@ -1852,10 +1930,12 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                         const int nl = (int)S.n_list[nsub];
                         const int nnext = nsub == 2 ? 0 : nsub + 1;
                         if (tid == 0) S.n_list[nnext == 2 ? 0 : nnext + 1] = 0;
+                        if (tid < T / 32) S.spawn_bits[nnext == 2 ? 0 : nnext + 1][tid] = 0;
                         nsub = nnext;
                         if constexpr (!PAIR) {
                             if (nl == 0) continue;
                         }
+#pragma unroll 1
                         for (int k = tid; k < nl; k += T) {
                             const int item = S.list[k];
                             const int ix = item & 0xFF, iy = item >> 8;
@@ -1871,6 +1951,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                         // every row of the chunk, its columns 3 apart: each thread takes all of
                         // its cells in turn
                         int qe = q, re = r;
+#pragma unroll 1
                         for (;;) {
                             const int ex = rx + re * px, ey = dyb + qe * py;
                             if (ey >= yend) break;
@@ -1900,7 +1981,34 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
 
         // ---- write back the cells this CTA changed (full-state rows inside the world),
         // one warp per row
-        {
+        if (tma) {
+            // four cells at a time, whole groups that hold a changed cell: the other cells of
+            // the tile go back as they were staged (no other chunk-pass runs on them meanwhile)
+            const int gpr = Tl.RW / 4, groups = gpr * Tl.RHF;
+            const float rgpr = __frcp_rn((float)gpr);
+            for (int e = tid; e < groups; e += T) {
+                const uint4 o = *reinterpret_cast<const uint4 *>(&Tl.s_w[4 * e]);
+                if (!((o.x | o.y | o.z | o.w) & CW_DIRTY)) continue;
+                int r, q4;
+                divmod_small(e, gpr, rgpr, r, q4);
+                const int gx = Tl.x0 + 4 * q4, gy = Tl.y0 + r;
+                if ((unsigned)gy >= (unsigned)H || (unsigned)gx >= (unsigned)W) continue;
+                const size_t gi = (size_t)gy * W + gx;
+                constexpr uint32_t FL = (CW_FLAGS & ~CW_VIS) >> 8;
+                *reinterpret_cast<uint2 *>(&w.id[gi]) =
+                    make_uint2((o.x & CW_ID) | (o.y & CW_ID) << 16, (o.z & CW_ID) | (o.w & CW_ID) << 16);
+                *reinterpret_cast<uint32_t *>(&w.fl[gi]) = (o.x >> 8 & FL) | (o.y >> 8 & FL) << 8 |
+                                                           (o.z >> 8 & FL) << 16 | (o.w >> 8 & FL) << 24;
+                *reinterpret_cast<uint4 *>(&w.sc[gi]) = *reinterpret_cast<const uint4 *>(&Tl.s_sc[4 * e]);
+                *reinterpret_cast<uint4 *>(&w.col[gi]) = *reinterpret_cast<const uint4 *>(&Tl.s_col[4 * e]);
+                if (w.dirty) {
+                    if (o.x & CW_DIRTY) w.dirty[gi] = 1;
+                    if (o.y & CW_DIRTY) w.dirty[gi + 1] = 1;
+                    if (o.z & CW_DIRTY) w.dirty[gi + 2] = 1;
+                    if (o.w & CW_DIRTY) w.dirty[gi + 3] = 1;
+                }
+            }
+        } else {
             const int lane = tid & 31, wid = tid >> 5;
             for (int r = wid; r < Tl.RHF; r += T / 32) {
                 const int gy = Tl.y0 + r;
@@ -1926,11 +2034,12 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
         }
         if (!SEQ && tid == 0 && rank == 0) w.cp_count[cp] = running;
         // the chunk-pass's ledger counts (the sweeps ended with a barrier)
-        for (int i = tid; i < LED_ROWS * 64; i += T) {
+        for (int i = tid; i < LED_TICK * 64; i += T) {
             const int32_t v = S.led[i];
             if (v == 0) continue;
             S.led[i] = 0;
-            atomicAdd((unsigned long long *)&w.ledger[(i / 64) * MAXMAT + (i % 64)], (unsigned long long)(long long)v);
+            const int row = i / 64 < LED_XN ? i / 64 : i / 64 + 1;
+            atomicAdd((unsigned long long *)&w.ledger[row * MAXMAT + (i % 64)], (unsigned long long)(long long)v);
         }
         __syncthreads();
         FSE_PT(9)
