@@ -758,7 +758,7 @@ static void free_world(fse_world *w) {
     WorldDev &h = w->h;
     void *ptrs[] = {h.id, h.col, h.sc, h.fl, h.df, h.tp, h.tnew, h.stage, h.cp_count, h.cp_base, h.p_state, h.p_box0,
                     h.p_box1, h.p_cell, h.p_prev, h.chg, h.scan_tmp, h.ledger, h.airmap, w->ctr, w->d, w->claim,
-                    w->mask_bits, w->obj_list, w->obj_n, h.merge_list, h.merge_count, h.merge_claim, h.cdone};
+                    w->mask_bits, w->obj_list, w->obj_n, w->obj_scr, h.merge_list, h.merge_count, h.merge_claim, h.cdone};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     PartSoA *ps[2] = {&h.p, &h.q};

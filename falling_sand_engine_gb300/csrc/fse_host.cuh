@@ -52,6 +52,8 @@ struct fse_world {
     uint32_t *obj_list;   // object list scratch
     size_t obj_list_cap;
     int64_t *obj_n;       // object list count
+    uint8_t *obj_scr;     // stamp / readback workspace, grown on first use and kept until fse_world_trim
+    size_t obj_scr_bytes;
     std::map<int, cudaGraphExec_t> graphs;  // n_ticks -> step graph
     std::map<int, long long> graph_kernels;  // n_ticks -> kernels one replay launches
     size_t bytes;         // device bytes owned
