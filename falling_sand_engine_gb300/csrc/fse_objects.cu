@@ -2,8 +2,7 @@
 // (source/engine/game.cpp:1768-1814), readback after it (game.cpp:1896-1983) and
 // the per-tick OBJECT-cell export to the host-side rigid-body solver.
 //
-// Stamp and readback resolve body tiles inside one CTA per world by deferred
-// acceptance (see k_obj_rounds): the result is the reference's tile-by-tile one,
+// Stamp and readback resolve body tiles by deferred acceptance (see k_obj_settle): the result is the reference's tile-by-tile one,
 // and displaced particles are appended in (body, tile) order.
 #include <algorithm>
 #include <vector>
@@ -65,38 +64,7 @@ __device__ __forceinline__ bool tile_usable(const WorldDev &w, const MatTable *_
     return cid == body_id;
 }
 
-// tile g proposes its next usable cell from ptr[g] on (a cell claimed by an
-// earlier tile is skipped for good); returns the proposer displaced from that cell
-// (or 0xffffffff), and records the cell in held[g] (-1 when none is left)
-__device__ __forceinline__ uint32_t tile_propose(const WorldDev &w, const MatTable *__restrict__ mt,
-                                                 const fse_body *__restrict__ bodies,
-                                                 const uint32_t *__restrict__ prefix, int nb, int mode, uint32_t g,
-                                                 uint32_t *ptr, int32_t *held, uint32_t *claim) {
-    const int bi = body_of(prefix, nb, g);
-    const fse_body b = bodies[bi];
-    const int t = (int)(g - prefix[bi]);
-    int wx, wy;
-    body_pos(b, t / b.h, t % b.h, wx, wy);
-    int d = (int)ptr[g];
-    for (; d < 5; d++) {
-        const int xd = wx + c_dirs[d][0], yd = wy + c_dirs[d][1];
-        if (xd < 0 || yd < 0 || xd >= w.W || yd >= w.H) continue;
-        const int c = yd * w.W + xd;
-        if (!tile_usable(w, mt, mode, c, (int)b.id) || claim[c] < g) continue;
-        const uint32_t old = atomicMin(&claim[c], g);
-        ptr[g] = (uint32_t)d;
-        held[g] = c;
-        return old;
-    }
-    ptr[g] = 5;
-    held[g] = -1;
-    return 0xffffffffu;
-}
-
 // mode 0 = stamp, 1 = readback; prefix[b] = first global tile index of body b.
-// Scratch of prefix[nb] entries: ptr (the next offset to try, 5 = none left), held
-// (the cell a tile holds, -1 = none), two work lists (list_b twice as long) and a
-// queued mark; na counts list_a.
 //
 // The reference walks the tiles one after another (bodies in order, tx-major,
 // ty-minor): each takes the first of its five cells that is usable at that moment
@@ -105,94 +73,89 @@ __device__ __forceinline__ uint32_t tile_propose(const WorldDev &w, const MatTab
 // keeping its lowest proposer (claim = atomicMin of the tile index) and displacing
 // higher ones, a rejected or displaced tile proposing its next cell: deferred
 // acceptance with the same priority order at every cell, whose outcome is the
-// sequential one. Usability is read from the grid before any write, since only the
-// taking itself makes a cell unusable. After one round over all tiles, only the
-// tiles that lost a cell and the holders their proposals displace are looked at.
-// Displaced particles are then appended in tile order.
-//
-// Every tile's first proposal, the search for the tiles that lost theirs, and the
-// outcome run over the whole GPU; only the later rounds, over the few tiles still
-// open, run in one CTA, whose barriers they need. In one CTA throughout, 260,000 tiles
-// of 200 boxes took 4.0 ms a call, all of it waiting on memory with 32 warps on one SM.
-__global__ void __launch_bounds__(256) k_obj_first(const WorldDev *__restrict__ wd, const MatTable *__restrict__ mt,
+// sequential one, in whatever order the proposals are made. Usability is read from the
+// grid before any write, since only the taking itself makes a cell unusable. Displaced
+// particles are then appended in tile order.
+
+// a tile's own cell and which of its five cells it may take
+struct ObjTile {
+    int32_t x, y;  // may lie outside the world
+    uint32_t use;  // bit d: the cell at c_dirs[d]
+    int32_t pad;
+};
+
+__global__ void __launch_bounds__(256) k_obj_tiles(const WorldDev *__restrict__ wd, const MatTable *__restrict__ mt,
                                                    const fse_body *__restrict__ bodies,
-                                                   const uint32_t *__restrict__ prefix, int nb, uint32_t *ptr,
-                                                   int32_t *held, uint32_t *queued, uint32_t *claim, int mode,
-                                                   int32_t *na) {
+                                                   const uint32_t *__restrict__ prefix, int nb, int mode,
+                                                   ObjTile *tiles) {
+    const WorldDev &w = *wd;
     const uint32_t total = prefix[nb];
-    if (blockIdx.x == 0 && threadIdx.x == 0) *na = 0;
     for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
-        ptr[g] = 0;
-        queued[g] = 0;
-        tile_propose(*wd, mt, bodies, prefix, nb, mode, g, ptr, held, claim);
+        const int bi = body_of(prefix, nb, g);
+        const fse_body &b = bodies[bi];
+        const int t = (int)(g - prefix[bi]);
+        ObjTile o;
+        body_pos(b, t / b.h, t % b.h, o.x, o.y);
+        o.use = 0;
+        o.pad = 0;
+#pragma unroll
+        for (int d = 0; d < 5; d++) {
+            const long long x = (long long)o.x + c_dirs[d][0], y = (long long)o.y + c_dirs[d][1];
+            if (x < 0 || y < 0 || x >= w.W || y >= w.H) continue;
+            if (tile_usable(w, mt, mode, (int)y * w.W + (int)x, (int)b.id)) o.use |= 1u << d;
+        }
+        tiles[g] = o;
     }
 }
 
-// the tiles that lost their cell to an earlier one
-__global__ void __launch_bounds__(256) k_obj_losers(uint32_t total, uint32_t *ptr, int32_t *held, uint32_t *list_a,
-                                                    const uint32_t *__restrict__ claim, int32_t *na) {
-    const int lane = threadIdx.x & 31;
-    for (uint32_t g0 = blockIdx.x * blockDim.x; g0 < total; g0 += gridDim.x * blockDim.x) {
-        const uint32_t g = g0 + threadIdx.x;
-        bool open = false;
-        if (g < total) {
-            const int c = held[g];
-            if (c >= 0 && claim[c] != g) {
-                held[g] = -1;
-                const uint32_t d = ptr[g] + 1;
-                ptr[g] = d;
-                open = d < 5;
-            }
+// Every thread takes a tile through its proposals; a tile that it displaces from a cell is
+// taken through its further ones by the same thread, from the cell that it lost (which of
+// its five that was follows from its position). So a chain of displacements, up to some
+// hundred tiles long where boxes read back overlapping cells, waits for two memory round
+// trips a link and for no other tile. (Rounds over work lists in one CTA, with a barrier and a
+// dozen dependent loads a round, took 1.9 ms of a call with 260,000 tiles.)
+__global__ void __launch_bounds__(256) k_obj_settle(const WorldDev *__restrict__ wd, uint32_t total,
+                                                    const ObjTile *__restrict__ tiles, uint32_t *claim) {
+    const int W = wd->W;
+    for (uint32_t first = blockIdx.x * blockDim.x + threadIdx.x; first < total; first += gridDim.x * blockDim.x) {
+        uint32_t g = first;
+        ObjTile o = tiles[g];
+        uint32_t left = o.use;  // the cells not yet proposed to
+        // ends: each step uses up one of some tile's five cells, for good
+        while (left) {
+            const int d = __ffs(left) - 1;
+            left &= left - 1;
+            const int c = (o.y + c_dirs[d][1]) * W + o.x + c_dirs[d][0];
+            const uint32_t old = atomicMin(&claim[c], g);
+            if (old < g) continue;  // taken by an earlier tile
+            if (old == 0xffffffffu) break;
+            g = old;  // displaced from c
+            o = tiles[g];
+            const int x = c % W - o.x, y = c / W - o.y;
+            int lost = 0;
+#pragma unroll
+            for (int k = 0; k < 5; k++)
+                if (c_dirs[k][0] == x && c_dirs[k][1] == y) lost = k;
+            left = o.use & ~((2u << lost) - 1u);
         }
-        const unsigned m = __ballot_sync(0xffffffffu, open);
-        int at = 0;
-        if (lane == 0 && m) at = atomicAdd(na, __popc(m));
-        at = __shfl_sync(0xffffffffu, at, 0);
-        if (open) list_a[at + __popc(m & ((1u << lane) - 1u))] = g;
     }
 }
 
-// the rounds over the open tiles (list_a) and the holders they displace
-__global__ void __launch_bounds__(1024) k_obj_rounds(WorldDev *wd, const MatTable *__restrict__ mt,
-                                                     const fse_body *__restrict__ bodies,
-                                                     const uint32_t *__restrict__ prefix, int nb, uint32_t *ptr,
-                                                     int32_t *held, uint32_t *list_a, uint32_t *list_b,
-                                                     uint32_t *queued, uint32_t *claim, int mode, const int32_t *na0) {
-    WorldDev &w = *wd;
-    __shared__ int s_na, s_nb;
-    const uint32_t total = prefix[nb];
-    if (threadIdx.x == 0) s_na = *na0;
-    __syncthreads();
-    for (long long round = 0; s_na > 0; round++) {
-        if (round > 8LL * total + 8) {  // cannot happen: every round moves a pointer forward
-            if (threadIdx.x == 0) atomicOr(w.err, ERR_TIMEOUT);
-            break;
+// the cell a tile holds in the end (-1: none)
+__global__ void __launch_bounds__(256) k_obj_held(const WorldDev *__restrict__ wd, uint32_t total,
+                                                  const ObjTile *__restrict__ tiles, const uint32_t *__restrict__ claim,
+                                                  int32_t *held) {
+    const int W = wd->W;
+    for (uint32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < total; g += gridDim.x * blockDim.x) {
+        const ObjTile o = tiles[g];
+        int h = -1;
+#pragma unroll
+        for (int d = 0; d < 5; d++) {
+            if (!(o.use >> d & 1)) continue;
+            const int c = (o.y + c_dirs[d][1]) * W + o.x + c_dirs[d][0];
+            if (claim[c] == g) h = c;
         }
-        const int na = s_na;
-        if (threadIdx.x == 0) s_nb = 0;
-        __syncthreads();
-        // propose; the proposer and the holder it may displace are checked next
-        for (int j = threadIdx.x; j < na; j += blockDim.x) {
-            const uint32_t g = list_a[j];
-            const uint32_t old = tile_propose(w, mt, bodies, prefix, nb, mode, g, ptr, held, claim);
-            if (held[g] >= 0 && atomicExch(&queued[g], 1u) == 0u) list_b[atomicAdd(&s_nb, 1)] = g;
-            if (old != 0xffffffffu && old > g && atomicExch(&queued[old], 1u) == 0u) list_b[atomicAdd(&s_nb, 1)] = old;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) s_na = 0;
-        __syncthreads();
-        const int nbv = s_nb;
-        for (int j = threadIdx.x; j < nbv; j += blockDim.x) {
-            const uint32_t g = list_b[j];
-            queued[g] = 0;
-            const int c = held[g];
-            if (c >= 0 && claim[c] != g) {
-                held[g] = -1;
-                ptr[g] += 1;
-                if (ptr[g] < 5) list_a[atomicAdd(&s_na, 1)] = g;
-            }
-        }
-        __syncthreads();
+        held[g] = h;
     }
 }
 
@@ -456,9 +419,9 @@ static int obj_run(fse_world *w, fse_body *bodies, int n, int mode, int64_t *out
         bytes += (b + 255) & ~(size_t)255;
         return at;
     };
-    const size_t o_b = part(n * sizeof(fse_body)), o_pref = part((size_t)(n + 1) * 4), o_ptr = part(total * 4);
-    const size_t o_la = part(total * 4), o_lb = part(2 * total * 4), o_q = part(total * 4), o_held = part(total * 4);
-    const size_t o_blk = part(OBJ_BLOCKS * 4), o_na = part(4), o_rem = part(8);
+    const size_t o_b = part(n * sizeof(fse_body)), o_pref = part((size_t)(n + 1) * 4);
+    const size_t o_tiles = part(total * sizeof(ObjTile)), o_held = part(total * 4);
+    const size_t o_blk = part(OBJ_BLOCKS * 4), o_rem = part(8);
     if (w->obj_scr_bytes < bytes) {
         if (w->obj_scr) cudaFree(w->obj_scr);
         w->obj_scr = nullptr;
@@ -471,19 +434,18 @@ static int obj_run(fse_world *w, fse_body *bodies, int n, int mode, int64_t *out
     }
     uint8_t *s = w->obj_scr;
     fse_body *d_b = (fse_body *)(s + o_b);
-    uint32_t *d_pref = (uint32_t *)(s + o_pref), *d_ptr = (uint32_t *)(s + o_ptr), *d_la = (uint32_t *)(s + o_la);
-    uint32_t *d_lb = (uint32_t *)(s + o_lb), *d_q = (uint32_t *)(s + o_q);
-    int32_t *d_held = (int32_t *)(s + o_held), *d_blk = (int32_t *)(s + o_blk), *d_na = (int32_t *)(s + o_na);
+    uint32_t *d_pref = (uint32_t *)(s + o_pref);
+    ObjTile *d_tiles = (ObjTile *)(s + o_tiles);
+    int32_t *d_held = (int32_t *)(s + o_held), *d_blk = (int32_t *)(s + o_blk);
     long long *d_rem = (long long *)(s + o_rem), rem = 0;
     cudaMemcpyAsync(d_b, bodies, n * sizeof(fse_body), cudaMemcpyHostToDevice, w->stream);
     cudaMemcpyAsync(d_pref, prefix.data(), (size_t)(n + 1) * 4, cudaMemcpyHostToDevice, w->stream);
     cudaMemsetAsync(d_rem, 0, 8, w->stream);
     const int wide = (int)std::max<size_t>(1, std::min<size_t>((total + 255) / 256, (size_t)sm_count() * 8));
     const int blocks = (int)std::max<size_t>(1, std::min<size_t>((total + 1023) / 1024, OBJ_BLOCKS));
-    k_obj_first<<<wide, 256, 0, w->stream>>>(w->d, g_dev_mt, d_b, d_pref, n, d_ptr, d_held, d_q, w->claim, mode, d_na);
-    k_obj_losers<<<wide, 256, 0, w->stream>>>((uint32_t)total, d_ptr, d_held, d_la, w->claim, d_na);
-    k_obj_rounds<<<1, 1024, 0, w->stream>>>(w->d, g_dev_mt, d_b, d_pref, n, d_ptr, d_held, d_la, d_lb, d_q, w->claim,
-                                            mode, d_na);
+    k_obj_tiles<<<wide, 256, 0, w->stream>>>(w->d, g_dev_mt, d_b, d_pref, n, mode, d_tiles);
+    k_obj_settle<<<wide, 256, 0, w->stream>>>(w->d, (uint32_t)total, d_tiles, w->claim);
+    k_obj_held<<<wide, 256, 0, w->stream>>>(w->d, (uint32_t)total, d_tiles, w->claim, d_held);
     if (mode == 0)
         k_obj_count<<<blocks, 1024, 0, w->stream>>>(w->d, g_dev_mt, (uint32_t)total, d_held, d_blk);
     k_obj_apply<<<blocks, 1024, 0, w->stream>>>(w->d, g_dev_mt, d_b, d_pref, n, d_held, w->claim, mode, d_blk, d_rem);
