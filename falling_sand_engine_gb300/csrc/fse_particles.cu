@@ -166,16 +166,17 @@ __device__ __forceinline__ int32_t fill_code(int i) { return 0x7fffffff - i; }
 // the material particle i sees at cell c: the grid's, or the tile a particle of
 // lower index deposits there (fills are rewritten between iterations by other
 // blocks, so they are read past L1)
-__device__ __forceinline__ int view_id(const WorldDev &w, const uint8_t *s_type, int c, int i) {
-    int id = w.id[c];
-    if (s_type[id] == T_AIR) {
-        const int32_t v = __ldcg(&w.df[c]);
-        if (v != 0) {
-            const int j = 0x7fffffff - v;
-            if (j < i) id = w.p.id[j];
-        }
+// of a cell with grid material id and fill record v
+__device__ __forceinline__ int view_of(const WorldDev &w, const uint8_t *s_type, int id, int32_t v, int i) {
+    if (s_type[id] == T_AIR && v != 0) {
+        const int j = 0x7fffffff - v;
+        if (j < i) id = w.p.id[j];
     }
     return id;
+}
+__device__ __forceinline__ int view_id(const WorldDev &w, const uint8_t *s_type, int c, int i) {
+    const int id = w.id[c];
+    return view_of(w, s_type, id, __ldcg(&w.df[c]), i);
 }
 
 // which 8x8 blocks hold AIR, from the grid the cell tick left (one thread per block);
@@ -260,7 +261,28 @@ __device__ bool part_flight(const WorldDev &w, const uint8_t *s_type, int i) {
             const int div = (int)__fadd_rn(__fadd_rn(fabsf(vx), fabsf(vy)), 1.0f);
             const float dvx = __fdiv_rn(vx, (float)div), dvy = __fdiv_rn(vy, (float)div);
             int hit = 0;  // 1: deposit at the previous cell, 2: spiral search
+            // The cells of the next steps are read together, ids and fill records, before the
+            // steps are taken: a path does not depend on what it meets until it ends there, and
+            // read step by step each cell is a chain of two or three memory round trips.
+            constexpr int AHEAD = 4;
+            uint16_t aid[AHEAD];
+            int32_t adf[AHEAD];
             for (int s = 0; s < div; s++) {  // :2071-2184
+                if (s % AHEAD == 0) {
+                    float px = x, py = y;
+#pragma unroll
+                    for (int k = 0; k < AHEAD; k++) {
+                        px = __fadd_rn(px, dvx);
+                        py = __fadd_rn(py, dvy);
+                        aid[k] = 0;
+                        adf[k] = 0;
+                        if (s + k < div && !out_of_world(px, py, W, H)) {
+                            const int c = (int)py * W + (int)px;
+                            aid[k] = w.id[c];
+                            adf[k] = __ldcg(&w.df[c]);
+                        }
+                    }
+                }
                 x = __fadd_rn(x, dvx);
                 y = __fadd_rn(y, dvy);
                 if (out_of_world(x, y, W, H)) {
@@ -268,7 +290,15 @@ __device__ bool part_flight(const WorldDev &w, const uint8_t *s_type, int i) {
                     break;
                 }
                 bx.add((int)x, (int)y);
-                const int ct = s_type[view_id(w, s_type, (int)y * W + (int)x, i)];
+                int id = aid[0];
+                int32_t rec = adf[0];
+#pragma unroll
+                for (int k = 1; k < AHEAD; k++)
+                    if (s % AHEAD == k) {
+                        id = aid[k];
+                        rec = adf[k];
+                    }
+                const int ct = s_type[view_of(w, s_type, id, rec, i)];
                 if (!(bits & 1) && ct != T_AIR) {
                     const bool isObject = ct == T_OBJECT;
                     int ps = (bits >> 2) & 3;
@@ -380,7 +410,7 @@ struct GridBar {
 
 __device__ __forceinline__ void grid_sync(GridBar *gb, unsigned nblocks, int32_t *err) {
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (nblocks > 1 && threadIdx.x == 0) {
         volatile unsigned *vgen = &gb->gen;
         const unsigned g = *vgen;
         __threadfence();
@@ -405,6 +435,8 @@ __device__ __forceinline__ void grid_sync(GridBar *gb, unsigned nblocks, int32_t
 
 constexpr int SERIAL_MAX_ITER = 1 << 16;
 constexpr int SERIAL_MAX_WORLDS = 4096;  // worlds of one launch (a batch holds at most 4095)
+constexpr int ONE_BLOCK_PARTICLES = 4096;  // up to here the update runs in one block,
+constexpr int BLOCK_PARTICLES = 1024;      // beyond in one block for each so many particles
 constexpr int SERIAL_THREADS = 1024;  // one block per SM: 152 arrivals at each grid barrier
 
 // index g of a flattened index space: its entry in s_pref (prefix sums over the
@@ -451,6 +483,17 @@ __device__ __forceinline__ int block_excl_sum(int v, int *s_warp, int *total) {
 // s_apref[n_act] the total. Every thread of the block calls it; returns n_act.
 template <class F>
 __device__ int active_worlds(int n_worlds, F count, int *s_ids, int *s_apref, int *s_warp) {
+    if (n_worlds == 1) {  // no scans: their barriers would take most of a small update
+        const int c = count(0);
+        __syncthreads();  // the last index space has been used
+        if (threadIdx.x == 0) {
+            s_ids[0] = 0;
+            s_apref[0] = 0;
+            s_apref[c > 0 ? 1 : 0] = c;
+        }
+        __syncthreads();
+        return c > 0 ? 1 : 0;
+    }
     const int seg = (n_worlds + SERIAL_THREADS - 1) / SERIAL_THREADS;
     const int k0 = min((int)threadIdx.x * seg, n_worlds), k1 = min(k0 + seg, n_worlds);
     int sum = 0, nact = 0;
@@ -506,11 +549,17 @@ __global__ void __launch_bounds__(SERIAL_THREADS) k_part_serial(const WorldDev *
     __syncthreads();
     const int total = s_pref[n_worlds];
     auto parts = [&](int k) { return s_pref[k + 1] - s_pref[k]; };
+    // Small populations run on few blocks, and the fewest on one, whose barriers are the
+    // block's own: with all 152 blocks the ~30 grid barriers of an update cost more than
+    // its work.
+    const unsigned nb = min(gridDim.x, total <= ONE_BLOCK_PARTICLES
+                                           ? 1u
+                                           : (unsigned)(total + BLOCK_PARTICLES - 1) / BLOCK_PARTICLES);
+    if (blockIdx.x >= nb) return;
     GridBar *gb = (GridBar *)worlds[0].bar;
-    const unsigned nb = gridDim.x;
     int32_t *err = worlds[0].err;
     int32_t *cnt = worlds[0].req_count;
-    const int gtid = (int)(blockIdx.x * blockDim.x + threadIdx.x), gstride = (int)(gridDim.x * blockDim.x);
+    const int gtid = (int)(blockIdx.x * blockDim.x + threadIdx.x), gstride = (int)(nb * blockDim.x);
     const int lane = threadIdx.x & 31;
     int it = 0;
     for (;; it++) {
