@@ -274,12 +274,33 @@ __global__ void k_temp_commit(const WorldDev *__restrict__ worlds, int gated) {
     }
 }
 
-// per-cell temperature view <-> int16 buffer
-__global__ void k_temp_read(const WorldDev *__restrict__ wd, const MatTable *__restrict__ mt, int16_t *out) {
+// Per-cell temperature view -> int16 buffer, eight cells a thread in 16-byte accesses and
+// the types from shared memory. Bound by memory, 10 bytes a cell (id, scalar and tp read, the
+// view written); cell by cell with the type looked up in global memory it took 32 us for
+// 4096 x 2048 cells.
+__global__ void __launch_bounds__(256) k_temp_read(const WorldDev *__restrict__ wd, const MatTable *__restrict__ mt,
+                                                   int16_t *out) {
+    __shared__ uint8_t s_soup[MAXMAT];
+    for (int k = threadIdx.x; k < MAXMAT; k += blockDim.x) s_soup[k] = k < mt->n && mt_type(mt->a[k]) == T_SOUP;
+    __syncthreads();
     const WorldDev &w = *wd;
-    const size_t n = (size_t)w.W * w.H;
-    for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
-        out[i] = mt_type(mt->a[w.id[i]]) == T_SOUP ? (w.tp ? w.tp[i] : (int16_t)0) : (int16_t)w.sc[i];
+    const size_t n = (size_t)w.W * w.H, n8 = n / 8;
+    const size_t t0 = blockIdx.x * (size_t)blockDim.x + threadIdx.x, step = (size_t)gridDim.x * blockDim.x;
+    for (size_t k = t0; k < n8; k += step) {
+        const uint4 id = reinterpret_cast<const uint4 *>(w.id)[k];
+        const int4 lo = reinterpret_cast<const int4 *>(w.sc)[2 * k], hi = reinterpret_cast<const int4 *>(w.sc)[2 * k + 1];
+        const uint4 tp = w.tp ? reinterpret_cast<const uint4 *>(w.tp)[k] : make_uint4(0, 0, 0, 0);
+        // two cells a word
+        auto pair = [&](uint32_t i, uint32_t t, int a, int b) {
+            const uint32_t u = s_soup[i & 0xFF] ? t & 0xFFFFu : (uint32_t)a & 0xFFFFu;
+            const uint32_t v = s_soup[(i >> 16) & 0xFF] ? t >> 16 : (uint32_t)b & 0xFFFFu;
+            return u | (v << 16);
+        };
+        reinterpret_cast<uint4 *>(out)[k] = make_uint4(pair(id.x, tp.x, lo.x, lo.y), pair(id.y, tp.y, lo.z, lo.w),
+                                                       pair(id.z, tp.z, hi.x, hi.y), pair(id.w, tp.w, hi.z, hi.w));
+    }
+    for (size_t i = n8 * 8 + t0; i < n; i += step)
+        out[i] = s_soup[w.id[i] & 0xFF] ? (w.tp ? w.tp[i] : (int16_t)0) : (int16_t)w.sc[i];
 }
 __global__ void k_temp_write(const WorldDev *__restrict__ wd, const MatTable *__restrict__ mt, const int16_t *in) {
     const WorldDev &w = *wd;
