@@ -758,7 +758,7 @@ static void free_world(fse_world *w) {
     WorldDev &h = w->h;
     void *ptrs[] = {h.id, h.col, h.sc, h.fl, h.df, h.tp, h.tnew, h.stage, h.cp_count, h.cp_base, h.p_state, h.p_box0,
                     h.p_box1, h.p_cell, h.p_prev, h.chg, h.scan_tmp, h.ledger, h.airmap, w->ctr, w->d, w->claim,
-                    w->mask_bits, w->obj_list, w->obj_n, w->obj_scr, h.merge_list, h.merge_count, h.merge_claim, h.cdone};
+                    w->mask_bits, w->obj_list, w->obj_n, w->obj_scr, w->rec, h.merge_list, h.merge_count, h.merge_claim, h.cdone};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     PartSoA *ps[2] = {&h.p, &h.q};
@@ -1459,56 +1459,71 @@ int fse_particles_add(fse_world *w, const fse_particle *parts, int n) {
     return FSE_OK;
 }
 
+// n particles from index i0 on as fse_particle records: a block reads its 256 particles'
+// planes coalesced, turns them in shared memory (15 words a record: consecutive threads
+// write to different banks) and writes the records coalesced
+static_assert(sizeof(fse_particle) == 60, "15 words a record");
+__global__ void __launch_bounds__(256) k_part_records(const WorldDev *__restrict__ wd, int i0, int n, uint32_t *out) {
+    __shared__ uint32_t s[256 * 15];
+    const PartSoA &p = wd->p;
+    for (int b = blockIdx.x * 256; b < n; b += gridDim.x * 256) {
+        const int k = b + (int)threadIdx.x;
+        if (k < n) {
+            const int i = i0 + k;
+            uint32_t *r = s + threadIdx.x * 15;
+            r[0] = __float_as_uint(p.x[i]);
+            r[1] = __float_as_uint(p.y[i]);
+            r[2] = __float_as_uint(p.vx[i]);
+            r[3] = __float_as_uint(p.vy[i]);
+            r[4] = __float_as_uint(p.ax[i]);
+            r[5] = __float_as_uint(p.ay[i]);
+            r[6] = __float_as_uint(p.tx[i]);
+            r[7] = __float_as_uint(p.ty[i]);
+            r[8] = __float_as_uint(p.tf[i]);
+            r[9] = (uint32_t)p.life[i];
+            r[10] = (uint32_t)p.fade[i];
+            r[11] = p.col[i];
+            r[12] = (uint32_t)p.sc[i];
+            r[13] = (uint32_t)p.id[i] | ((uint32_t)p.fl[i] << 16) | ((uint32_t)p.bits[i] << 24);
+            r[14] = p.tp ? (uint32_t)(uint16_t)p.tp[i] : 0u;
+        }
+        __syncthreads();
+        const int words = min(256, n - b) * 15;
+        for (int j = threadIdx.x; j < words; j += 256) out[(size_t)b * 15 + j] = s[j];
+        __syncthreads();
+    }
+}
+
+// The records are made on the device and cross the link as they are, in pieces of at most
+// 15 MB. (Copying the 17 planes to host vectors and filling the records there took 6 ms
+// for half a million particles.)
 int fse_particles_read(fse_world *w, fse_particle *out, int cap, int *out_n) {
     if (!w || cap < 0 || (cap > 0 && !out)) return FSE_E_INVAL;
     int n;
     int rc = fse_particles_count(w, &n);
     if (rc) return rc;
     if (out_n) *out_n = n;
-    int m = std::min(n, cap);
+    const int m = std::min(n, cap);
     if (m == 0) return FSE_OK;
-    std::vector<float> f[9];
-    std::vector<int32_t> life(m), fade(m), sc(m);
-    std::vector<int16_t> tp(m);
-    std::vector<uint32_t> col(m);
-    std::vector<uint16_t> id(m);
-    std::vector<uint8_t> fl(m), bits(m);
-    PartSoA &P = w->h.p;
-    float *src[9] = {P.x, P.y, P.vx, P.vy, P.ax, P.ay, P.tx, P.ty, P.tf};
-    for (int k = 0; k < 9; k++) {
-        f[k].resize(m);
-        FSE_CUDA_TRY(cudaMemcpyAsync(f[k].data(), src[k], m * 4, cudaMemcpyDeviceToHost, w->stream));
+    const int piece = 1 << 18;
+    const size_t bytes = (size_t)std::min(m, piece) * sizeof(fse_particle);
+    if (w->rec_bytes < bytes) {
+        if (w->rec) cudaFree(w->rec);
+        w->rec = nullptr;
+        w->rec_bytes = 0;
+        if (cudaMalloc((void **)&w->rec, bytes) != cudaSuccess) {
+            w->rec = nullptr;
+            return FSE_E_NOMEM;
+        }
+        w->rec_bytes = bytes;
     }
-    FSE_CUDA_TRY(cudaMemcpyAsync(life.data(), P.life, m * 4, cudaMemcpyDeviceToHost, w->stream));
-    FSE_CUDA_TRY(cudaMemcpyAsync(fade.data(), P.fade, m * 4, cudaMemcpyDeviceToHost, w->stream));
-    FSE_CUDA_TRY(cudaMemcpyAsync(sc.data(), P.sc, m * 4, cudaMemcpyDeviceToHost, w->stream));
-    if (P.tp) FSE_CUDA_TRY(cudaMemcpyAsync(tp.data(), P.tp, m * 2, cudaMemcpyDeviceToHost, w->stream));
-    FSE_CUDA_TRY(cudaMemcpyAsync(col.data(), P.col, m * 4, cudaMemcpyDeviceToHost, w->stream));
-    FSE_CUDA_TRY(cudaMemcpyAsync(id.data(), P.id, m * 2, cudaMemcpyDeviceToHost, w->stream));
-    FSE_CUDA_TRY(cudaMemcpyAsync(fl.data(), P.fl, m, cudaMemcpyDeviceToHost, w->stream));
-    FSE_CUDA_TRY(cudaMemcpyAsync(bits.data(), P.bits, m, cudaMemcpyDeviceToHost, w->stream));
+    for (int i = 0; i < m; i += piece) {
+        const int k = std::min(piece, m - i);
+        k_part_records<<<std::min(ceil_div(k, 256), sm_count() * 4), 256, 0, w->stream>>>(w->d, i, k, w->rec);
+        FSE_CUDA_TRY(cudaGetLastError());
+        FSE_CUDA_TRY(cudaMemcpyAsync(out + i, w->rec, (size_t)k * sizeof(fse_particle), cudaMemcpyDeviceToHost, w->stream));
+    }
     FSE_CUDA_TRY(cudaStreamSynchronize(w->stream));
-    for (int i = 0; i < m; i++) {
-        fse_particle &p = out[i];
-        p.x = f[0][i];
-        p.y = f[1][i];
-        p.vx = f[2][i];
-        p.vy = f[3][i];
-        p.ax = f[4][i];
-        p.ay = f[5][i];
-        p.target_x = f[6][i];
-        p.target_y = f[7][i];
-        p.target_force = f[8][i];
-        p.lifetime = life[i];
-        p.fade_time = fade[i];
-        p.colour = col[i];
-        p.scalar = sc[i];
-        p.id = id[i];
-        p.flags = fl[i];
-        p.bits = bits[i];
-        p.temperature = tp[i];
-        p.reserved = 0;
-    }
     return FSE_OK;
 }
 

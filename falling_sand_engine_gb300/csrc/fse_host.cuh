@@ -54,6 +54,9 @@ struct fse_world {
     int64_t *obj_n;       // object list count
     uint8_t *obj_scr;     // stamp / readback workspace, grown on first use and kept until fse_world_trim
     size_t obj_scr_bytes;
+    // fse_particles_read's records, grown on first use (at most 15 MB) and kept until fse_world_trim
+    uint32_t *rec;
+    size_t rec_bytes;
     std::map<int, cudaGraphExec_t> graphs;  // n_ticks -> step graph
     std::map<int, long long> graph_kernels;  // n_ticks -> kernels one replay launches
     size_t bytes;         // device bytes owned

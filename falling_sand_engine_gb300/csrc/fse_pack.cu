@@ -895,6 +895,9 @@ int fse_world_trim(fse_world *w) {
     if (w->obj_scr) cudaFree(w->obj_scr);
     w->obj_scr = nullptr;
     w->obj_scr_bytes = 0;
+    if (w->rec) cudaFree(w->rec);
+    w->rec = nullptr;
+    w->rec_bytes = 0;
     return FSE_OK;
 }
 
