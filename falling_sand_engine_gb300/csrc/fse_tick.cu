@@ -1315,7 +1315,9 @@ static size_t tile_smem(int C, int own, int halo, int width) {
 // and writing back its own rows; sub-phases end with a cluster barrier. A chunk's
 // sub-phases then run on two SMs, and an SM holds halves of two chunks whose
 // barriers interleave.
-template <int HALO, bool TEMP, bool SEQ, bool F32, bool PAIR = false, bool FUSED = false>
+// CC: the chunk edge where it is known when compiling (128, the reference's), else 0:
+// the tile's rows, planes and lattices are then constants
+template <int HALO, bool TEMP, bool SEQ, bool F32, bool PAIR = false, bool FUSED = false, int CC = 0>
 __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 : 1)
     k_colour_pass(const WorldDev *__restrict__ worlds, const uint32_t *__restrict__ items, int n_items, int iter_arg,
                   int tk_arg, const MatTable *__restrict__ mt, const FusedTick ft) {
@@ -1482,7 +1484,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
             __syncthreads();
             continue;
         }
-        const int C = w.C, W = w.W, H = w.H;
+        const int C = CC ? CC : w.C, W = w.W, H = w.H;
         const int nb = (w.nCy - oy + 1) / 2;
         const int cx = w.zx + (ox + 2 * (slot / nb)) * C, cy = w.zy + (oy + 2 * (slot % nb)) * C;
         const uint32_t cp = (uint32_t)((iter * 4 + tk) * w.max_slots + slot);
@@ -1494,7 +1496,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
         TileData Tl;
         const bool tma = kTma && w.tmap != nullptr;
         // with TMA the rows start on a 16-byte boundary and are tma_tile_width wide
-        Tl.RW = tma ? tma_tile_width(C) : C + HALO_LO + HALO;
+        Tl.RW = CC || tma ? tma_tile_width(C) : C + HALO_LO + HALO;
         Tl.RHF = own + HALO_LO + HALO;
         Tl.RHI = own + HALO_LO + 10;
         Tl.x0 = tma ? ((cx - HALO_LO) & ~3) : cx - HALO_LO;
@@ -2080,33 +2082,52 @@ size_t colour_pass_smem(int C, int halo) {
 
 #endif
 
-template <int HALO, bool TEMP, bool SEQ = false, bool F32 = false>
-static cudaError_t launch_t(const WorldDev *worlds, const uint32_t *items, int n_items, int iter, int tk,
+template <int HALO, bool TEMP, bool SEQ = false, bool F32 = false, int CC = 0>
+static cudaError_t launch_cc(const WorldDev *worlds, const uint32_t *items, int n_items, int iter, int tk,
                             const MatTable *mt, size_t sm, int grid, cudaStream_t s) {
     // opt in to the full shared-memory carve-out once per instantiation
     static size_t set = 0;
     if (set < sm) {
-        cudaFuncSetAttribute(k_colour_pass<HALO, TEMP, SEQ, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaFuncSetAttribute(k_colour_pass<HALO, TEMP, SEQ, F32, false, false, CC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)sm);
         set = sm;
     }
-    k_colour_pass<HALO, TEMP, SEQ, F32><<<grid, CP_THREADS, sm, s>>>(worlds, items, n_items, iter, tk, mt,
+    k_colour_pass<HALO, TEMP, SEQ, F32, false, false, CC><<<grid, CP_THREADS, sm, s>>>(worlds, items, n_items, iter, tk, mt,
                                                                      FusedTick{});
     return cudaGetLastError();
 }
 
+// chunks of 128 with a 2-cell halo run the instantiation that knows its chunk edge
+template <int HALO, bool TEMP, bool SEQ = false, bool F32 = false>
+static cudaError_t launch_t(const WorldDev *worlds, const uint32_t *items, int n_items, int iter, int tk,
+                            const MatTable *mt, int C, size_t sm, int grid, cudaStream_t s) {
+    if constexpr (HALO == 2 && !SEQ) {
+        if (C == 128) return launch_cc<HALO, TEMP, SEQ, F32, 128>(worlds, items, n_items, iter, tk, mt, sm, grid, s);
+    }
+    return launch_cc<HALO, TEMP, SEQ, F32>(worlds, items, n_items, iter, tk, mt, sm, grid, s);
+}
+
 // the fused tick: one CTA per SM (the tile takes most of an SM's shared memory)
-template <int HALO, bool TEMP, bool F32>
-static cudaError_t launch_fused_t(const WorldDev *worlds, const FusedTick &ft, const MatTable *mt, size_t sm,
+template <int HALO, bool TEMP, bool F32, int CC>
+static cudaError_t launch_fused_cc(const WorldDev *worlds, const FusedTick &ft, const MatTable *mt, size_t sm,
                                   int grid, cudaStream_t s) {
     static size_t set = 0;
     if (set < sm) {
-        cudaFuncSetAttribute(k_colour_pass<HALO, TEMP, false, F32, false, true>,
+        cudaFuncSetAttribute(k_colour_pass<HALO, TEMP, false, F32, false, true, CC>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
         set = sm;
     }
-    k_colour_pass<HALO, TEMP, false, F32, false, true><<<grid, CP_THREADS, sm, s>>>(worlds, nullptr, 0, 0, 0, mt, ft);
+    k_colour_pass<HALO, TEMP, false, F32, false, true, CC><<<grid, CP_THREADS, sm, s>>>(worlds, nullptr, 0, 0, 0, mt, ft);
     return cudaGetLastError();
+}
+
+template <int HALO, bool TEMP, bool F32>
+static cudaError_t launch_fused_t(const WorldDev *worlds, const FusedTick &ft, const MatTable *mt, int C, size_t sm,
+                                  int grid, cudaStream_t s) {
+    if constexpr (HALO == 2) {
+        if (C == 128) return launch_fused_cc<HALO, TEMP, F32, 128>(worlds, ft, mt, sm, grid, s);
+    }
+    return launch_fused_cc<HALO, TEMP, F32, 0>(worlds, ft, mt, sm, grid, s);
 }
 
 // shared memory of one CTA of a pair: half the chunk's rows plus the reach of its rules
@@ -2156,11 +2177,11 @@ cudaError_t launch_colour_fused(const WorldDev *worlds, const FusedTick &ft, con
 #endif
     const size_t sm = colour_pass_smem(C, halo);
     if (temp) {
-        if (halo == 5) return launch_fused_t<5, true, FSE_FUSED_F32>(worlds, ft, mt, sm, grid, s);
-        return launch_fused_t<2, true, FSE_FUSED_F32>(worlds, ft, mt, sm, grid, s);
+        if (halo == 5) return launch_fused_t<5, true, FSE_FUSED_F32>(worlds, ft, mt, C, sm, grid, s);
+        return launch_fused_t<2, true, FSE_FUSED_F32>(worlds, ft, mt, C, sm, grid, s);
     }
-    if (halo == 5) return launch_fused_t<5, false, FSE_FUSED_F32>(worlds, ft, mt, sm, grid, s);
-    return launch_fused_t<2, false, FSE_FUSED_F32>(worlds, ft, mt, sm, grid, s);
+    if (halo == 5) return launch_fused_t<5, false, FSE_FUSED_F32>(worlds, ft, mt, C, sm, grid, s);
+    return launch_fused_t<2, false, FSE_FUSED_F32>(worlds, ft, mt, C, sm, grid, s);
 }
 #elif defined(FSE_TICK_PAIR_TU)
 // chunks split over CTA pairs, Q16.16 amounts (FSE_TICK_PAIR_TU = 1) or f32 (2)
@@ -2187,43 +2208,43 @@ cudaError_t launch_colour_pass_pair(const WorldDev *worlds, const uint32_t *item
 #define FSE_F32_SEQ (FSE_TICK_F32_TU == 2)
 #if FSE_TICK_F32_TU == 2
 cudaError_t launch_colour_pass_f32_seq(const WorldDev *worlds, const uint32_t *items, int n_items, int iter, int tk,
-                                       const MatTable *mt, int halo, size_t sm, int grid, cudaStream_t s, bool temp) {
+                                       const MatTable *mt, int halo, int C, size_t sm, int grid, cudaStream_t s, bool temp) {
 #else
 cudaError_t launch_colour_pass_f32(const WorldDev *worlds, const uint32_t *items, int n_items, int iter, int tk,
-                                   const MatTable *mt, int halo, size_t sm, int grid, cudaStream_t s, bool temp) {
+                                   const MatTable *mt, int halo, int C, size_t sm, int grid, cudaStream_t s, bool temp) {
 #endif
     if (temp) {
-        if (halo == 5) return launch_t<5, true, FSE_F32_SEQ, true>(worlds, items, n_items, iter, tk, mt, sm, grid, s);
-        return launch_t<2, true, FSE_F32_SEQ, true>(worlds, items, n_items, iter, tk, mt, sm, grid, s);
+        if (halo == 5) return launch_t<5, true, FSE_F32_SEQ, true>(worlds, items, n_items, iter, tk, mt, C, sm, grid, s);
+        return launch_t<2, true, FSE_F32_SEQ, true>(worlds, items, n_items, iter, tk, mt, C, sm, grid, s);
     }
-    if (halo == 5) return launch_t<5, false, FSE_F32_SEQ, true>(worlds, items, n_items, iter, tk, mt, sm, grid, s);
-    return launch_t<2, false, FSE_F32_SEQ, true>(worlds, items, n_items, iter, tk, mt, sm, grid, s);
+    if (halo == 5) return launch_t<5, false, FSE_F32_SEQ, true>(worlds, items, n_items, iter, tk, mt, C, sm, grid, s);
+    return launch_t<2, false, FSE_F32_SEQ, true>(worlds, items, n_items, iter, tk, mt, C, sm, grid, s);
 }
 #elif defined(FSE_TICK_SEQ_TU)
 cudaError_t launch_colour_pass_seq(const WorldDev *worlds, const uint32_t *items, int n_items, int iter, int tk,
-                                   const MatTable *mt, int halo, size_t sm, int grid, cudaStream_t s, bool temp) {
+                                   const MatTable *mt, int halo, int C, size_t sm, int grid, cudaStream_t s, bool temp) {
     if (temp) {
-        if (halo == 5) return launch_t<5, true, true>(worlds, items, n_items, iter, tk, mt, sm, grid, s);
-        return launch_t<2, true, true>(worlds, items, n_items, iter, tk, mt, sm, grid, s);
+        if (halo == 5) return launch_t<5, true, true>(worlds, items, n_items, iter, tk, mt, C, sm, grid, s);
+        return launch_t<2, true, true>(worlds, items, n_items, iter, tk, mt, C, sm, grid, s);
     }
-    if (halo == 5) return launch_t<5, false, true>(worlds, items, n_items, iter, tk, mt, sm, grid, s);
-    return launch_t<2, false, true>(worlds, items, n_items, iter, tk, mt, sm, grid, s);
+    if (halo == 5) return launch_t<5, false, true>(worlds, items, n_items, iter, tk, mt, C, sm, grid, s);
+    return launch_t<2, false, true>(worlds, items, n_items, iter, tk, mt, C, sm, grid, s);
 }
 #elif defined(FSE_TICK_TEMP_TU)
 cudaError_t launch_colour_pass_temp(const WorldDev *worlds, const uint32_t *items, int n_items, int iter, int tk,
-                                    const MatTable *mt, int halo, size_t sm, int grid, cudaStream_t s) {
-    if (halo == 5) return launch_t<5, true>(worlds, items, n_items, iter, tk, mt, sm, grid, s);
-    return launch_t<2, true>(worlds, items, n_items, iter, tk, mt, sm, grid, s);
+                                    const MatTable *mt, int halo, int C, size_t sm, int grid, cudaStream_t s) {
+    if (halo == 5) return launch_t<5, true>(worlds, items, n_items, iter, tk, mt, C, sm, grid, s);
+    return launch_t<2, true>(worlds, items, n_items, iter, tk, mt, C, sm, grid, s);
 }
 #else
 cudaError_t launch_colour_pass_temp(const WorldDev *worlds, const uint32_t *items, int n_items, int iter, int tk,
-                                    const MatTable *mt, int halo, size_t sm, int grid, cudaStream_t s);
+                                    const MatTable *mt, int halo, int C, size_t sm, int grid, cudaStream_t s);
 cudaError_t launch_colour_pass_seq(const WorldDev *worlds, const uint32_t *items, int n_items, int iter, int tk,
-                                   const MatTable *mt, int halo, size_t sm, int grid, cudaStream_t s, bool temp);
+                                   const MatTable *mt, int halo, int C, size_t sm, int grid, cudaStream_t s, bool temp);
 cudaError_t launch_colour_pass_f32(const WorldDev *worlds, const uint32_t *items, int n_items, int iter, int tk,
-                                   const MatTable *mt, int halo, size_t sm, int grid, cudaStream_t s, bool temp);
+                                   const MatTable *mt, int halo, int C, size_t sm, int grid, cudaStream_t s, bool temp);
 cudaError_t launch_colour_pass_f32_seq(const WorldDev *worlds, const uint32_t *items, int n_items, int iter, int tk,
-                                       const MatTable *mt, int halo, size_t sm, int grid, cudaStream_t s, bool temp);
+                                       const MatTable *mt, int halo, int C, size_t sm, int grid, cudaStream_t s, bool temp);
 
 cudaError_t launch_colour_pass_pair(const WorldDev *worlds, const uint32_t *items, int n_items, int iter, int tk,
                                     const MatTable *mt, int halo, int C, int clusters, cudaStream_t s, bool temp);
@@ -2243,12 +2264,12 @@ cudaError_t launch_colour_pass(const WorldDev *worlds, const uint32_t *items, in
         if (f32) return launch_colour_pass_pair_f32(worlds, items, n_items, iter, tk, mt, halo, C, grid, s, temp);
         return launch_colour_pass_pair(worlds, items, n_items, iter, tk, mt, halo, C, grid, s, temp);
     }
-    if (f32 && seq) return launch_colour_pass_f32_seq(worlds, items, n_items, iter, tk, mt, halo, sm, grid, s, temp);
-    if (f32) return launch_colour_pass_f32(worlds, items, n_items, iter, tk, mt, halo, sm, grid, s, temp);
-    if (seq) return launch_colour_pass_seq(worlds, items, n_items, iter, tk, mt, halo, sm, grid, s, temp);
-    if (temp) return launch_colour_pass_temp(worlds, items, n_items, iter, tk, mt, halo, sm, grid, s);
-    if (halo == 5) return launch_t<5, false>(worlds, items, n_items, iter, tk, mt, sm, grid, s);
-    return launch_t<2, false>(worlds, items, n_items, iter, tk, mt, sm, grid, s);
+    if (f32 && seq) return launch_colour_pass_f32_seq(worlds, items, n_items, iter, tk, mt, halo, C, sm, grid, s, temp);
+    if (f32) return launch_colour_pass_f32(worlds, items, n_items, iter, tk, mt, halo, C, sm, grid, s, temp);
+    if (seq) return launch_colour_pass_seq(worlds, items, n_items, iter, tk, mt, halo, C, sm, grid, s, temp);
+    if (temp) return launch_colour_pass_temp(worlds, items, n_items, iter, tk, mt, halo, C, sm, grid, s);
+    if (halo == 5) return launch_t<5, false>(worlds, items, n_items, iter, tk, mt, C, sm, grid, s);
+    return launch_t<2, false>(worlds, items, n_items, iter, tk, mt, C, sm, grid, s);
 }
 #endif
 
