@@ -324,16 +324,19 @@ struct Tile : TileData {
         set_planes(i, sc, col);
     }
     __device__ __forceinline__ void set_nothing(int i) const { put_dry(i, mw[id_air], 0, 0); }
-    // write the cell at s over d; the visited mark stays with the position
-    __device__ __forceinline__ void move(int d, int dg, int s, int sg) const {
-        const uint32_t v = s_w[s];
+    // write the cell at s, of word v and (a SOUP cell) pending diff dfv, over d; the visited
+    // mark stays with the position
+    __device__ __forceinline__ void move(int d, int dg, int s, int sg, uint32_t v, int32_t dfv) const {
         set_word(d, (v & ~CW_VIS) | CW_DIRTY | (s_w[d] & CW_VIS));
         set_planes(d, s_sc[s], s_col[s]);
         if (cw_is(v, T_SOUP)) {
-            df[dg] = df[sg];
+            df[dg] = dfv;
             if (TEMP && tp) tp[dg] = tp[sg];
         }
     }
+    // the pending diff of the cell of word v at g, if it is SOUP (it comes from HBM: load it
+    // well before its use)
+    __device__ __forceinline__ int32_t df_if_soup(uint32_t v, int g) const { return cw_is(v, T_SOUP) ? df[g] : 0; }
     // Temperatures of SOUP cells live in HBM beside the diff; the tile's scalar is
     // their amount. They move only where a SOUP cell moves or is made, so the
     // rules touch them at those few places and nowhere else.
@@ -382,6 +385,9 @@ struct Ctx {
     // member whose address escapes keeps the whole context in local memory
     SpawnEv *ev;
     int ev_n;  // particles the cell emits (0: none)
+    // the pending diff that a liquid in free fall loses: counted when its particles are
+    // emitted, so that the rule does not wait for the load
+    int32_t ev_df;
     // start the draws of the cell at (x, y); most cells never draw, so the key
     // (two hash rounds) is computed only when the first draw needs it
     __device__ __forceinline__ void at(int x, int y) {
@@ -523,7 +529,7 @@ template <class TL>
 __device__ __forceinline__ void swap_liquid(const TL &T, uint32_t w0, int32_t sc, uint32_t col, int32_t diff, int i,
                                             int g, int n, int gn) {
     const int16_t tv = T.tp_load(g);
-    T.move(i, g, n, gn);
+    T.move(i, g, n, gn, T.at(n), T.df_load(gn));
     Cell t;
     t.w = w0;
     t.sc = sc;
@@ -603,7 +609,8 @@ __device__ __forceinline__ uint32_t settle_word(uint32_t w0) {
 }
 
 // ------------------------------------------------- sweep A, liquids
-// world.cpp:1269-1567. The neighbours are read first, all together (nothing the cell
+// world.cpp:1269-1567 but for the free fall (class_a finds the cells in free fall, and leaves
+// out those that have settled). The neighbours are read first, all together (nothing the cell
 // writes before it reads them is among them: a flow writes only the cell it enters).
 // Q16.16 amounts, or with F32 the reference's own float amounts: the same branches
 // in f32 with every operation rounded on its own, and the cell's fluidAmountDiff read
@@ -625,15 +632,6 @@ __device__ __forceinline__ void rule_a_soup(const TL &T, Ctx &c, uint32_t w0, in
     const uint32_t wb = T.at(i + RW);
     const bool airBelow = cw_air(wb);
     const int g = T.gi(x, y);
-    if (airBelow && sc > Q_FREEFALL) {
-        const uint32_t w2 = T.at(i + 2 * RW), w3 = T.at(i + 3 * RW), w4 = T.at(i + 4 * RW);
-        if (cw_air(w2) && cw_air(w3) && cw_air(w4)) {
-            led_add64(c, LED_DF, w0, T.df_load(g));
-            free_fall(T, c, w0, sc, col, sc >> 18, i, g, x, y);
-            return;
-        }
-    }
-    if (w0 & CW_MOVED) return;
     const uint32_t wl = T.at(i - 1), wr = T.at(i + 1), wt = T.at(i - RW);
     const int32_t sb = T.s_sc[i + RW], sl = T.s_sc[i - 1], sr = T.s_sc[i + 1], su = T.s_sc[i - RW];
     int32_t rem = sc, down = 0, left = 0, right = 0, up = 0;
@@ -737,15 +735,6 @@ __device__ __forceinline__ void rule_a_soup_f32(const TL &T, Ctx &c, uint32_t w0
     const uint32_t wb = T.at(i + RW);
     const bool airBelow = cw_air(wb);
     const int g = T.gi(x, y);
-    // tile.fluidAmount > 0.005 compares in double (0.005 is a double literal)
-    if (airBelow && (double)amount > 0.005) {
-        const uint32_t w2 = T.at(i + 2 * RW), w3 = T.at(i + 3 * RW), w4 = T.at(i + 4 * RW);
-        if (cw_air(w2) && cw_air(w3) && cw_air(w4)) {
-            free_fall(T, c, w0, sc, col, (int)__fdiv_rn(amount, 4.0f), i, g, x, y);  // int n = tile.fluidAmount / 4
-            return;
-        }
-    }
-    if (w0 & CW_MOVED) return;
     float dfv = __int_as_float(T.df_load(g));
     const uint32_t wl = T.at(i - 1), wr = T.at(i + 1), wt = T.at(i - RW);
     const float sb = __int_as_float(T.s_sc[i + RW]), sl = __int_as_float(T.s_sc[i - 1]);
@@ -930,7 +919,8 @@ __device__ __forceinline__ bool rule_a_react(const TL &T, Ctx &c, uint32_t w0, i
 
 // ----------------------------------------------------------------- sweep A
 // Whether sweep A may change cell i (a superset of the cells that its rule changes):
-// 0 no, 1 a liquid, 2 another cell. Cells whose material is not updated in this
+// 0 no, 1 a liquid, 2 another cell or a liquid in free fall (world.cpp:1283-1305), so that
+// the warps of liquids that flow do not take the long way through an emission. Cells whose material is not updated in this
 // iteration are marked visited here (world.cpp:1093-1096).
 template <class TL>
 __device__ __forceinline__ int class_a(const TL &T, const Ctx &c, int i) {
@@ -943,13 +933,22 @@ __device__ __forceinline__ int class_a(const TL &T, const Ctx &c, int i) {
     const uint32_t wn = T.at(cw_is(w0, T_GAS) ? i - T.RW : i + T.RW);
     if (cw_is(w0, T_SOUP)) {
         const int32_t sc = T.s_sc[i];
-        // a settled liquid only falls or dries up
-        bool small;
-        if constexpr (TL::kF32)
-            small = __int_as_float(sc) < F_MINV;
-        else
+        bool none, small, fall;
+        if constexpr (TL::kF32) {
+            const float amount = __int_as_float(sc);
+            none = amount == 0.0f;
+            small = amount < F_MINV;
+            // tile.fluidAmount > 0.005 compares in double (0.005 is a double literal)
+            fall = cw_air(wn) && (double)amount > 0.005;
+        } else {
+            none = sc == 0;
             small = sc < Q_MINV;
-        return sc != 0 && (!(w0 & CW_MOVED) || cw_air(wn) || small) ? 1 : 0;
+            fall = cw_air(wn) && sc > Q_FREEFALL;
+        }
+        if (none) return 0;
+        if (fall) fall = cw_air(T.at(i + 2 * T.RW) | T.at(i + 3 * T.RW) | T.at(i + 4 * T.RW));
+        // a settled liquid only falls or dries up
+        return small ? 1 : (fall ? 2 : (w0 & CW_MOVED ? 0 : 1));
     }
     bool act = (w0 & CW_FIRE) != 0;
     if (cw_is(w0, T_SAND)) act = c.has_inter || (w0 & CW_REACT) || wn < cw_sink(w0);
@@ -957,16 +956,17 @@ __device__ __forceinline__ int class_a(const TL &T, const Ctx &c, int i) {
     return act ? 2 : 0;
 }
 
-// c.ev_n: the particles the cell emits (its event in *c.ev)
+// the rules: c.ev_n = the particles the cell emits (its event in *c.ev)
 template <class TL>
-__device__ __forceinline__ void rule_a(const TL &T, Ctx &c, int i, int x, int y) {
-    const uint32_t w0 = T.at(i);
-    if (w0 & CW_VIS) return;  // world.cpp:1091
-    if (!(w0 & CW_LIVE)) {    // world.cpp:1093-1096
-        T.set_word(i, w0 | CW_VIS);
-        return;
-    }
-    c.at(x, y);
+__device__ __forceinline__ void rule_a_liquid(const TL &T, Ctx &c, uint32_t w0, int i, int x, int y) {
+    if constexpr (TL::kF32)
+        rule_a_soup_f32(T, c, w0, i, x, y);
+    else
+        rule_a_soup(T, c, w0, i, x, y);
+}
+// a cell of class 2, of word w0
+template <class TL>
+__device__ __forceinline__ void rule_a(const TL &T, Ctx &c, uint32_t w0, int i, int x, int y) {
     if (w0 & CW_FIRE) rule_a_fire(T, c, w0, i, x, y);
     if (cw_is(w0, T_SAND)) {
         const uint32_t wb = T.at(i + T.RW);  // world.cpp:1150
@@ -975,9 +975,11 @@ __device__ __forceinline__ void rule_a(const TL &T, Ctx &c, int i, int x, int y)
         if ((w0 & CW_REACT) && rule_a_react(T, c, w0, i, x, y)) return;
         // world.cpp:1206-1267
         if (!(wb < lim)) return;
+        const int g = T.gi(x, y);
+        const int32_t dfb = T.df_if_soup(wb, g + T.W);
         const bool canL = T.at(i + T.RW - 1) < lim, canR = T.at(i + T.RW + 1) < lim;
         if (!((canL || canR) && c.D() % 20 == 0)) {
-            const int g = T.gi(x, y), n = i + T.RW;
+            const int n = i + T.RW;
             const int32_t sc = T.s_sc[i];
             const uint32_t col = T.s_col[i];
             bool falls = cw_air(wb);
@@ -985,7 +987,7 @@ __device__ __forceinline__ void rule_a(const TL &T, Ctx &c, int i, int x, int y)
                 const uint32_t w2 = T.at(i + 2 * T.RW), w3 = T.at(i + 3 * T.RW), w4 = T.at(i + 4 * T.RW);
                 falls = cw_air(w2) && cw_air(w3) && cw_air(w4);
             }
-            T.move(i, g, n, g + T.W);
+            T.move(i, g, n, g + T.W, wb, dfb);
             if (falls) {
                 float vx = (float)((int)(c.D() % 10) - 5) / 20.0f;
                 float vy = (float)(-((int)(c.D() % 2) + 3)) / 10.0f + 1.5f;
@@ -1004,11 +1006,15 @@ __device__ __forceinline__ void rule_a(const TL &T, Ctx &c, int i, int x, int y)
                 }
             }
         }
-    } else if (cw_is(w0, T_SOUP)) {
-        if constexpr (TL::kF32)
-            rule_a_soup_f32(T, c, w0, i, x, y);
-        else
-            rule_a_soup(T, c, w0, i, x, y);
+    } else if (cw_is(w0, T_SOUP)) {  // in free fall
+        const int g = T.gi(x, y);
+        const int32_t sc = T.s_sc[i];
+        if constexpr (TL::kF32) {
+            free_fall(T, c, w0, sc, T.s_col[i], (int)__fdiv_rn(__int_as_float(sc), 4.0f), i, g, x, y);  // int n = tile.fluidAmount / 4
+        } else {
+            c.ev_df = T.df_load(g);
+            free_fall(T, c, w0, sc, T.s_col[i], sc >> 18, i, g, x, y);
+        }
     } else if (cw_is(w0, T_GAS)) {  // world.cpp:1569-1585
         const int n = i - T.RW;
         const uint32_t above = T.at(n), aboveL = T.at(n - 1), aboveR = T.at(n + 1);
@@ -1072,8 +1078,10 @@ __device__ __forceinline__ void rule_b(const TL &T, Ctx &c, uint32_t w0, int i, 
     if (cw_is(w0, T_SAND)) {  // world.cpp:1602-1727
         const int RW = T.RW;
         const uint32_t lim = cw_sink(w0);
-        const bool canL = T.at(i + RW - 1) < lim;
-        const bool canR = T.at(i + RW + 1) < lim;
+        const uint32_t wl = T.at(i + RW - 1), wr = T.at(i + RW + 1);
+        const bool canL = wl < lim, canR = wr < lim;
+        const int g = T.gi(x, y);
+        const int32_t dfl = canL ? T.df_if_soup(wl, g + T.W - 1) : 0, dfr = canR ? T.df_if_soup(wr, g + T.W + 1) : 0;
         bool stopped = !(w0 & CW_MOVED);
         c.at(x, y);
         const int a = c.fr[cw_id(w0)];
@@ -1097,7 +1105,6 @@ __device__ __forceinline__ void rule_b(const TL &T, Ctx &c, uint32_t w0, int i, 
         }
         // the moving cell as it was when its turn began
         uint32_t t = w0;
-        const int g = T.gi(x, y);
         const int32_t sc = T.s_sc[i];
         const uint32_t col = T.s_col[i];
         const int slip = a & 0xFF;
@@ -1116,12 +1123,14 @@ __device__ __forceinline__ void rule_b(const TL &T, Ctx &c, uint32_t w0, int i, 
         }
         const int o = goL ? -1 : 1;  // towards the left or the right
         const int s = i + o, d = i + RW + o, gd = g + T.W + o;
+        const uint32_t wd = T.at(d);
+        const int32_t dfd = goL ? dfl : dfr;
         if (T.air(s)) {
-            T.move(s, g + o, d, gd);
+            T.move(s, g + o, d, gd, wd, dfd);
             if (goL) T.setvis(s);
             T.set_nothing(i);
         } else {
-            T.move(i, g, d, gd);
+            T.move(i, g, d, gd, wd, dfd);
             T.setvis(i);
         }
         if (slip > 0 && c.D() % (uint32_t)(20 * slip) == 0) t &= ~CW_MOVED;
@@ -1718,8 +1727,14 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                         const int x = cx + dx, y = cy + dy, i = Tl.li(x, y);
                         if (sweep == 0) {
                             c.ev_n = 0;
-                            rule_a(Tl, c, i, x, y);
+                            c.at(x, y);
+                            const int cls = class_a(Tl, c, i);
+                            if (cls == 1)
+                                rule_a_liquid(Tl, c, Tl.at(i), i, x, y);
+                            else if (cls == 2)
+                                rule_a(Tl, c, Tl.at(i), i, x, y);
                             if (c.ev_n > 0) {
+                                if (!F32 && c.ev->kind == 2) led_add64(c, LED_DF, S.mw[c.ev->id], c.ev_df);
                                 const int base = atomicAdd(w.stage_count, c.ev_n);
                                 emit_spawns<TEMP, F32>(w, *c.ev, c.ev_n, cp * (uint32_t)w.cp_rows + (uint32_t)k,
                                                        (uint32_t)spawned, base);
@@ -1809,10 +1824,17 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                         FSE_PT(2)
                         c.ev_n = 0;
                         int e = 0;
-                        if (tid < (int)(nl & 0xFFFF) || tid >= T - (int)(nl >> 16)) {
+                        const bool liquid = tid < (int)(nl & 0xFFFF);
+                        if (liquid || tid >= T - (int)(nl >> 16)) {
                             const int item = S.list[tid];
                             const int ix = item & 0xFF, iy = item >> 8;
-                            rule_a(Tl, c, Tl.li(cx + ix, cy + iy), cx + ix, cy + iy);
+                            const int x = cx + ix, y = cy + iy, i = Tl.li(x, y);
+                            const uint32_t w0 = Tl.at(i);
+                            c.at(x, y);
+                            if (liquid)
+                                rule_a_liquid(Tl, c, w0, i, x, y);
+                            else
+                                rule_a(Tl, c, w0, i, x, y);
                             if (c.ev_n > 0) {
                                 int qe, re, t_;
                                 divmod_small(iy - dyb, py, __frcp_rn((float)py), qe, t_);
@@ -1825,17 +1847,16 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                         __syncwarp();
                         const int lane = tid & 31, wid = tid >> 5;
                         const unsigned sp = __ballot_sync(0xffffffffu, c.ev_n > 0);
-                        int slot = 0;
+                        int slot = 0, spi = 0;
                         seq++;
                         if (sp) {
-                            int inc = c.ev_n;
+                            spi = c.ev_n;
 #pragma unroll
                             for (int o = 1; o < 32; o <<= 1) {
-                                const int t = __shfl_up_sync(0xffffffffu, inc, o);
-                                if (lane >= o) inc += t;
+                                const int t = __shfl_up_sync(0xffffffffu, spi, o);
+                                if (lane >= o) spi += t;
                             }
-                            if (lane == 31) slot = atomicAdd(w.stage_count, inc);
-                            slot = __shfl_sync(0xffffffffu, slot, 31) + inc - c.ev_n;
+                            if (lane == 31) slot = atomicAdd(w.stage_count, spi);
                             if (c.ev_n > 0) atomicOr(&S.spawn_bits[sub][e >> 5], 1u << (e & 31));
                             if (c.ev_n > 1) S.many = seq;
                         }
@@ -1898,7 +1919,13 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                             running += tot_p;
                         }
                         // the (chunk-pass, rank) key orders the particles later
-                        if (c.ev_n > 0) emit_spawns<TEMP, F32>(w, *c.ev, c.ev_n, cp, (uint32_t)(before + rank_e), slot);
+                        if (sp) {
+                            slot = __shfl_sync(0xffffffffu, slot, 31) + spi - c.ev_n;
+                            if (c.ev_n > 0) {
+                                emit_spawns<TEMP, F32>(w, *c.ev, c.ev_n, cp, (uint32_t)(before + rank_e), slot);
+                                if (!F32 && c.ev->kind == 2) led_add64(c, LED_DF, S.mw[c.ev->id], c.ev_df);
+                            }
+                        }
                         running += tot;
                         FSE_PT(4)
                     } else if (sweep == 1) {
