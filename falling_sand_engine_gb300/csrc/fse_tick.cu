@@ -119,18 +119,6 @@ struct Cell {
     int32_t df;
 };
 
-struct SpawnEv {
-    int kind;  // 1 sand, 2 soup, 3 fire
-    int x, y;
-    uint16_t id;
-    uint8_t fl;
-    uint32_t col;
-    int32_t sc;
-    float vx, vy;
-    uint32_t ck, k0;
-    int16_t tp;  // temperature of a SOUP tile (kind 2; set only where temperatures are kept)
-};
-
 // ------------------------------------------------------- shared-memory tile
 // Region: x in [cx - 2, cx + C + HALO), full state for y in [cy - 2, cy + C + HALO),
 // words only down to y < cy + C + 10 (the deepest read, the friction pillar of
@@ -381,9 +369,13 @@ struct Ctx {
     long long *led_g;      // global ledger [LED_ROWS][MAXMAT]
     const uint32_t *mw;    // material words (shared)
     const uint16_t *fr;    // slipperiness | stability << 8 (shared)
-    // the cell's spawn event, a local of its own: emit_spawns takes its address, and a
-    // member whose address escapes keeps the whole context in local memory
-    SpawnEv *ev;
+    // the cell's spawn event: its particles' kind (1 sand, 2 soup, 3 fire), id and flags as
+    // in their records, colour, scalar, temperature, and the velocity of the first
+    int ev_kind;
+    uint32_t ev_idfl, ev_col;
+    int32_t ev_sc;
+    float ev_vx, ev_vy;
+    int16_t ev_tp;
     int ev_n;  // particles the cell emits (0: none)
     // the pending diff that a liquid in free fall loses: counted when its particles are
     // emitted, so that the rule does not wait for the load
@@ -563,18 +555,34 @@ __device__ __forceinline__ void water_on_lava(const TL &T, Ctx &c, uint32_t w0, 
         }
 }
 
-__device__ __forceinline__ void spawn_one(Ctx &c, int kind, int x, int y, uint32_t w, int32_t sc, uint32_t col,
-                                          float vx, float vy) {
+// velocities of spawned particles by their draws, as the reference's divisions give them
+// (world.cpp:1222,1298; divided once per CTA, as a division is a dozen instructions)
+struct SpawnVel {
+    float sand_vx[10];  // (k - 5) / 20.0f
+    float soup_vx[10];  // (k - 5) / 30.0f
+    float sand_vy[2];   // -(k + 3) / 10.0f + 1.5f
+    float soup_vy[2];   // -(k + 3) / 10.0f + 1.0f
+};
+__shared__ SpawnVel s_vel;
+__device__ __forceinline__ void spawn_vel_init(int tid) {
+    if (tid < 10) {
+        s_vel.sand_vx[tid] = (float)(tid - 5) / 20.0f;
+        s_vel.soup_vx[tid] = (float)(tid - 5) / 30.0f;
+    }
+    if (tid < 2) {
+        s_vel.sand_vy[tid] = (float)(-(tid + 3)) / 10.0f + 1.5f;
+        s_vel.soup_vy[tid] = (float)(-(tid + 3)) / 10.0f + 1.0f;
+    }
+}
+
+__device__ __forceinline__ void spawn_one(Ctx &c, int kind, uint32_t w, int32_t sc, uint32_t col, float vx, float vy) {
     c.ev_n = 1;
-    c.ev->kind = kind;
-    c.ev->x = x;
-    c.ev->y = y;
-    c.ev->id = (uint16_t)cw_id(w);
-    c.ev->fl = (uint8_t)((w & (CW_FLAGS & ~CW_VIS)) >> 8);
-    c.ev->col = col;
-    c.ev->sc = sc;
-    c.ev->vx = vx;
-    c.ev->vy = vy;
+    c.ev_kind = kind;
+    c.ev_idfl = (w & CW_ID) | ((w & (CW_FLAGS & ~CW_VIS)) << 8);
+    c.ev_col = col;
+    c.ev_sc = sc;
+    c.ev_vx = vx;
+    c.ev_vy = vy;
 }
 
 // a liquid cell in free fall becomes n particles (world.cpp:1283-1305)
@@ -585,16 +593,14 @@ __device__ __forceinline__ void free_fall(const TL &T, Ctx &c, uint32_t w0, int3
     if (n < 1) n = 1;
     led_add(c, LED_CN, w0, n - 1);
     c.ev_n = n;
-    c.ev->kind = 2;
-    c.ev->x = x;
-    c.ev->y = y + 1;
-    c.ev->id = (uint16_t)cw_id(w0);
-    c.ev->fl = 0;
-    c.ev->col = col;
-    c.ev->sc = sc;
-    if (TL::kTemp) c.ev->tp = T.tp_load(g);
-    c.ev->ck = c.key();
-    c.ev->k0 = c.k;
+    c.ev_kind = 2;
+    c.ev_idfl = w0 & CW_ID;
+    c.ev_col = col;
+    c.ev_sc = sc;
+    if (TL::kTemp) c.ev_tp = T.tp_load(g);
+    // the cell's first draws (its other particles draw theirs when they are written)
+    c.ev_vx = s_vel.soup_vx[draw_k(c.key(), 0u) % 10];
+    c.ev_vy = s_vel.soup_vy[draw_k(c.key(), 1u) % 2];
     c.k += 2 * n;
 }
 
@@ -823,7 +829,7 @@ __device__ __forceinline__ void rule_a_fire(const TL &T, Ctx &c, uint32_t w0, in
     if (c.D() % 10 == 0) {
         float vx = (float)((int)(c.D() % 10) - 5) / 20.0f;
         float vy = -((float)(int)(c.D() % 10) / 10.0f) / 3.0f + -0.5f;
-        spawn_one(c, 3, x, y - 1, w0, sc, col, vx, vy);
+        spawn_one(c, 3, w0, sc, col, vx, vy);
         led_add(c, LED_CN, w0, 1);
     }
     if (c.D() % 150 == 0) {
@@ -956,7 +962,7 @@ __device__ __forceinline__ int class_a(const TL &T, const Ctx &c, int i) {
     return act ? 2 : 0;
 }
 
-// the rules: c.ev_n = the particles the cell emits (its event in *c.ev)
+// the rules: c.ev_n = the particles the cell emits
 template <class TL>
 __device__ __forceinline__ void rule_a_liquid(const TL &T, Ctx &c, uint32_t w0, int i, int x, int y) {
     if constexpr (TL::kF32)
@@ -989,9 +995,9 @@ __device__ __forceinline__ void rule_a(const TL &T, Ctx &c, uint32_t w0, int i, 
             }
             T.move(i, g, n, g + T.W, wb, dfb);
             if (falls) {
-                float vx = (float)((int)(c.D() % 10) - 5) / 20.0f;
-                float vy = (float)(-((int)(c.D() % 2) + 3)) / 10.0f + 1.5f;
-                spawn_one(c, 1, x, y + 1, w0, sc, col, vx, vy);
+                const float vx = s_vel.sand_vx[c.D() % 10];
+                const float vy = s_vel.sand_vy[c.D() % 2];
+                spawn_one(c, 1, w0, sc, col, vx, vy);
             } else {
                 const uint32_t t = c.D() % 2 == 0 ? w0 | CW_MOVED : w0;
                 T.set_word(n, t | CW_DIRTY | CW_VIS);
@@ -1203,65 +1209,43 @@ __device__ __forceinline__ void lattice(int sweep, int mode, int &px, int &py) {
     }
 }
 
-// write the particles of one spawn event (world.cpp:1110-1119,1222,1298)
+// write the particles of the active cell's spawn event (world.cpp:1110-1119,1222,1298), three
+// 16-byte stores each
+static_assert(sizeof(SpawnRec) == 48, "three 16-byte stores");
 template <bool TEMP, bool F32>
-static __device__ __noinline__ void emit_spawns(const WorldDev &w, const SpawnEv &ev, int n, uint32_t cp,
-                                                uint32_t rank0, int base) {
-    int32_t base_amt = 0, extra = 0;
-    if (ev.kind == 2) {
+__device__ __forceinline__ void emit_spawns(const WorldDev &w, Ctx &c, uint32_t cp, uint32_t rank0, int base) {
+    const int n = c.ev_n;
+    int32_t amount = c.ev_sc, extra = 0;
+    if (c.ev_kind == 2 && n > 1) {
         if (F32) {
             // f32 amt = tile.fluidAmount / n for every particle (world.cpp:1292)
-            base_amt = __float_as_int(__fdiv_rn(__int_as_float(ev.sc), (float)n));
+            amount = __float_as_int(__fdiv_rn(__int_as_float(c.ev_sc), (float)n));
         } else {
-            base_amt = ev.sc / n;
-            extra = ev.sc % n;
+            amount = c.ev_sc / n;
+            extra = c.ev_sc % n;
         }
     }
+    const uint32_t bits = c.ev_kind == 3 ? 2u << 24 : 0u;
+    const uint32_t life = c.ev_kind == 3 ? 30u | 10u << 16 : 60u << 16;  // lifetime, fade
+    const uint32_t temp = (TEMP && c.ev_kind == 2) ? (uint32_t)(uint16_t)c.ev_tp : 0u;
+    const float x = (float)c.kx, y = (float)(c.ev_kind == 3 ? c.ky - 1 : c.ky + 1);
+    float vx = c.ev_vx, vy = c.ev_vy;
+#pragma unroll 1
     for (int i = 0; i < n; i++) {
-        int slot = base + i;
+        const int slot = base + i;
         if (slot >= w.stage_cap) {
             atomicOr(w.err, ERR_SPAWN_CAP);
             return;
         }
-        SpawnRec r;
-        r.cp = cp;
-        r.rank = rank0 + (uint32_t)i;
-        r.x = (float)ev.x;
-        r.y = (float)ev.y;
-        r.id = ev.id;
-        r.colour = ev.col;
-        r.temp = (TEMP && ev.kind == 2) ? ev.tp : (int16_t)0;
-        r.pad = 0;
-        if (ev.kind == 1) {
-            r.vx = ev.vx;
-            r.vy = ev.vy;
-            r.ay = 0.1f;
-            r.scalar = ev.sc;
-            r.flags = ev.fl;
-            r.bits = 0;
-            r.lifetime = 0;
-            r.fade = 60;
-        } else if (ev.kind == 3) {
-            r.vx = ev.vx;
-            r.vy = ev.vy;
-            r.ay = 0.01f;
-            r.scalar = ev.sc;
-            r.flags = ev.fl;
-            r.bits = 2;
-            r.lifetime = 30;
-            r.fade = 10;
-        } else {
-            uint32_t d0 = draw_k(ev.ck, ev.k0 + 2u * (uint32_t)i), d1 = draw_k(ev.ck, ev.k0 + 2u * (uint32_t)i + 1u);
-            r.vx = (float)((int)(d0 % 10) - 5) / 30.0f;
-            r.vy = (float)(-((int)(d1 % 2) + 3)) / 10.0f + 1.0f;
-            r.ay = 0.1f;
-            r.scalar = base_amt + (i < extra ? 1 : 0);
-            r.flags = 0;
-            r.bits = 0;
-            r.lifetime = 0;
-            r.fade = 60;
+        if (i > 0) {
+            vx = s_vel.soup_vx[draw_k(c.key(), 2u * (uint32_t)i) % 10];
+            vy = s_vel.soup_vy[draw_k(c.key(), 2u * (uint32_t)i + 1u) % 2];
         }
-        w.stage[slot] = r;
+        uint4 *r = reinterpret_cast<uint4 *>(&w.stage[slot]);
+        r[0] = make_uint4(cp, rank0 + (uint32_t)i, __float_as_uint(x), __float_as_uint(y));
+        r[1] = make_uint4(__float_as_uint(vx), __float_as_uint(vy), __float_as_uint(c.ev_kind == 3 ? 0.01f : 0.1f),
+                          c.ev_col);
+        r[2] = make_uint4((uint32_t)(amount + (i < extra ? 1 : 0)), c.ev_idfl | bits, life, temp);
     }
 }
 
@@ -1285,6 +1269,7 @@ struct SmemHeadT {
     // the last sub-phase in which a cell spawned more than one particle
     uint32_t spawn_bits[3][NT / 32];
     int many;
+    int running[2];  // spawns of the chunk-pass so far, in turn
     uint32_t n_list[3];  // lengths of the lists of this sub-phase and of the next two, in turn
     // CTA pair: what the partner wrote here: [0..1] its chunk flags, [2..3] its spawn
     // count of a sweep-A sub-phase (alternate slots)
@@ -1359,8 +1344,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
     int seq = 0;  // sub-phases of sweep A so far
     int nsub = 0;  // the list count of the next sub-phase of sweeps A and B
     Ctx c;
-    SpawnEv ev_store;  // outside the context (see Ctx::ev)
-    c.ev = &ev_store;
+    spawn_vel_init(tid);
     c.iter = iter_arg;
     c.mt = mt;
     c.led_s = S.led;
@@ -1533,6 +1517,8 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
             Tl.pd = (rank ? half : -half) * Tl.RW;
         }
 
+        if (tid == 0) S.running[0] = 0;
+
         // ---- stage the tile, one warp per row. The 4-byte planes go straight to
         // shared memory, as two tensor copies (TMA) or with cp.async; ids and flags
         // are loaded a row at a time, all loads of a row in flight together. The
@@ -1702,7 +1688,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
 
         const int mode = c.has_inter ? 2 : (fire ? 1 : 0);
         const int cw = min(C, W - cx), chh = min(C, H - cy);
-        int running = 0;  // spawns emitted so far by this chunk-pass
+        int rb = 0;       // which of S.running holds the spawns of the chunk-pass so far
         int nsub_a = 0;   // CTA pair: the exchange slot of the sweep-A sub-phase
         c.led_g = w.ledger;
         // The reference's order as a wavefront: thread k updates chunk row k counted
@@ -1734,10 +1720,10 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                             else if (cls == 2)
                                 rule_a(Tl, c, Tl.at(i), i, x, y);
                             if (c.ev_n > 0) {
-                                if (!F32 && c.ev->kind == 2) led_add64(c, LED_DF, S.mw[c.ev->id], c.ev_df);
+                                if (!F32 && c.ev_kind == 2) led_add64(c, LED_DF, S.mw[c.ev_idfl & CW_ID], c.ev_df);
                                 const int base = atomicAdd(w.stage_count, c.ev_n);
-                                emit_spawns<TEMP, F32>(w, *c.ev, c.ev_n, cp * (uint32_t)w.cp_rows + (uint32_t)k,
-                                                       (uint32_t)spawned, base);
+                                emit_spawns<TEMP, F32>(w, c, cp * (uint32_t)w.cp_rows + (uint32_t)k, (uint32_t)spawned,
+                                                       base);
                                 spawned += c.ev_n;
                             }
                         } else if (sweep == 1) {
@@ -1864,22 +1850,23 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                         // spawned particles are ranked in enumeration order: from the bits of the
                         // spawning cells, a word per lane of every warp, without another barrier
                         const bool any = __syncthreads_or(c.ev_n > 0);
-                        int tot = 0, before = running, rank_e = 0;
-                        bool slow = false;
+                        // (only the warps that need them, and the first, which keeps the count)
+                        int tot = 0, rank_e = 0, before = S.running[rb];
                         if (any) {
-                            slow = S.many == seq;
-                            if (!slow) {
-                                const uint32_t word = lane < T / 32 ? S.spawn_bits[sub][lane] : 0u;
-                                int inc = __popc(word);
+                            if (S.many != seq) {
+                                if (sp || wid == 0) {
+                                    const uint32_t word = lane < T / 32 ? S.spawn_bits[sub][lane] : 0u;
+                                    int inc = __popc(word);
 #pragma unroll
-                                for (int o = 1; o < 32; o <<= 1) {
-                                    const int t = __shfl_up_sync(0xffffffffu, inc, o);
-                                    if (lane >= o) inc += t;
+                                    for (int o = 1; o < 32; o <<= 1) {
+                                        const int t = __shfl_up_sync(0xffffffffu, inc, o);
+                                        if (lane >= o) inc += t;
+                                    }
+                                    tot = __shfl_sync(0xffffffffu, inc, 31);
+                                    const uint32_t we = __shfl_sync(0xffffffffu, word, e >> 5);
+                                    rank_e = __shfl_sync(0xffffffffu, inc - __popc(word), e >> 5) +
+                                             __popc(we & ((1u << (e & 31)) - 1u));
                                 }
-                                tot = __shfl_sync(0xffffffffu, inc, 31);
-                                const uint32_t we = __shfl_sync(0xffffffffu, word, e >> 5);
-                                rank_e = __shfl_sync(0xffffffffu, inc - __popc(word), e >> 5) +
-                                         __popc(we & ((1u << (e & 31)) - 1u));
                             } else {
                                 // some cell spawns several: a scan over their counts
                                 S.cnt[tid] = 0;
@@ -1915,18 +1902,24 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                                                (uint32_t)tot);
                             cluster_sync();
                             const int tot_p = (int)S.xch[slot_t];
+                            if (any || tot_p) {
+                                if (tid == 0) S.running[rb ^ 1] = before + tot + tot_p;
+                                rb ^= 1;
+                            }
                             if (rank) before += tot_p;
-                            running += tot_p;
+                        } else if (any) {
+                            // read after the next barrier at the earliest
+                            if (tid == 0) S.running[rb ^ 1] = before + tot;
+                            rb ^= 1;
                         }
                         // the (chunk-pass, rank) key orders the particles later
                         if (sp) {
                             slot = __shfl_sync(0xffffffffu, slot, 31) + spi - c.ev_n;
                             if (c.ev_n > 0) {
-                                emit_spawns<TEMP, F32>(w, *c.ev, c.ev_n, cp, (uint32_t)(before + rank_e), slot);
-                                if (!F32 && c.ev->kind == 2) led_add64(c, LED_DF, S.mw[c.ev->id], c.ev_df);
+                                emit_spawns<TEMP, F32>(w, c, cp, (uint32_t)(before + rank_e), slot);
+                                if (!F32 && c.ev_kind == 2) led_add64(c, LED_DF, S.mw[c.ev_idfl & CW_ID], c.ev_df);
                             }
                         }
-                        running += tot;
                         FSE_PT(4)
                     } else if (sweep == 1) {
                         // at most 43 x 43 < 2 T cells: two per thread. Liquids take their
@@ -2061,7 +2054,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                 }
             }
         }
-        if (!SEQ && tid == 0 && rank == 0) w.cp_count[cp] = running;
+        if (!SEQ && tid == 0 && rank == 0) w.cp_count[cp] = S.running[rb];
         // the chunk-pass's ledger counts (the sweeps ended with a barrier)
         for (int i = tid; i < LED_TICK * 64; i += T) {
             const int32_t v = S.led[i];
