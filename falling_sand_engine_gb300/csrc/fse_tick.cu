@@ -345,6 +345,11 @@ struct Tile : TileData {
         const uint32_t n = on ? w | CW_MOVED : w & ~CW_MOVED;
         if (n != w) set_word(i, n | CW_DIRTY);
     }
+    // clear the moved flag of cell i if it is a liquid that has settled
+    __device__ __forceinline__ void wake_soup(int i, uint32_t w) const {
+        if ((w & (CW_TYPE | CW_MOVED)) == ((uint32_t)T_SOUP << MW_TYPE_SHIFT | CW_MOVED))
+            set_word(i, (w & ~CW_MOVED) | CW_DIRTY);
+    }
     __device__ __forceinline__ void set_moved(int i, bool on) const { set_moved_w(i, s_w[i], on); }
     // f32 worlds: fluidAmountDiff += v as the reference's float add. No other cell of
     // the sub-phase (or wavefront step) touches this diff, and the ones that touched
@@ -623,7 +628,11 @@ __device__ __forceinline__ uint32_t settle_word(uint32_t w0) {
 // when its turn begins (it already holds the flows of the cells updated before it) and
 // written back with its own flows subtracted in order, as the reference's copy of the
 // tile does.
-template <class TL>
+//
+// MIXED: the cell above or below may be another liquid, to trade places with or to react
+// with (few are: class_a lists those with the other cells; the way through the trades,
+// though no lane took it, made the rule of a single liquid a third slower).
+template <bool MIXED, class TL>
 __device__ __forceinline__ void rule_a_soup(const TL &T, Ctx &c, uint32_t w0, int i, int x, int y) {
     const int32_t sc = T.s_sc[i];
     if (sc == 0) return;
@@ -646,7 +655,7 @@ __device__ __forceinline__ void rule_a_soup(const TL &T, Ctx &c, uint32_t w0, in
         const int32_t dst = airBelow ? 0 : sb;
         down = clampflow(vflow(sc, dst) - dst, sc);
         rem -= down;
-    } else if (c.iter == 0 && cw_is(wb, T_SOUP)) {
+    } else if (MIXED && c.iter == 0 && cw_is(wb, T_SOUP)) {
         if (c.D() % 10 == 0) {
             swap_liquid(T, w0, sc, col, T.df_load(g), i, g, i + RW, g + T.W);
             return;
@@ -674,7 +683,7 @@ __device__ __forceinline__ void rule_a_soup(const TL &T, Ctx &c, uint32_t w0, in
             up = clampflow(rem - vflow(rem, dst), rem);
             rem -= up;
             gone = rem < Q_MINV;
-        } else if (c.iter == 0 && cw_is(wt, T_SOUP)) {
+        } else if (MIXED && c.iter == 0 && cw_is(wt, T_SOUP)) {
             swap_up = c.D() % 10 == 0;
         }
     }
@@ -715,18 +724,18 @@ __device__ __forceinline__ void rule_a_soup(const TL &T, Ctx &c, uint32_t w0, in
     if (dd == 0) {
         wn = settle_word(w0);
     } else {
-        if (cw_is(wt, T_SOUP)) T.set_moved_w(i - RW, wt, false);
-        if (cw_is(wb, T_SOUP)) T.set_moved_w(i + RW, wb, false);
-        if (cw_is(wl, T_SOUP)) T.set_moved_w(i - 1, wl, false);
-        if (cw_is(wr, T_SOUP)) T.set_moved_w(i + 1, wr, false);
+        T.wake_soup(i - RW, wt);
+        T.wake_soup(i + RW, wb);
+        T.wake_soup(i - 1, wl);
+        T.wake_soup(i + 1, wr);
         atomicAdd(pd, dd);
     }
     T.set_word(i, wn | CW_DIRTY);
-    if (cw_id(w0) == c.id_water && cw_id(wb) == c.id_lava)
+    if (MIXED && cw_id(w0) == c.id_water && cw_id(wb) == c.id_lava)
         water_on_lava(T, c, wn, (long long)sc + T.df_load(g), i, g);
 }
 
-template <class TL>
+template <bool MIXED, class TL>
 __device__ __forceinline__ void rule_a_soup_f32(const TL &T, Ctx &c, uint32_t w0, int i, int x, int y) {
     const int32_t sc = T.s_sc[i];
     const float amount = __int_as_float(sc);
@@ -767,7 +776,7 @@ __device__ __forceinline__ void rule_a_soup_f32(const TL &T, Ctx &c, uint32_t w0
     if ((airBelow && c.iter <= 2) || cw_same(wb, w0)) {
         const float dst = airBelow ? 0.0f : sb;
         flow_to(clampflow_f(__fsub_rn(vflow_f(start, dst), dst), start), i + RW, wb, g + T.W, 1, true);
-    } else if (c.iter == 0 && cw_is(wb, T_SOUP)) {
+    } else if (MIXED && c.iter == 0 && cw_is(wb, T_SOUP)) {
         if (c.D() % 10 == 0) {  // the cell leaves its position with its diff
             swap_liquid(T, w0, sc, col, __float_as_int(dfv), i, g, i + RW, g + T.W);
             return;
@@ -792,7 +801,7 @@ __device__ __forceinline__ void rule_a_soup_f32(const TL &T, Ctx &c, uint32_t w0
             const float dst = cw_air(wt) ? 0.0f : su;
             flow_to(clampflow_f(__fsub_rn(rem, vflow_f(rem, dst)), rem), i - RW, wt, g - T.W, 1, false);
             done = rem < F_MINV;
-        } else if (c.iter == 0 && cw_is(wt, T_SOUP)) {
+        } else if (MIXED && c.iter == 0 && cw_is(wt, T_SOUP)) {
             swap_up = c.D() % 10 == 0;
         }
     }
@@ -807,14 +816,14 @@ __device__ __forceinline__ void rule_a_soup_f32(const TL &T, Ctx &c, uint32_t w0
     } else if (start == rem) {
         wn = settle_word(w0);
     } else {
-        if (cw_is(wt, T_SOUP)) T.set_moved_w(i - RW, wt, false);
-        if (cw_is(wb, T_SOUP)) T.set_moved_w(i + RW, wb, false);
-        if (cw_is(wl, T_SOUP)) T.set_moved_w(i - 1, wl, false);
-        if (cw_is(wr, T_SOUP)) T.set_moved_w(i + 1, wr, false);
+        T.wake_soup(i - RW, wt);
+        T.wake_soup(i + RW, wb);
+        T.wake_soup(i - 1, wl);
+        T.wake_soup(i + 1, wr);
     }
     T.set_word(i, wn | CW_DIRTY);
     T.df[g] = __float_as_int(dfv);
-    if (!done && cw_id(w0) == c.id_water && cw_id(wb) == c.id_lava) water_on_lava(T, c, wn, 0, i, g);
+    if (MIXED && !done && cw_id(w0) == c.id_water && cw_id(wb) == c.id_lava) water_on_lava(T, c, wn, 0, i, g);
 }
 
 // fire, world.cpp:1101-1146. Returns false where the cell burnt out (the sweep goes on
@@ -924,9 +933,21 @@ __device__ __forceinline__ bool rule_a_react(const TL &T, Ctx &c, uint32_t w0, i
 }
 
 // ----------------------------------------------------------------- sweep A
+// a liquid of amount sc with four AIR cells below (world.cpp:1283-1284)
+template <class TL>
+__device__ __forceinline__ bool soup_falls(const TL &T, int i, int32_t sc) {
+    bool enough;
+    if constexpr (TL::kF32)
+        enough = (double)__int_as_float(sc) > 0.005;  // in double: 0.005 is a double literal
+    else
+        enough = sc > Q_FREEFALL;
+    return enough && cw_air(T.at(i + T.RW) | T.at(i + 2 * T.RW) | T.at(i + 3 * T.RW) | T.at(i + 4 * T.RW));
+}
+
 // Whether sweep A may change cell i (a superset of the cells that its rule changes):
-// 0 no, 1 a liquid, 2 another cell or a liquid in free fall (world.cpp:1283-1305), so that
-// the warps of liquids that flow do not take the long way through an emission. Cells whose material is not updated in this
+// 0 no, 1 a liquid, 2 another cell, a liquid in free fall (world.cpp:1283-1305) or one with
+// another liquid above or below, so that the warps of liquids that flow do not take the
+// long ways through an emission or a trade of places. Cells whose material is not updated in this
 // iteration are marked visited here (world.cpp:1093-1096).
 template <class TL>
 __device__ __forceinline__ int class_a(const TL &T, const Ctx &c, int i) {
@@ -939,22 +960,22 @@ __device__ __forceinline__ int class_a(const TL &T, const Ctx &c, int i) {
     const uint32_t wn = T.at(cw_is(w0, T_GAS) ? i - T.RW : i + T.RW);
     if (cw_is(w0, T_SOUP)) {
         const int32_t sc = T.s_sc[i];
-        bool none, small, fall;
+        bool none, small;
         if constexpr (TL::kF32) {
             const float amount = __int_as_float(sc);
             none = amount == 0.0f;
             small = amount < F_MINV;
-            // tile.fluidAmount > 0.005 compares in double (0.005 is a double literal)
-            fall = cw_air(wn) && (double)amount > 0.005;
         } else {
             none = sc == 0;
             small = sc < Q_MINV;
-            fall = cw_air(wn) && sc > Q_FREEFALL;
         }
         if (none) return 0;
-        if (fall) fall = cw_air(T.at(i + 2 * T.RW) | T.at(i + 3 * T.RW) | T.at(i + 4 * T.RW));
-        // a settled liquid only falls or dries up
-        return small ? 1 : (fall ? 2 : (w0 & CW_MOVED ? 0 : 1));
+        if (small) return 1;
+        if (cw_air(wn) && soup_falls(T, i, sc)) return 2;
+        if (w0 & CW_MOVED) return 0;  // a settled liquid only falls or dries up
+        const uint32_t wt = T.at(i - T.RW);
+        const bool mixed = (cw_is(wn, T_SOUP) && !cw_same(wn, w0)) || (cw_is(wt, T_SOUP) && !cw_same(wt, w0));
+        return mixed ? 2 : 1;
     }
     bool act = (w0 & CW_FIRE) != 0;
     if (cw_is(w0, T_SAND)) act = c.has_inter || (w0 & CW_REACT) || wn < cw_sink(w0);
@@ -963,12 +984,12 @@ __device__ __forceinline__ int class_a(const TL &T, const Ctx &c, int i) {
 }
 
 // the rules: c.ev_n = the particles the cell emits
-template <class TL>
+template <bool MIXED, class TL>
 __device__ __forceinline__ void rule_a_liquid(const TL &T, Ctx &c, uint32_t w0, int i, int x, int y) {
     if constexpr (TL::kF32)
-        rule_a_soup_f32(T, c, w0, i, x, y);
+        rule_a_soup_f32<MIXED>(T, c, w0, i, x, y);
     else
-        rule_a_soup(T, c, w0, i, x, y);
+        rule_a_soup<MIXED>(T, c, w0, i, x, y);
 }
 // a cell of class 2, of word w0
 template <class TL>
@@ -1012,9 +1033,13 @@ __device__ __forceinline__ void rule_a(const TL &T, Ctx &c, uint32_t w0, int i, 
                 }
             }
         }
-    } else if (cw_is(w0, T_SOUP)) {  // in free fall
-        const int g = T.gi(x, y);
+    } else if (cw_is(w0, T_SOUP)) {
         const int32_t sc = T.s_sc[i];
+        if (!soup_falls(T, i, sc)) {  // another liquid above or below
+            rule_a_liquid<true>(T, c, w0, i, x, y);
+            return;
+        }
+        const int g = T.gi(x, y);
         if constexpr (TL::kF32) {
             free_fall(T, c, w0, sc, T.s_col[i], (int)__fdiv_rn(__int_as_float(sc), 4.0f), i, g, x, y);  // int n = tile.fluidAmount / 4
         } else {
@@ -1716,7 +1741,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                             c.at(x, y);
                             const int cls = class_a(Tl, c, i);
                             if (cls == 1)
-                                rule_a_liquid(Tl, c, Tl.at(i), i, x, y);
+                                rule_a_liquid<false>(Tl, c, Tl.at(i), i, x, y);
                             else if (cls == 2)
                                 rule_a(Tl, c, Tl.at(i), i, x, y);
                             if (c.ev_n > 0) {
@@ -1818,7 +1843,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                             const uint32_t w0 = Tl.at(i);
                             c.at(x, y);
                             if (liquid)
-                                rule_a_liquid(Tl, c, w0, i, x, y);
+                                rule_a_liquid<false>(Tl, c, w0, i, x, y);
                             else
                                 rule_a(Tl, c, w0, i, x, y);
                             if (c.ev_n > 0) {
