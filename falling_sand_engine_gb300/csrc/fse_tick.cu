@@ -374,6 +374,7 @@ struct Ctx {
     long long *led_g;      // global ledger [LED_ROWS][MAXMAT]
     const uint32_t *mw;    // material words (shared)
     const uint16_t *fr;    // slipperiness | stability << 8 (shared)
+    const uint2 *fric;     // by drop over stability (at most 11): 1000 / d, 2^32 / that (shared)
     // the cell's spawn event: its particles' kind (1 sand, 2 soup, 3 fire), id and flags as
     // in their records, colour, scalar, temperature, and the velocity of the first
     int ev_kind;
@@ -951,15 +952,15 @@ __device__ __forceinline__ bool soup_falls(const TL &T, int i, int32_t sc) {
 // iteration are marked visited here (world.cpp:1093-1096).
 template <class TL>
 __device__ __forceinline__ int class_a(const TL &T, const Ctx &c, int i) {
-    const uint32_t w0 = T.at(i);
+    // what any class asks, in one round of loads
+    const uint32_t w0 = T.at(i), wn = T.at(i + T.RW), wt = T.at(i - T.RW);
+    const int32_t sc = T.s_sc[i];
     if (w0 & CW_VIS) return 0;
     if (!(w0 & CW_LIVE)) {
         T.set_word(i, w0 | CW_VIS);
         return 0;
     }
-    const uint32_t wn = T.at(cw_is(w0, T_GAS) ? i - T.RW : i + T.RW);
     if (cw_is(w0, T_SOUP)) {
-        const int32_t sc = T.s_sc[i];
         bool none, small;
         if constexpr (TL::kF32) {
             const float amount = __int_as_float(sc);
@@ -973,13 +974,12 @@ __device__ __forceinline__ int class_a(const TL &T, const Ctx &c, int i) {
         if (small) return 1;
         if (cw_air(wn) && soup_falls(T, i, sc)) return 2;
         if (w0 & CW_MOVED) return 0;  // a settled liquid only falls or dries up
-        const uint32_t wt = T.at(i - T.RW);
         const bool mixed = (cw_is(wn, T_SOUP) && !cw_same(wn, w0)) || (cw_is(wt, T_SOUP) && !cw_same(wt, w0));
         return mixed ? 2 : 1;
     }
     bool act = (w0 & CW_FIRE) != 0;
     if (cw_is(w0, T_SAND)) act = c.has_inter || (w0 & CW_REACT) || wn < cw_sink(w0);
-    if (cw_is(w0, T_GAS)) act = cw_air(wn);
+    if (cw_is(w0, T_GAS)) act = cw_air(wt);
     return act ? 2 : 0;
 }
 
@@ -1002,6 +1002,7 @@ __device__ __forceinline__ void rule_a(const TL &T, Ctx &c, uint32_t w0, int i, 
         if ((w0 & CW_REACT) && rule_a_react(T, c, w0, i, x, y)) return;
         // world.cpp:1206-1267
         if (!(wb < lim)) return;
+        c.key();  // it will draw: the hashes run while the loads are under way
         const int g = T.gi(x, y);
         const int32_t dfb = T.df_if_soup(wb, g + T.W);
         const bool canL = T.at(i + T.RW - 1) < lim, canR = T.at(i + T.RW + 1) < lim;
@@ -1115,15 +1116,19 @@ __device__ __forceinline__ void rule_b(const TL &T, Ctx &c, uint32_t w0, int i, 
         const int32_t dfl = canL ? T.df_if_soup(wl, g + T.W - 1) : 0, dfr = canR ? T.df_if_soup(wr, g + T.W + 1) : 0;
         bool stopped = !(w0 & CW_MOVED);
         c.at(x, y);
+        c.key();  // it will draw: the hashes run while the loads are under way
         const int a = c.fr[cw_id(w0)];
         if (stopped) {
             // world.cpp:1619-1627 over the AIR snapshot taken when sweep B began
             const int drop = __popc(T.air10(i + RW - 1, x - 1, y + 1) | T.air10(i + RW + 1, x + 1, y + 1));
             int d = drop + 1 - (a >> 8);
             if (d > 0) {
-                int chance = 1000 / d;
-                if (chance < 1000) {
-                    if (c.D() % (uint32_t)chance == 0) {
+                // chance = 1000 / d, 2 <= d <= 11 (1000 or more never): draw % chance == 0,
+                // with the quotient by multiplication, which is at most one short
+                if (d >= 2) {
+                    const uint2 f = c.fric[d];
+                    const uint32_t draw = c.D(), rest = draw - __umulhi(draw, f.y) * f.x;
+                    if (rest == 0 || rest == f.x) {
                         stopped = false;
                         T.set_moved_w(i, w0, true);
                     }
@@ -1280,8 +1285,12 @@ template <int NT>
 struct SmemHeadT {
     uint32_t mw[MAXMAT];  // material -> cell word of this iteration
     uint16_t fr[MAXMAT];  // slipperiness | stability << 8
+    uint2 fric[12];       // d: 1000 / d and 2^32 / that
     int32_t led[LED_TICK * 64];   // the chunk-pass's ledger counts (led_slot)
-    int scan[32];
+    union {
+        uint32_t vote[32];  // each warp's activity (bit 0) and fire (bit 1) votes of the chunk-pass
+        int scan[32];       // in its sweeps: the warps' spawn totals of a sub-phase
+    };
     // the pillar snapshot of sweep B (chunk edge <= 128)
     uint32_t air[(128 + 2) * 5];
     // the cells of a sub-phase that a rule may change (dx | dy << 8); after a sweep-A
@@ -1299,7 +1308,6 @@ struct SmemHeadT {
     // CTA pair: what the partner wrote here: [0..1] its chunk flags, [2..3] its spawn
     // count of a sweep-A sub-phase (alternate slots)
     uint32_t xch[4];
-    uint32_t vote[32];  // each warp's activity (bit 0) and fire (bit 1) votes of the chunk-pass
 };
 
 // Dynamic shared memory of a CTA that updates `own` rows of a chunk of edge C: the
@@ -1359,6 +1367,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
     const int rank = PAIR ? (int)cluster_rank() : 0;
     int npass = 0;  // chunks taken so far (the same count in both CTAs of a pair)
     int mw_iter = -1;  // the iteration S.mw was built for
+    if (tid >= 1 && tid < 12) S.fric[tid] = make_uint2(1000u / tid, 0xFFFFFFFFu / (1000u / tid));
     for (int i = tid; i < MAXMAT; i += T)
         S.fr[i] = (uint16_t)(i < mt->n ? mt_slip(mt->a[i]) | (mt_stab(mt->a[i]) << 8) : 0);
     for (int i = tid; i < LED_TICK * 64; i += T) S.led[i] = 0;
@@ -1375,6 +1384,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
     c.led_s = S.led;
     c.mw = S.mw;
     c.fr = S.fr;
+    c.fric = S.fric;
     c.id_fire = mt->id_fire;
     c.id_water = mt->id_water;
     c.id_lava = mt->id_lava;
