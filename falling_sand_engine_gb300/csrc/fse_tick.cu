@@ -1189,10 +1189,9 @@ __device__ __forceinline__ void rule_b(const TL &T, Ctx &c, uint32_t w0, int i, 
 }
 
 // ----------------------------------------------------------------- sweep C
+// w0: the word of a GAS cell not yet visited
 template <class TL>
-__device__ __forceinline__ void rule_c(const TL &T, Ctx &c, int i, int x, int y) {
-    const uint32_t w0 = T.at(i);
-    if ((w0 & CW_VIS) || !cw_is(w0, T_GAS)) return;  // world.cpp:1831
+__device__ __forceinline__ void rule_c(const TL &T, Ctx &c, uint32_t w0, int i, int x, int y) {
     // world.cpp:1862-1889
     const bool l = T.air(i - 1), r = T.air(i + 1), steam = cw_id(w0) == c.id_steam;
     if (!l && !r && !steam) return;
@@ -1770,7 +1769,8 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                                 rule_b(Tl, c, w0, i, x, y);
                             }
                         } else {
-                            rule_c(Tl, c, i, x, y);
+                            const uint32_t w0 = Tl.at(i);
+                            if (!(w0 & CW_VIS) && cw_is(w0, T_GAS)) rule_c(Tl, c, w0, i, x, y);  // world.cpp:1831
                         }
                     }
                     __syncthreads();
@@ -2007,18 +2007,29 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                     } else {
                         // every row of the chunk, its columns 3 apart: each thread takes all of
                         // its cells in turn
+                        // (three words loaded at a time: most cells are no gas)
                         int qe = q, re = r;
 #pragma unroll 1
-                        for (;;) {
-                            const int ex = rx + re * px, ey = dyb + qe * py;
-                            if (ey >= yend) break;
-                            if (ex < cw) rule_c(Tl, c, Tl.li(cx + ex, cy + ey), cx + ex, cy + ey);
-                            qe += dq;
-                            re += dr;
-                            if (re >= nxm) {
-                                re -= nxm;
-                                qe++;
+                        while (dyb + qe * py < yend) {
+                            int i3[3], x3[3], y3[3];
+                            uint32_t w3[3];
+#pragma unroll
+                            for (int k = 0; k < 3; k++) {
+                                const int ex = rx + re * px, ey = dyb + qe * py;
+                                x3[k] = cx + ex;
+                                y3[k] = cy + ey;
+                                i3[k] = Tl.li(x3[k], y3[k]);
+                                w3[k] = ex < cw && ey < yend ? Tl.at(i3[k]) : CW_VIS;
+                                qe += dq;
+                                re += dr;
+                                if (re >= nxm) {
+                                    re -= nxm;
+                                    qe++;
+                                }
                             }
+#pragma unroll
+                            for (int k = 0; k < 3; k++)
+                                if (!(w3[k] & CW_VIS) && cw_is(w3[k], T_GAS)) rule_c(Tl, c, w3[k], i3[k], x3[k], y3[k]);
                         }
                         FSE_PT(7)
                         if constexpr (PAIR)
