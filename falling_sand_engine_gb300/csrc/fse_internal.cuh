@@ -183,8 +183,8 @@ struct WorldDev {
     int32_t part_cap;
     uint8_t *p_state;       // per particle: 0 alive, 1 dead; during the update its outcome
     // per particle during the update: the cells it read as a box (x0 | y0 << 16 and
-    // x1 | y1 << 16; box0 -1: none), the cell it fills or merges into (-1: none), the
-    // fill cell an iteration moved it away from; box0 holds the merge cell afterwards
+    // x1 | y1 << 16; box0 -1: none), the cell it fills or merges into (-1: none); box0
+    // holds the merge cell afterwards. p_prev: the cells an iteration's fills moved away from
     int32_t *p_box0, *p_box1, *p_cell, *p_prev;
     int32_t *req_count;     // [3] counters of the update (fill changes of even / odd iterations)
     uint32_t *chg;          // 2 x airmap blocks: lowest index whose fill changed there (read / written by an iteration)

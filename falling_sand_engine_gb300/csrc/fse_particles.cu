@@ -225,19 +225,21 @@ struct Box {
 // of the cells it read into p_box0 / p_box1. A particle that must search the spiral
 // (world.cpp:2093-2147) returns true with its kind and cell not yet written; the
 // caller's warp walks the spiral with it (warp_spiral) and finishes it.
-__device__ bool part_flight(const WorldDev &w, const uint8_t *s_type, int i) {
+// kind and cell are returned as well: stored and loaded again they would cost a round trip.
+__device__ bool part_flight(const WorldDev &w, const uint8_t *s_type, int i, uint8_t &kind, int &cell) {
+    // all of the particle's state in one round trip
     uint8_t bits = w.p.bits[i];
     int32_t life = w.p.life[i];
     float x = w.p.x[i], y = w.p.y[i], vx = w.p.vx[i], vy = w.p.vy[i];
+    const float ax = w.p.ax[i], ay = w.p.ay[i], tf = w.p.tf[i];
     const int W = w.W, H = w.H;
-    uint8_t kind = PS_ALIVE;
-    int cell = -1;
+    kind = PS_ALIVE;
+    cell = -1;
     bool spiral = false;
     Box bx = {W, H, -1, -1};
     if ((bits & 2) && life <= 0) {  // :2033-2037
         kind = PS_DESTROY;
     } else {
-        const float tf = w.p.tf[i];
         if (tf != 0.f) {  // :2039-2051
             const float tdx = __fsub_rn(w.p.tx[i], x), tdy = __fsub_rn(w.p.ty[i], y);
             const float nf = __fsqrt_rn(__fadd_rn(__fmul_rn(tdx, tdx), __fmul_rn(tdy, tdy)));
@@ -256,8 +258,8 @@ __device__ bool part_flight(const WorldDev &w, const uint8_t *s_type, int i) {
             // having read no cell
         } else {
             bx.add(lx, ly);
-            vx = __fadd_rn(vx, w.p.ax[i]);  // :2063-2064
-            vy = __fadd_rn(vy, w.p.ay[i]);
+            vx = __fadd_rn(vx, ax);  // :2063-2064
+            vy = __fadd_rn(vy, ay);
             const int div = (int)__fadd_rn(__fadd_rn(fabsf(vx), fabsf(vy)), 1.0f);
             const float dvx = __fdiv_rn(vx, (float)div), dvy = __fdiv_rn(vy, (float)div);
             int hit = 0;  // 1: deposit at the previous cell, 2: spiral search
@@ -267,6 +269,9 @@ __device__ bool part_flight(const WorldDev &w, const uint8_t *s_type, int i) {
             constexpr int AHEAD = 4;
             uint16_t aid[AHEAD];
             int32_t adf[AHEAD];
+            // and the cell it starts from, where a hit deposits
+            const int id0 = w.id[ly * W + lx];
+            const int32_t df0 = __ldcg(&w.df[ly * W + lx]);
             for (int s = 0; s < div; s++) {  // :2071-2184
                 if (s % AHEAD == 0) {
                     float px = x, py = y;
@@ -311,7 +316,7 @@ __device__ bool part_flight(const WorldDev &w, const uint8_t *s_type, int i) {
                         if (bits & 2)
                             kind = PS_DESTROY;
                         else
-                            hit = (s_type[view_id(w, s_type, ly * W + lx, i)] != T_AIR) ? 2 : 1;
+                            hit = (s_type[view_of(w, s_type, id0, df0, i)] != T_AIR) ? 2 : 1;
                         break;
                     }
                 }
@@ -393,11 +398,6 @@ __device__ uint8_t warp_spiral(const WorldDev &w, const uint8_t *s_type, int i, 
     }
     *ring = max(abs((int)c_spiral[n - 1][0]), abs((int)c_spiral[n - 1][1]));
     return PS_FAIL;
-}
-
-// the fill a particle's outcome makes (-1: none)
-__device__ __forceinline__ int fill_of(const WorldDev &w, int i) {
-    return w.p_state[i] == PS_FILL ? w.p_cell[i] : -1;
 }
 
 // Grid-wide barrier of the cooperative update. The spin is bounded: if it ever
@@ -526,15 +526,17 @@ __device__ int active_worlds(int n_worlds, F count, int *s_ids, int *s_apref, in
 // what it read. Iteration work is restricted to the worlds that need it: a world
 // whose fills did not change in an iteration has converged (its particles read
 // only its own cells), so later iterations skip its particles, and the fills that
-// changed are listed per world (chg_n[parity] of them, their indices in the first
-// part_cap entries of merge_list, free until the commit) so that clearing their
-// records does not scan the particles. req_count[0..1] of world 0 count every
+// changed are listed per world (chg_n[parity] of them, the cells they moved away from in
+// p_prev) so that clearing their records does not scan the particles. An iteration of a
+// small population lasts as long as its chain of memory round trips, so what a phase reads
+// of a particle is loaded together and passed on in registers. req_count[0..1] of world 0 count every
 // world's fill changes of even and odd iterations; stats[0] of world 0 receives
 // the number of iterations. Dynamic shared memory: 3 * n_worlds + 2 ints.
 __global__ void __launch_bounds__(SERIAL_THREADS) k_part_serial(const WorldDev *__restrict__ worlds, int n_worlds,
                                                                  const MatTable *__restrict__ mt) {
     __shared__ uint8_t s_type[MAXMAT];
     __shared__ int s_warp[SERIAL_THREADS / 32];
+    __shared__ int s_first;  // one world: the first particle that an iteration looks at
     extern __shared__ int s_dyn[];
     int *s_pref = s_dyn;                       // [n_worlds + 1] particles before world k
     int *s_apref = s_dyn + n_worlds + 1;       // [n_worlds + 1] the active index space
@@ -581,30 +583,31 @@ __global__ void __launch_bounds__(SERIAL_THREADS) k_part_serial(const WorldDev *
                                         n_worlds,
                                         [&](int k) {
                                             const int32_t *cn = worlds[k].chg_n;
-                                            return __ldcg(&cn[1 - par]) > 0
-                                                       ? max(0, parts(k) - 1 - __ldcg(&cn[2 + par]))
-                                                       : 0;
+                                            const int n = __ldcg(&cn[1 - par]), lo = __ldcg(&cn[2 + par]);
+                                            if (n_worlds == 1 && threadIdx.x == 0) s_first = lo + 1;
+                                            return n > 0 ? max(0, parts(k) - 1 - lo) : 0;
                                         },
                                         s_ids, s_apref, s_warp);
         const int total_a = s_apref[n_act];
         for (int gb0 = gtid - lane; gb0 < total_a; gb0 += gstride) {
             const int g = gb0 + lane;
             bool work = g < total_a, spiral = false;
-            int wi = 0, i = 0, before = -1;
+            int wi = 0, i = 0, before = -1, cell = -1;
+            uint8_t kind = PS_ALIVE;
             if (work) {
                 const int j = entry_of(s_apref, n_act, g);
                 wi = s_ids[j];
                 i = g - s_apref[j];
                 const WorldDev &w = worlds[wi];
                 if (it > 0) {
-                    i += __ldcg(&w.chg_n[2 + par]) + 1;
-                    const int32_t b0 = w.p_box0[i];
+                    i += n_worlds == 1 ? s_first : __ldcg(&w.chg_n[2 + par]) + 1;
+                    const int32_t b0 = w.p_box0[i], b1 = w.p_box1[i], c0 = w.p_cell[i];
+                    const uint8_t k0 = w.p_state[i];
                     if (b0 < 0) {
                         work = false;  // read no cell: nothing can change it
                     } else {
                         const int nblk = w.amw * w.amh;
                         const uint32_t *seen = w.chg + (size_t)par * nblk;
-                        const int32_t b1 = w.p_box1[i];
                         const int x0 = (b0 & 0xFFFF) >> 3, y0 = ((uint32_t)b0 >> 16) >> 3;
                         const int x1 = (b1 & 0xFFFF) >> 3, y1 = ((uint32_t)b1 >> 16) >> 3;
                         // the lowest changing index over the box's blocks (the loads do not
@@ -615,10 +618,10 @@ __global__ void __launch_bounds__(SERIAL_THREADS) k_part_serial(const WorldDev *
                         if (lo >= (uint32_t)i)
                             work = false;
                         else
-                            before = fill_of(w, i);
+                            before = k0 == PS_FILL ? c0 : -1;
                     }
                 }
-                if (work) spiral = part_flight(w, s_type, i);
+                if (work) spiral = part_flight(w, s_type, i, kind, cell);
             }
             // the spirals of this warp's particles, one after another, 32 cells a step
             unsigned pend = __ballot_sync(0xffffffffu, spiral);
@@ -634,11 +637,13 @@ __global__ void __launch_bounds__(SERIAL_THREADS) k_part_serial(const WorldDev *
                 }
                 sx = __shfl_sync(0xffffffffu, sx, src);
                 sy = __shfl_sync(0xffffffffu, sy, src);
-                int cell, ring;
-                const uint8_t k = warp_spiral(sw, s_type, si, sx, sy, &cell, &ring);
+                int sc, ring;
+                const uint8_t k = warp_spiral(sw, s_type, si, sx, sy, &sc, &ring);
                 if (lane == src) {
+                    kind = k;
+                    cell = sc;
                     sw.p_state[si] = k;
-                    sw.p_cell[si] = cell;
+                    sw.p_cell[si] = sc;
                     if (k == PS_FAIL) {  // :2141-2144
                         sw.q.vy[si] = -4.0f;
                         sw.q.y[si] = __fsub_rn(sy, 16.0f);
@@ -659,17 +664,17 @@ __global__ void __launch_bounds__(SERIAL_THREADS) k_part_serial(const WorldDev *
             }
             if (work) {
                 const WorldDev &w = worlds[wi];
-                const int after = fill_of(w, i);
+                const int after = kind == PS_FILL ? cell : -1;
                 if (after != before) {
                     const int nblk = w.amw * w.amh;
                     uint32_t *mark = w.chg + (size_t)(1 - par) * nblk;
                     atomicAdd(&cnt[par], 1);
-                    w.merge_list[atomicAdd(&w.chg_n[par], 1)] = i;  // at most once per particle
+                    // listed (at most once per particle): the cell whose record B1 clears
+                    w.p_prev[atomicAdd(&w.chg_n[par], 1)] = before;
                     atomicMin(&w.chg_n[3 - par], i);
                     if (before >= 0)
                         atomicMin(&mark[(before / w.W >> 3) * w.amw + ((before % w.W) >> 3)], (uint32_t)i);
                     if (after >= 0) atomicMin(&mark[(after / w.W >> 3) * w.amw + ((after % w.W) >> 3)], (uint32_t)i);
-                    w.p_prev[i] = before;  // the cell whose record B1 clears
                 }
             }
         }
@@ -680,12 +685,12 @@ __global__ void __launch_bounds__(SERIAL_THREADS) k_part_serial(const WorldDev *
         // this iteration), and the marks A read (set by the last iteration's changes)
         {
             const int na = active_worlds(
-                n_worlds, [&](int k) { return __ldcg(&worlds[k].chg_n[par]); }, s_ids, s_apref, s_warp);
+                n_worlds, [&](int k) { return n_worlds == 1 ? changed : __ldcg(&worlds[k].chg_n[par]); }, s_ids,
+                s_apref, s_warp);
             for (int g = gtid; g < s_apref[na]; g += gstride) {
                 const int j = entry_of(s_apref, na, g);
                 const WorldDev &w = worlds[s_ids[j]];
-                const int i = w.merge_list[g - s_apref[j]];
-                const int c = w.p_prev[i];
+                const int c = w.p_prev[g - s_apref[j]];
                 if (c >= 0) w.df[c] = 0;
             }
         }
@@ -709,13 +714,15 @@ __global__ void __launch_bounds__(SERIAL_THREADS) k_part_serial(const WorldDev *
         // index stays. The last iteration's counts have been used: cleared for the next.
         {
             const int na = active_worlds(
-                n_worlds, [&](int k) { return __ldcg(&worlds[k].chg_n[par]) > 0 ? parts(k) : 0; }, s_ids,
+                n_worlds,
+                [&](int k) { return n_worlds == 1 || __ldcg(&worlds[k].chg_n[par]) > 0 ? parts(k) : 0; }, s_ids,
                 s_apref, s_warp);
             for (int g = gtid; g < s_apref[na]; g += gstride) {
                 const int j = entry_of(s_apref, na, g);
                 const WorldDev &w = worlds[s_ids[j]];
                 const int i = g - s_apref[j];
-                const int c = fill_of(w, i);
+                const int kc = w.p_cell[i];
+                const int c = w.p_state[i] == PS_FILL ? kc : -1;
                 // records only grow, so one already at or above this fill's code stays
                 // there: only the cells cleared in B1 take atomics
                 if (c >= 0 && __ldcg(&w.df[c]) < fill_code(i)) atomicMax(&w.df[c], fill_code(i));
