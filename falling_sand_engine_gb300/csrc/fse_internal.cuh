@@ -196,7 +196,7 @@ struct WorldDev {
     long long *ledger;      // [LED_ROWS][MAXMAT]
     int32_t *err;
     unsigned *bar;          // grid barrier {count, generation} of the cooperative deposit kernel
-    uint8_t *airmap;        // per 8x8 block of cells: 1 if it held AIR when the particle tick began
+    uint8_t *airmap;        // per 8x8 block of cells: whether it held AIR (1) or liquid (2) when the particle tick began
     int amw, amh;           // airmap size in blocks
     // render state, NULL unless the world renders: cells written since the last
     // dirty pass, and the tick's flows per cell (Q16.16, x then y, wrapping sums)
