@@ -465,8 +465,8 @@ __device__ __forceinline__ void grid_sync(GridBar *gb, unsigned nblocks, int32_t
 
 constexpr int SERIAL_MAX_ITER = 1 << 16;
 constexpr int SERIAL_MAX_WORLDS = 4096;  // worlds of one launch (a batch holds at most 4095)
-constexpr int ONE_BLOCK_PARTICLES = 4096;  // up to here the update runs in one block,
-constexpr int BLOCK_PARTICLES = 1024;      // beyond in one block for each so many particles
+constexpr int ONE_BLOCK_PARTICLES = 1024;  // up to here the update runs in one block,
+constexpr int BLOCK_PARTICLES = 256;       // beyond in one block for each so many particles
 constexpr int SERIAL_THREADS = 1024;  // one block per SM: 152 arrivals at each grid barrier
 
 // index g of a flattened index space: its entry in s_pref (prefix sums over the
@@ -584,9 +584,11 @@ __global__ void __launch_bounds__(SERIAL_THREADS) k_part_serial(const WorldDev *
     __syncthreads();
     const int total = s_pref[n_worlds];
     auto parts = [&](int k) { return s_pref[k + 1] - s_pref[k]; };
-    // Small populations run on few blocks, and the fewest on one, whose barriers are the
-    // block's own: with all 152 blocks the ~30 grid barriers of an update cost more than
-    // its work.
+    // Small populations run on few blocks, whose grid barriers are cheaper than those of all
+    // 152, and the fewest on one, whose barriers are the block's own. A quarter of a block's
+    // threads' worth of particles spreads their spirals over more warps: with 1024 a block the
+    // 8192 x 8192 world with 200 boxes took 16.1 ms a step, with 256 14.9; one block up to
+    // 512, 1024 or 4096 particles measured the same.
     const unsigned nb = min(gridDim.x, total <= ONE_BLOCK_PARTICLES
                                            ? 1u
                                            : (unsigned)(total + BLOCK_PARTICLES - 1) / BLOCK_PARTICLES);
@@ -622,8 +624,13 @@ __global__ void __launch_bounds__(SERIAL_THREADS) k_part_serial(const WorldDev *
                                         },
                                         s_ids, s_apref, s_warp);
         const int total_a = s_apref[n_act];
-        for (int gb0 = gtid - lane; gb0 < total_a; gb0 += gstride) {
-            const int g = gb0 + lane;
+        // Where one pass takes all, neighbours in the list go to different warps: those that
+        // search spirals come in runs (a body's displaced particles), and a warp walks its
+        // particles' spirals one after another. Larger populations keep coalesced loads.
+        const bool spread = total_a <= gstride;
+        const int nwarps = gstride / 32, warp = gtid / 32;
+        for (int gb0 = spread ? 0 : gtid - lane; gb0 < total_a; gb0 += gstride) {
+            const int g = spread ? lane * nwarps + warp : gb0 + lane;
             bool work = g < total_a, spiral = false;
             int wi = 0, i = 0, before = -1, cell = -1;
             uint8_t kind = PS_ALIVE;
