@@ -10,7 +10,6 @@
 #include <cctype>
 #include <atomic>
 #include <mutex>
-#include <set>
 #include <string>
 #include <vector>
 
@@ -251,13 +250,10 @@ static bool flow_thresholds(double k, float thr[256]) {
 // 1 + the number of different densities below theirs (at most 254 of them, as the table
 // always holds an AIR and a SOLID material). A NaN compares with nothing: nothing sinks
 // into it (255), and as sand it sinks into AIR alone (the colour pass's cw_sink).
-uint32_t density_rank(const HostMat &m) {
+uint32_t density_rank(const HostMat &m, const std::vector<float> &sorted) {
     if (m.type == T_AIR) return 0u;
     if (m.type == T_SOLID || std::isnan(m.density)) return 255u;
-    std::set<float> below;
-    for (const HostMat &o : g_mats)
-        if (o.type != T_AIR && o.type != T_SOLID && o.density < m.density) below.insert(o.density);
-    return 1u + (uint32_t)below.size();
+    return 1u + (uint32_t)(std::lower_bound(sorted.begin(), sorted.end(), m.density) - sorted.begin());
 }
 
 void build_table(MatTable &t) {
@@ -274,6 +270,11 @@ void build_table(MatTable &t) {
     t.id_lava = idx("LAVA", -1);
     t.id_steam = idx("STEAM", -1);
     t.id_obsidian = idx("OBSIDIAN", -1);
+    std::vector<float> densities;  // the different ones that can be sunk into
+    for (const HostMat &m : g_mats)
+        if (m.type != T_AIR && m.type != T_SOLID && !std::isnan(m.density)) densities.push_back(m.density);
+    std::sort(densities.begin(), densities.end());
+    densities.erase(std::unique(densities.begin(), densities.end()), densities.end());
     for (int i = 0; i < t.n; i++) {
         const HostMat &m = g_mats[i];
         int iters = std::min(std::max(m.iterations, 0), 255);
@@ -281,7 +282,7 @@ void build_table(MatTable &t) {
         t.a[i] = (uint32_t)m.type | ((uint32_t)iters << 8) | ((uint32_t)slip << 16) |
                  ((uint32_t)max_stability(m.slip) << 24);
         t.word[i] = (uint32_t)i | ((uint32_t)m.type << MW_TYPE_SHIFT) | (i == t.id_fire ? MW_FIRE : 0u) |
-                    (m.n_react > 0 ? MW_REACT : 0u) | (density_rank(m) << MW_RANK_SHIFT);
+                    (m.n_react > 0 ? MW_REACT : 0u) | (density_rank(m, densities) << MW_RANK_SHIFT);
         t.f_base[i] = m.f_base;
         t.f_pack[i] = (uint32_t)(m.f_shift & 0xFF) | ((uint32_t)(m.f_lo & 0xFFF) << 8) | ((uint32_t)(m.f_mod & 0xFFF) << 20);
         t.f_scalar[i] = m.f_scalar;

@@ -2,18 +2,31 @@
 // as one colour-pass kernel.
 //
 // A launch handles one chunk colour of one iteration (world.cpp:1050-1077) for a
-// list of chunks, possibly of many worlds. Each CTA stages its chunk plus a halo in
-// shared memory (id, flags, scalar, colour; the pending fluid diff stays in HBM and
-// is touched only by SOUP cells), runs sweeps A, B and C as sequences of lattice
-// sub-phases separated by __syncthreads(), and writes back only the cells it
-// changed. Inside a sub-phase every cell is processed by its own thread; the
-// lattice spacing makes every write set disjoint from every other cell's read and
-// write sets, so the result does not depend on thread timing.
+// list of chunks, possibly of many worlds, or every pass of a tick (the fused tick).
+// Each CTA stages its chunk plus a halo in shared memory (a word per cell, scalar,
+// colour; the pending fluid diff stays in HBM and is touched only by SOUP cells), runs
+// sweeps A, B and C as sequences of lattice sub-phases separated by __syncthreads(), and
+// writes back only the cells it changed. The lattice spacing makes every write set of a
+// sub-phase disjoint from every other cell's read and write sets, so the result does not
+// depend on thread timing.
 //
-// A sub-phase costs about one rule's dependent chain of shared-memory accesses
-// plus one barrier, whatever the mix of materials in a warp (sorting cells by type
-// first was measured and did not pay), so every thread simply runs the rule of its
-// own cells; spawned particles are ranked in the lattice enumeration order.
+// What bounds it: the slowest warp of each of the 30 sub-phases, one after another, as the
+// tile takes an SM's shared memory and a chunk-pass its SM. A wet 128 x 128 chunk takes 95 us
+// a pass (140 us before the steps below), of which sweep A's rules take about 45%,
+// finding and listing its cells and its barriers 20%, sweep B 25%, staging and write-back
+// 10%; DRAM moves 3% of what it could. So what counts is the length of the chain of
+// dependent instructions and loads that a warp goes through in a sub-phase:
+// - one word per cell answers what a rule asks of a neighbour (see CW_*);
+// - a sub-phase first finds the cells that a rule may change and deals them to the threads,
+//   liquids to the first warps and the others to the last, so that a warp runs one rule
+//   with most of its lanes; the rare cases (free fall, another liquid beside, fire,
+//   reactions) are with the others, so that they do not lengthen the flowing liquids' rule;
+// - what comes from HBM (the diff of a displaced or falling liquid, a staging slot) is asked
+//   for as soon as its address is known, and used after the next barrier where it can be.
+// Tried and slower: blocks of the chunk that wait only for their neighbours (mbarrier
+// arrivals release, and so wait for the diff reductions in flight: 215 us a pass against
+// 131 then), requesting the next sub-phase's diffs a sub-phase ahead (512 x 512 tick 1.005 ->
+// 1.052 ms).
 //
 // The reference copies neighbour cells into locals and writes those copies back
 // later; no rule modifies such a neighbour between the copy and the write-back, so
@@ -1339,8 +1352,7 @@ static size_t tile_smem(int C, int own, int halo, int width) {
 // updates the top half of its rows, rank 1 the bottom half, each staging its half
 // plus the rows its rules reach (the shared rows are kept equal by mirrored writes)
 // and writing back its own rows; sub-phases end with a cluster barrier. A chunk's
-// sub-phases then run on two SMs, and an SM holds halves of two chunks whose
-// barriers interleave.
+// sub-phases then run on two SMs.
 // CC: the chunk edge where it is known when compiling (128, the reference's), else 0:
 // the tile's rows, planes and lattices are then constants
 template <int HALO, bool TEMP, bool SEQ, bool F32, bool PAIR = false, bool FUSED = false, int CC = 0>
