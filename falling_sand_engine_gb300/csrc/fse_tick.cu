@@ -1747,7 +1747,11 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
         // of one step touch the same cell. Each row ranks its own spawns.
         auto sweeps_seq = [&](const auto &Tl) {
             const int s = mode == 2 ? 11 : (mode == 1 ? 5 : 3);
-            const int k = tid, dy = chh - 1 - tid;
+            // row k on lane k / 32 of warp k % 32: a warp runs the rules of its lanes' cells one
+            // after another, so four rows a warp on all warps end a step sooner than 32 rows on
+            // four (1024 x 512 with f32 amounts: 18.7 against 15.2 ms a step)
+            static_assert(CP_THREADS >= 1024, "a thread for each of 32 rows on each of 32 lanes");
+            const int k = (tid & 31) * 32 + (tid >> 5), dy = chh - 1 - k;
             const bool row = k < chh;
             int spawned = 0;
             for (int sweep = 0; sweep < 3; sweep++) {
@@ -1788,7 +1792,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                     __syncthreads();
                 }
             }
-            if (tid < w.cp_rows) w.cp_count[cp * w.cp_rows + tid] = spawned;
+            if (k < w.cp_rows) w.cp_count[cp * w.cp_rows + k] = spawned;
         };
         auto sweeps = [&](const auto &Tl) {
 #pragma unroll 1
