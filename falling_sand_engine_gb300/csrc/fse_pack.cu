@@ -190,14 +190,14 @@ __device__ int seg_run(Src &s, int n, int a, int b, int &anchor, uint8_t *dst, i
     const int mflimit = n - 12, mend = n - 5;
     const int lim = min(mend, b);       // a match ends at the latest here
     const int stop = min(b, mflimit + 1);  // matches start before here
+    const int dist = c_dist[lane & 15];  // this lane's candidate
     int p = a, m = 0, first = -1, fixed = 0;
     if (!EMIT) anchor = a;
     while (p < stop && op >= 0) {
         // candidates at p itself: lane k < 16 tests distance k
         s.need(p - ENC_BACK, p + 136);
         int q0 = p;
-        unsigned cm = __ballot_sync(FULL, lane < 16 && c_dist[lane & 15] <= p && p + 4 <= lim &&
-                                              s.load4(p) == s.load4(p - c_dist[lane & 15]));
+        unsigned cm = __ballot_sync(FULL, lane < 16 && dist <= p && p + 4 <= lim && s.load4(p) == s.load4(p - dist));
         if (!cm) {
             // none: the first position of [p + 1, p + 33) with a 4-byte match at some distance
             const int q = p + 1 + lane;
@@ -220,22 +220,33 @@ __device__ int seg_run(Src &s, int n, int a, int b, int &anchor, uint8_t *dst, i
             cm = __shfl_sync(FULL, m, f);
             s.need(q0 - ENC_BACK, q0 + 136);
         }
-        // run lengths: lane k extends candidate k by itself up to 128 bytes, 4 at a time
+        // run lengths: lane k extends candidate k by itself up to 128 bytes, 16 at a time (ten
+        // words loaded together; 4 bytes at a time each step was a shared-memory round trip of
+        // its own, four loads for the unaligned pair: packing 4096 x 2048 cells took 2.19 ms
+        // against 1.86). The last step ends within the 136 bytes that the window covers after q0.
         int L = 0;
         bool open = false;
         if (lane < 16 && ((cm >> lane) & 1u)) {
-            const int d = c_dist[lane];
+            const int d = dist;
             const int top = min(lim - q0, 128);
             L = 4;
             while (L < top) {
-                const int take = min(4, top - L);
-                uint32_t diff = s.load4(q0 + L) ^ s.load4(q0 + L - d);
-                if (take < 4) diff |= 0xffffffffu << (8 * take);
-                if (diff) {
-                    L += (__ffs(diff) - 1) >> 3;
-                    break;
+                const int x = q0 + L, y = x - d;
+                uint32_t u[5], v[5];
+#pragma unroll
+                for (int k = 0; k < 5; k++) {
+                    u[k] = s.word((x >> 2) + k);
+                    v[k] = s.word((y >> 2) + k);
                 }
-                L += 4;
+                int same = 16;
+#pragma unroll
+                for (int k = 3; k >= 0; k--) {
+                    const uint32_t diff = __funnelshift_r(u[k], u[k + 1], (x & 3) * 8) ^
+                                          __funnelshift_r(v[k], v[k + 1], (y & 3) * 8);
+                    if (diff) same = 4 * k + ((__ffs(diff) - 1) >> 3);
+                }
+                L = min(L + same, top);
+                if (same < 16) break;
             }
             open = L == 128 && q0 + 128 < lim;
         }
