@@ -399,7 +399,8 @@ class World:
 
     # -- exact checkpoints
     def trim(self):
-        """Free the device scratch kept by pack / unpack / the tile-struct calls."""
+        """Free the device scratch kept by pack / unpack / the tile-struct and body calls and
+        the particle read-out."""
         check(self.lib.fse_world_trim(self.h), "trim")
 
     def checkpoint(self):
