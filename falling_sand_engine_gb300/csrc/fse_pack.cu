@@ -223,36 +223,41 @@ __device__ int seg_run(Src &s, int n, int a, int b, int &anchor, uint8_t *dst, i
             cm = __shfl_sync(FULL, m, f);
             s.need(q0 - ENC_BACK, q0 + 136);
         }
-        // run lengths: lane k extends candidate k by itself up to 128 bytes, 16 at a time (ten
-        // words loaded together; 4 bytes at a time each step was a shared-memory round trip of
-        // its own, four loads for the unaligned pair: packing 4096 x 2048 cells took 2.19 ms
-        // against 1.86). The last step ends within the 136 bytes that the window covers after q0.
-        int L = 0;
-        bool open = false;
-        if (lane < 16 && ((cm >> lane) & 1u)) {
-            const int d = dist;
-            const int top = min(lim - q0, 128);
-            L = 4;
-            while (L < top) {
-                const int x = q0 + L, y = x - d;
+        // run lengths: lanes k and k + 16 extend candidate k up to 128 bytes, 32 a step (ten
+        // words loaded together by each: packing 4096 x 2048 cells 1.62 -> 1.58 ms against 16 a
+        // step; 4 bytes a step took 0.33 ms more). The last step ends within the 136 bytes that
+        // the window covers after q0. Finding q0 from the equal bytes of six words, lane k at
+        // distance k for 16 positions at once, instead of the test at p and the scan above was
+        // slower (1.62 -> 1.90 ms): most matches begin at p.
+        const int top = min(lim - q0, 128);
+        const bool mine = (cm >> (lane & 15)) & 1u;
+        int L = 4;
+        bool go = mine && L < top;
+        while (__any_sync(FULL, go)) {
+            int same = 0;
+            if (go) {
+                const int x = q0 + L + (lane & 16), y = x - dist;
                 uint32_t u[5], v[5];
 #pragma unroll
                 for (int k = 0; k < 5; k++) {
                     u[k] = s.word((x >> 2) + k);
                     v[k] = s.word((y >> 2) + k);
                 }
-                int same = 16;
+                same = 16;
 #pragma unroll
                 for (int k = 3; k >= 0; k--) {
                     const uint32_t diff = __funnelshift_r(u[k], u[k + 1], (x & 3) * 8) ^
                                           __funnelshift_r(v[k], v[k + 1], (y & 3) * 8);
                     if (diff) same = 4 * k + ((__ffs(diff) - 1) >> 3);
                 }
-                L = min(L + same, top);
-                if (same < 16) break;
             }
-            open = L == 128 && q0 + 128 < lim;
+            const int other = __shfl_xor_sync(FULL, same, 16);
+            const int lo = lane < 16 ? same : other;
+            const int add = lo < 16 ? lo : same + other;
+            L = min(L + add, top);
+            go = go && add == 32 && L < top;
         }
+        const bool open = mine && lane < 16 && L == 128 && q0 + 128 < lim;
         unsigned alive = __ballot_sync(FULL, open);
         if (alive) {
             // runs of 128 bytes and more: the whole warp extends them, 128 bytes per step
