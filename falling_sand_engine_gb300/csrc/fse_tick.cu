@@ -1810,7 +1810,12 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                         if (Tl.air(i)) bits |= 1u << b;
                     S.air[sx * 5 + wi] = bits;
                 }
-                __syncthreads();
+                // a pair waits for both snapshots: each reads rows that the partner's first
+                // sub-phase already changes (a liquid that dries up is mirrored into this tile)
+                if constexpr (PAIR)
+                    cluster_sync();
+                else
+                    __syncthreads();
             }
             int px, py;
             lattice(sweep, mode, px, py);
