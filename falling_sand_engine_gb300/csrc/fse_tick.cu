@@ -200,6 +200,8 @@ __device__ __forceinline__ void mbar_init(uint64_t *bar, unsigned count) {
 }
 // orders this thread's generic shared-memory accesses before later async-proxy ones
 __device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+// the same for global memory
+__device__ __forceinline__ void fence_proxy_async_global() { asm volatile("fence.proxy.async.global;" ::: "memory"); }
 __device__ __forceinline__ void mbar_expect_tx(uint64_t *bar, unsigned bytes) {
     asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_addr(bar)), "r"(bytes)
                  : "memory");
@@ -1571,6 +1573,9 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
         // chunk's ids decide the skip and the lattice mode.
         if (tma && tid == 0) {
             const char *tm = static_cast<const char *>(w.tmap);
+            // what the neighbours wrote (seen through their flags and the barrier above) comes
+            // before these copies, which read it through the async proxy
+            if constexpr (FUSED) fence_proxy_async_global();
             mbar_expect_tx(&s_tma_bar, 2u * (uint32_t)nfull * 4u);
             tma_load_2d(Tl.s_sc, tm, Tl.x0, Tl.y0, &s_tma_bar);
             tma_load_2d(Tl.s_col, tm + 128, Tl.x0, Tl.y0, &s_tma_bar);
@@ -2121,6 +2126,8 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
                 }
             }
         }
+        // the written cells come before the tensor copies of the chunk-passes that wait for this one
+        if constexpr (FUSED && kTma) fence_proxy_async_global();
         if (!SEQ && tid == 0 && rank == 0) w.cp_count[cp] = S.running[rb];
         // the chunk-pass's ledger counts (the sweeps ended with a barrier)
         for (int i = tid; i < LED_TICK * 64; i += T) {
