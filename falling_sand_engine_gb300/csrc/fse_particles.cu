@@ -1128,10 +1128,14 @@ cudaError_t launch_particle_tick(WorldDev *d_worlds, int n_worlds, const MatTabl
         // the blocks per SM depend on the shared memory the table's size asks for
         if (n_worlds > SERIAL_MAX_WORLDS) return cudaErrorInvalidValue;
         const size_t dyn = (size_t)(3 * n_worlds + 2) * sizeof(int);
-        static size_t dyn_set = 0;
-        if (dyn > 48 * 1024 && dyn > dyn_set) {
-            cudaFuncSetAttribute(k_part_serial, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dyn);
-            dyn_set = dyn;
+        // with the kernel's static arrays the table of the largest batches passes the 48 KB
+        // that need no opt-in
+        static bool opted_in = false;
+        if (!opted_in) {
+            const cudaError_t e = cudaFuncSetAttribute(k_part_serial, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                       (int)((3 * SERIAL_MAX_WORLDS + 2) * sizeof(int)));
+            if (e != cudaSuccess) return e;
+            opted_in = true;
         }
         static int nsm = 0;
         if (!nsm) {
@@ -1152,7 +1156,9 @@ cudaError_t launch_particle_tick(WorldDev *d_worlds, int n_worlds, const MatTabl
         attr[0].val.cooperative = 1;
         cfg.attrs = attr;
         cfg.numAttrs = 1;
-        cudaLaunchKernelEx(&cfg, k_part_serial, (const WorldDev *)d_worlds, n_worlds, mt);
+        // the kernels below work on the outcomes this one writes
+        const cudaError_t e = cudaLaunchKernelEx(&cfg, k_part_serial, (const WorldDev *)d_worlds, n_worlds, mt);
+        if (e != cudaSuccess) return e;
     }
     k_merge<<<n_worlds, 1024, 0, s>>>(d_worlds);
     const size_t pref = (size_t)(n_worlds + 1) * sizeof(int);
