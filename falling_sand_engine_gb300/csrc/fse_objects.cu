@@ -386,7 +386,8 @@ static int obj_prepare(fse_world *w) {
             return FSE_E_NOMEM;
         }
         w->bytes += n * 4;
-        cudaMemset(w->claim, 0xff, n * 4);
+        // in the order of the world's stream, which does not wait for the default stream
+        FSE_CUDA_TRY(cudaMemsetAsync(w->claim, 0xff, n * 4, w->stream));
     }
     return FSE_OK;
 }
