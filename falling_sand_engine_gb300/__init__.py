@@ -399,8 +399,8 @@ class World:
 
     # -- exact checkpoints
     def trim(self):
-        """Free the device scratch kept by pack / unpack / the tile-struct and body calls and
-        the particle read-out."""
+        """Free the device scratch kept by pack / unpack / the tile-struct calls, and what the
+        body calls and the particle read-out left in the memory that all worlds share."""
         check(self.lib.fse_world_trim(self.h), "trim")
 
     def checkpoint(self):

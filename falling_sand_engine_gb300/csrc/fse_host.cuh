@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -52,11 +53,8 @@ struct fse_world {
     uint32_t *obj_list;   // object list scratch
     size_t obj_list_cap;
     int64_t *obj_n;       // object list count
-    uint8_t *obj_scr;     // stamp / readback workspace, grown on first use and kept until fse_world_trim
-    size_t obj_scr_bytes;
-    // fse_particles_read's records, grown on first use (at most 15 MB) and kept until fse_world_trim
-    uint32_t *rec;
-    size_t rec_bytes;
+    uint32_t *rec;        // REC_OWN particle records of fse_particles_read, where no more are to be had
+    std::mutex rec_mu;    // held while rec is in use
     std::map<int, cudaGraphExec_t> graphs;  // n_ticks -> step graph
     std::map<int, long long> graph_kernels;  // n_ticks -> kernels one replay launches
     size_t bytes;         // device bytes owned
@@ -120,6 +118,27 @@ int particle_scan_blocks();
 int sm_count();
 int status_from_err(int err);
 int tick_halo();
+
+// Device memory of one call that ends with a synchronisation of its stream: a block that
+// such a call left idle, or a new one. (Nine cudaMalloc and cudaFree a call, each of which
+// waits for the device, took longer than a stamp of a few bodies.) The idle blocks are one
+// set for all worlds, streams and threads of a device, at most SCRATCH_KEEP bytes, until
+// fse_world_trim: memory that every world kept for itself would be out of sight of a
+// server's budget.
+constexpr size_t SCRATCH_KEEP = 64 << 20;
+struct CallScratch {
+    explicit CallScratch(cudaStream_t stream) : s(stream) {}
+    CallScratch(const CallScratch &) = delete;
+    CallScratch &operator=(const CallScratch &) = delete;
+    ~CallScratch();           // waits for the stream, then the block is idle
+    bool take(size_t bytes);  // once; false: no memory
+    uint8_t *p = nullptr;
+    size_t size = 0;
+    void *from = nullptr;
+    cudaStream_t s;
+};
+void scratch_trim();  // frees the idle blocks
+constexpr int REC_OWN = 2048;  // particle records that every world has room for
 
 // one world::tick() + optionally world::tickCells() for a set of worlds that
 // share a device descriptor table

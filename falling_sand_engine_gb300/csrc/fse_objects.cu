@@ -411,9 +411,7 @@ static int obj_run(fse_world *w, fse_body *bodies, int n, int mode, int64_t *out
         prefix[b + 1] = prefix[b] + (uint32_t)(bodies[b].w * bodies[b].h);
     }
     size_t total = prefix[n];
-    // the call's workspace, kept in the world (fse_world_trim frees it): nine allocations
-    // and as many freeings a call, each of which waits for the device, took longer than
-    // the kernels of a few bodies
+    // the call's workspace
     size_t bytes = 0;
     auto part = [&](size_t b) {
         const size_t at = bytes;
@@ -423,17 +421,9 @@ static int obj_run(fse_world *w, fse_body *bodies, int n, int mode, int64_t *out
     const size_t o_b = part(n * sizeof(fse_body)), o_pref = part((size_t)(n + 1) * 4);
     const size_t o_tiles = part(total * sizeof(ObjTile)), o_held = part(total * 4);
     const size_t o_blk = part(OBJ_BLOCKS * 4), o_rem = part(8);
-    if (w->obj_scr_bytes < bytes) {
-        if (w->obj_scr) cudaFree(w->obj_scr);
-        w->obj_scr = nullptr;
-        w->obj_scr_bytes = 0;
-        if (cudaMalloc((void **)&w->obj_scr, bytes) != cudaSuccess) {
-            w->obj_scr = nullptr;
-            return FSE_E_NOMEM;
-        }
-        w->obj_scr_bytes = bytes;
-    }
-    uint8_t *s = w->obj_scr;
+    CallScratch scr(w->stream);
+    if (!scr.take(bytes)) return FSE_E_NOMEM;
+    uint8_t *s = scr.p;
     fse_body *d_b = (fse_body *)(s + o_b);
     uint32_t *d_pref = (uint32_t *)(s + o_pref);
     ObjTile *d_tiles = (ObjTile *)(s + o_tiles);

@@ -977,12 +977,7 @@ int fse_world_trim(fse_world *w) {
     if (w->tile_stage) cudaFree(w->tile_stage);
     w->tile_stage = nullptr;
     w->tile_stage_bytes = 0;
-    if (w->obj_scr) cudaFree(w->obj_scr);
-    w->obj_scr = nullptr;
-    w->obj_scr_bytes = 0;
-    if (w->rec) cudaFree(w->rec);
-    w->rec = nullptr;
-    w->rec_bytes = 0;
+    scratch_trim();
     return FSE_OK;
 }
 

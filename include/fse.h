@@ -281,8 +281,8 @@ int fse_world_pack(fse_world *world, int generation_phase, uint8_t *out, int64_t
 int fse_world_unpack(fse_world *world, const uint8_t *in, const int64_t *offsets, int n_chunks, int8_t *out_phases,
                      int *out_bad_chunk);
 /* Pack, unpack and the tile-struct calls keep their device scratch (about 1 MB per
- * chunk for pack and unpack) between calls, the body calls their workspace and
- * fse_particles_read its records (at most 15 MB); this frees them. */
+ * chunk for pack and unpack) between calls; this frees them, and what the body calls and
+ * the particle read-out left in the memory that all worlds share (at most 64 MB). */
 int fse_world_trim(fse_world *world);
 
 /* Exact checkpoint of a world (the .pack files keep only material, colour and
