@@ -625,12 +625,10 @@ __device__ __forceinline__ void copy_run(uint8_t *dst, uint8_t *ring, const uint
         const uint8_t v = src8[(spos + lane) & smask];
         dst[k0 + lane] = v;
         ring[(k0 + lane) & (DEC_RING - 1)] = v;
-    } else if (lane >= 4 && lane - 4 < len - t0) {
-        const int j = t0 + lane - 4;
-        const uint8_t v = src8[(spos + j) & smask];
-        dst[k0 + j] = v;
-        ring[(k0 + j) & (DEC_RING - 1)] = v;
     }
+    const int tail = t0 + lane;  // a byte of the tail, loaded now and written last
+    const uint8_t tv = tail < len ? src8[(spos + tail) & smask] : 0;
+    __syncwarp();  // a run longer than the ring writes its slots again: the later bytes stay
     const uint32_t *src32 = reinterpret_cast<const uint32_t *>(src8);
     uint32_t *dst32 = reinterpret_cast<uint32_t *>(dst);
     uint32_t *ring32 = reinterpret_cast<uint32_t *>(ring);
@@ -641,6 +639,11 @@ __device__ __forceinline__ void copy_run(uint8_t *dst, uint8_t *ring, const uint
         const uint32_t v = sh ? __funnelshift_r(w0, src32[(sw + i + 1) & wmask], sh) : w0;
         dst32[a0 + i] = v;
         ring32[(a0 + i) & (DEC_RING / 4 - 1)] = v;
+    }
+    __syncwarp();
+    if (tail < len) {
+        dst[k0 + tail] = tv;
+        ring[(k0 + tail) & (DEC_RING - 1)] = tv;
     }
 }
 
