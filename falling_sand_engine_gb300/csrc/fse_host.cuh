@@ -161,7 +161,7 @@ bool temp_track_of(const std::vector<fse_world *> &ws);
 // Launch shapes of the colour pass (threads per CTA, chunk workers; 0 = one per chunk):
 // 0 one 1024-thread CTA per chunk; 1 one persistent CTA per SM walking the chunks;
 // 2 each chunk split over a CTA pair (a cluster of two 512-thread CTAs); 3 persistent
-// pairs, two CTAs per SM; 4 the fused tick (every pass in one launch, one CTA per SM,
+// pairs, one pair per SM of the GPU; 4 the fused tick (every pass in one launch, one CTA per SM,
 // chunk-passes started as their neighbourhoods finish), FUSED_GRID
 constexpr int COLOUR_SHAPES = 5;
 constexpr int FUSED_GRID = -1;

@@ -1356,9 +1356,12 @@ static size_t tile_smem(int C, int own, int halo, int width) {
 // and writing back its own rows; sub-phases end with a cluster barrier. A chunk's
 // sub-phases then run on two SMs.
 // CC: the chunk edge where it is known when compiling (128, the reference's), else 0:
-// the tile's rows, planes and lattices are then constants
+// the tile's rows, planes and lattices are then constants. Two CTAs of pairs share an SM up
+// to edge 124, so they are held to 64 registers each; one of edge 128 takes 120 KB, an SM of
+// its own and all the registers it asks for (4096 x 2048 step on pairs 3.02 -> 2.47 ms,
+// 512 x 512 1.58 -> 1.33; at edge 64, where two fit, 4.0 ms against 5.0 with one)
 template <int HALO, bool TEMP, bool SEQ, bool F32, bool PAIR = false, bool FUSED = false, int CC = 0>
-__global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 : 1)
+__global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR && CC != 128 ? 2 : 1)
     k_colour_pass(const WorldDev *__restrict__ worlds, const uint32_t *__restrict__ items, int n_items, int iter_arg,
                   int tk_arg, const MatTable *__restrict__ mt, const FusedTick ft) {
     static_assert(!(PAIR && SEQ), "the reference order runs a chunk in one CTA");
@@ -1537,7 +1540,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR ? 2 :
         TileData Tl;
         const bool tma = kTma && w.tmap != nullptr;
         // with TMA the rows start on a 16-byte boundary and are tma_tile_width wide
-        Tl.RW = CC || tma ? tma_tile_width(C) : C + HALO_LO + HALO;
+        Tl.RW = (CC && !PAIR) || tma ? tma_tile_width(C) : C + HALO_LO + HALO;
         Tl.RHF = own + HALO_LO + HALO;
         Tl.RHI = own + HALO_LO + 10;
         Tl.x0 = tma ? ((cx - HALO_LO) & ~3) : cx - HALO_LO;
@@ -2228,15 +2231,16 @@ static cudaError_t launch_fused_t(const WorldDev *worlds, const FusedTick &ft, c
 static size_t colour_pass_smem_pair(int C, int halo) { return tile_smem<CP_THREADS / 2>(C, C / 2, halo, 0); }
 
 // the chunks split over CTA pairs (thread-block clusters of two): `clusters` pairs
-template <int HALO, bool TEMP, bool F32>
-static cudaError_t launch_pair_t(const WorldDev *worlds, const uint32_t *items, int n_items, int iter, int tk,
-                                 const MatTable *mt, size_t sm, int clusters, cudaStream_t s) {
+template <int HALO, bool TEMP, bool F32, int CC>
+static cudaError_t launch_pair_cc(const WorldDev *worlds, const uint32_t *items, int n_items, int iter, int tk,
+                                  const MatTable *mt, size_t sm, int clusters, cudaStream_t s) {
     static size_t set = 0;
     if (set < sm) {
-        cudaFuncSetAttribute(k_colour_pass<HALO, TEMP, false, F32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sm);
-        // all of the unified L1/shared storage as shared memory, so that two CTAs fit an SM
-        cudaFuncSetAttribute(k_colour_pass<HALO, TEMP, false, F32, true>,
+        cudaFuncSetAttribute(k_colour_pass<HALO, TEMP, false, F32, true, false, CC>,
+                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
+        // all of the unified L1/shared storage as shared memory, so that two CTAs share an SM
+        // where they fit
+        cudaFuncSetAttribute(k_colour_pass<HALO, TEMP, false, F32, true, false, CC>,
                              cudaFuncAttributePreferredSharedMemoryCarveout, 100);
         set = sm;
     }
@@ -2252,8 +2256,15 @@ static cudaError_t launch_pair_t(const WorldDev *worlds, const uint32_t *items, 
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_colour_pass<HALO, TEMP, false, F32, true>, worlds, items, n_items, iter, tk, mt,
-                              FusedTick{});
+    return cudaLaunchKernelEx(&cfg, k_colour_pass<HALO, TEMP, false, F32, true, false, CC>, worlds, items, n_items, iter,
+                              tk, mt, FusedTick{});
+}
+
+template <int HALO, bool TEMP, bool F32>
+static cudaError_t launch_pair_t(const WorldDev *worlds, const uint32_t *items, int n_items, int iter, int tk,
+                                 const MatTable *mt, int C, size_t sm, int clusters, cudaStream_t s) {
+    if (C == 128) return launch_pair_cc<HALO, TEMP, F32, 128>(worlds, items, n_items, iter, tk, mt, sm, clusters, s);
+    return launch_pair_cc<HALO, TEMP, F32, 0>(worlds, items, n_items, iter, tk, mt, sm, clusters, s);
 }
 
 // Each translation unit that includes this file with one of the defines below
@@ -2290,11 +2301,11 @@ cudaError_t launch_colour_pass_pair(const WorldDev *worlds, const uint32_t *item
     const size_t sm = colour_pass_smem_pair(C, halo);
     if (temp) {
         if (halo == 5)
-            return launch_pair_t<5, true, FSE_PAIR_F32>(worlds, items, n_items, iter, tk, mt, sm, clusters, s);
-        return launch_pair_t<2, true, FSE_PAIR_F32>(worlds, items, n_items, iter, tk, mt, sm, clusters, s);
+            return launch_pair_t<5, true, FSE_PAIR_F32>(worlds, items, n_items, iter, tk, mt, C, sm, clusters, s);
+        return launch_pair_t<2, true, FSE_PAIR_F32>(worlds, items, n_items, iter, tk, mt, C, sm, clusters, s);
     }
-    if (halo == 5) return launch_pair_t<5, false, FSE_PAIR_F32>(worlds, items, n_items, iter, tk, mt, sm, clusters, s);
-    return launch_pair_t<2, false, FSE_PAIR_F32>(worlds, items, n_items, iter, tk, mt, sm, clusters, s);
+    if (halo == 5) return launch_pair_t<5, false, FSE_PAIR_F32>(worlds, items, n_items, iter, tk, mt, C, sm, clusters, s);
+    return launch_pair_t<2, false, FSE_PAIR_F32>(worlds, items, n_items, iter, tk, mt, C, sm, clusters, s);
 }
 #elif defined(FSE_TICK_F32_TU)
 // f32 liquid amounts (FSE_CFG_F32_FLUID), in the partitioned order (FSE_TICK_F32_TU
