@@ -1328,13 +1328,21 @@ struct SmemHeadT {
 // head, up to 128 bytes of padding (the planes start on a 128-byte boundary of the
 // window) and the planes of the largest tile
 template <int NT>
-static size_t tile_smem(int C, int own, int halo, int width) {
-    const size_t RW = (size_t)std::max(width, C + HALO_LO + halo), RHF = (size_t)own + HALO_LO + halo;
+constexpr size_t tile_smem(int C, int own, int halo, int width) {
+    const size_t RW = (size_t)(width > C + HALO_LO + halo ? width : C + HALO_LO + halo);
+    const size_t RHF = (size_t)own + HALO_LO + halo;
     const size_t RHI = (size_t)own + HALO_LO + 10;
     const size_t head = (sizeof(SmemHeadT<NT>) + 127) & ~(size_t)127;
     const size_t plane = (RW * RHF + 31) & ~(size_t)31;
     return 128 + head + (2 * plane + RW * RHI) * 4;
 }
+// The largest tile, a chunk of 128 with the 5-cell halo, beside the kernel's static
+// variables (the world's descriptor, the spawn velocities, the mbarrier and the fused
+// tick's words): a CTA takes at most 227 KB, and a launch that asks for more fails.
+constexpr size_t COLOUR_STATIC = ((sizeof(WorldDev) + 15) & ~(size_t)15) + ((sizeof(SpawnVel) + 15) & ~(size_t)15) + 32;
+static_assert(tile_smem<CP_THREADS>(128, 128, 5, 0) + COLOUR_STATIC <= 227 * 1024, "the 5-cell halo's tile");
+static_assert(tile_smem<CP_THREADS>(128, 128, 2, tma_tile_width(128)) + COLOUR_STATIC <= 227 * 1024,
+              "the tile of the tensor copies");
 
 // items: (world << 20) | chunk slot within the colour; iter, tk select the pass.
 // FUSED: every pass of the tick in one launch (iter, tk, items and n_items unused;
