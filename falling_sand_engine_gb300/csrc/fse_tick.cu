@@ -421,21 +421,28 @@ struct Ctx {
 
 // Ledger counts of one chunk-pass are 32-bit shared counters (native shared atomics;
 // 64-bit ones are compare-and-swap loops), added to the world's 64-bit ledger when the
-// chunk-pass ends. A counter takes amounts below 1024 only, so that a chunk-pass, with
-// at most 3 sweeps x 16384 cells and a few dozen entries a cell, cannot overflow it;
-// larger ones go to the world's ledger at once.
+// chunk-pass ends. A counter takes amounts below LED_SMALL only, larger ones go to the
+// world's ledger at once, so that a chunk-pass cannot overflow it: a cell's turns make at
+// most LED_ENTRIES entries in a row. In sweep A a sand's interactions make the most, at most
+// 4 of a pair (fse_material_set_interaction) with boxes of at most 25 cells each (a visited
+// box has no negative corner and reaches 5 cells at the farthest); fire converts at most 27
+// cells, water on lava 11, a reaction 4, a flow makes 4 new cells; sweeps B and C convert
+// the cell itself.
+constexpr int LED_SMALL = 1024, LED_ENTRIES = 128;
+static_assert(4 * 25 + 2 <= LED_ENTRIES && 27 + 2 <= LED_ENTRIES, "entries of a cell");
+static_assert((long long)LED_ENTRIES * 128 * 128 * (LED_SMALL - 1) <= INT32_MAX, "a counter holds a chunk-pass");
 constexpr int LED_TICK = 4;  // the rows the cell update counts in: all but LED_XN and LED_XF
 __host__ __device__ constexpr int led_slot(int row) { return row > LED_XN ? row - 1 : row; }
 __device__ __forceinline__ void led_add(Ctx &c, int row, uint32_t w, int32_t v) {
     if (v == 0 || cw_air(w)) return;
     const int mat = cw_id(w);
-    if (mat < 64 && v > -1024 && v < 1024)
+    if (mat < 64 && v > -LED_SMALL && v < LED_SMALL)
         atomicAdd(&c.led_s[led_slot(row) * 64 + mat], v);
     else
         atomicAdd((unsigned long long *)&c.led_g[row * MAXMAT + mat], (unsigned long long)(long long)v);
 }
 __device__ __forceinline__ void led_add64(Ctx &c, int row, uint32_t w, long long v) {
-    if (v > -1024 && v < 1024)
+    if (v > -LED_SMALL && v < LED_SMALL)
         led_add(c, row, w, (int32_t)v);
     else if (!cw_air(w))
         atomicAdd((unsigned long long *)&c.led_g[row * MAXMAT + cw_id(w)], (unsigned long long)v);
