@@ -165,20 +165,15 @@ __device__ __forceinline__ void load_types(uint8_t *s_type, const MatTable *mt) 
 
 __device__ __forceinline__ int32_t fill_code(int i) { return 0x7fffffff - i; }
 
-// the material particle i sees at cell c: the grid's, or the tile a particle of
-// lower index deposits there (fills are rewritten between iterations by other
-// blocks, so they are read past L1)
-// of a cell with grid material id and fill record v
+// the material particle i sees at a cell of grid material `id` and fill record v: the
+// grid's, or the tile a particle of lower index deposits there (fills are rewritten
+// between iterations by other blocks, so the records are read past L1)
 __device__ __forceinline__ int view_of(const WorldDev &w, const uint8_t *s_type, int id, int32_t v, int i) {
     if (s_type[id] == T_AIR && v != 0) {
         const int j = 0x7fffffff - v;
         if (j < i) id = w.p.id[j];
     }
     return id;
-}
-__device__ __forceinline__ int view_id(const WorldDev &w, const uint8_t *s_type, int c, int i) {
-    const int id = w.id[c];
-    return view_of(w, s_type, id, __ldcg(&w.df[c]), i);
 }
 
 // which 8x8 blocks hold AIR or liquid, from the grid the cell tick left (one thread per block);

@@ -102,7 +102,7 @@ __device__ __forceinline__ void divmod_small(int e, int n, float rn, int &q, int
 //
 // Ranks order the materials by density: AIR 0, SOLID 255 and the others by increasing
 // density from 1, equal densities equal ranks (MatTable::word, built on the host), so
-// that "AIR, or not SOLID and less dense" is one unsigned comparison (can_sink).
+// that "AIR, or not SOLID and less dense" is one unsigned comparison (cw_sink).
 constexpr uint32_t CW_ID = 0xFFu;
 constexpr uint32_t CW_FLAGS = 0xFF00u;  // the flags byte: MOVED, VISITED, settle count
 constexpr uint32_t CW_SETTLE = (uint32_t)SETTLE_MASK << 8;
@@ -510,11 +510,6 @@ __device__ __forceinline__ float clampflow_f(float flow, float rem) {
     if (flow < 0.0f) flow = 0.0f;
     const float lim = (rem < F_MAXFLOW) ? rem : F_MAXFLOW;
     return (flow > lim) ? lim : flow;
-}
-
-__device__ __forceinline__ bool can_sink(const uint32_t *ma, const float *md, int other, int self) {
-    int t = mt_type(ma[other]);
-    return t == T_AIR || (t != T_SOLID && md[other] < md[self]);
 }
 
 // the world of the CTA's current chunk
@@ -1671,7 +1666,7 @@ __global__ void __launch_bounds__(PAIR ? CP_THREADS / 2 : CP_THREADS, PAIR && CC
                         if (full) f[k] = w.fl[gb + gx];
                     }
                 }
-                if (full && !tma) {
+                if (full) {
 #pragma unroll
                     for (int k = 0; k < MAXRW / 32; k++) {
                         const int lx = lane + 32 * k, gx = Tl.x0 + lx;
