@@ -5,6 +5,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <atomic>
+#include <mutex>
+
 #include "../../include/fse.h"
 
 namespace fse {
@@ -260,5 +263,30 @@ __host__ __device__ __forceinline__ int32_t soup_scalar(const MatTable *mt, int 
 }
 
 __host__ __device__ __forceinline__ int ceil_div(int a, int b) { return (a + b - 1) / b; }
+
+// A kernel's dynamic shared memory beyond the 48 KB that need no opt-in. The attribute is a
+// device's own and stays until it is set again, so what it was set to is kept per device,
+// and only raised, under a lock: host threads may launch with different sizes at once.
+class SmemOptIn {
+    std::atomic<size_t> bytes[64] = {};
+    std::mutex mu;
+
+  public:
+    template <class K>
+    cudaError_t operator()(K *kernel, size_t want, int carveout = cudaSharedmemCarveoutDefault) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess) return e;
+        if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
+        if (bytes[dev].load(std::memory_order_acquire) >= want) return cudaSuccess;
+        std::lock_guard<std::mutex> lk(mu);
+        if (bytes[dev].load(std::memory_order_relaxed) >= want) return cudaSuccess;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)want);
+        if (e == cudaSuccess && carveout != cudaSharedmemCarveoutDefault)
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, carveout);
+        if (e == cudaSuccess) bytes[dev].store(want, std::memory_order_release);
+        return e;
+    }
+};
 
 }  // namespace fse

@@ -893,15 +893,13 @@ __global__ void __launch_bounds__(64, 1) k_lz4_decode(const uint8_t *__restrict_
 }
 
 // decode n_blocks blocks whose longest is max_len bytes
-void launch_decode(const uint8_t *src, const long long *offs, const int *lens, int n_blocks, int max_len, int expect,
+bool launch_decode(const uint8_t *src, const long long *offs, const int *lens, int n_blocks, int max_len, int expect,
                    uint8_t *out, int slot, int *status, cudaStream_t s) {
-    static bool attr = false;
-    if (!attr) {
-        cudaFuncSetAttribute(k_lz4_decode, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_FIXED + DEC_CAP_MAX);
-        attr = true;
-    }
+    static SmemOptIn opt_in;
+    if (opt_in(k_lz4_decode, DEC_FIXED + DEC_CAP_MAX) != cudaSuccess) return false;
     const int cap_in = std::max(DEC_WIN, std::min(DEC_CAP_MAX, (max_len + 15) & ~15));
     k_lz4_decode<<<n_blocks, 64, DEC_FIXED + cap_in, s>>>(src, offs, lens, n_blocks, expect, out, slot, status, cap_in);
+    return cudaGetLastError() == cudaSuccess;
 }
 
 // chunks whose records name a material outside the table: the lowest such chunk
@@ -1158,9 +1156,13 @@ int fse_world_unpack(fse_world *w, const uint8_t *in, const int64_t *offsets, in
             rc = FSE_E_CUDA;
             break;
         }
-        launch_decode(din, doff, dlen, g, *std::max_element(hl.begin(), hl.begin() + g), PK_SRC1, rec, PK_SRC1, dst, s);
-        launch_decode(din, doff + g, dlen + g, g, *std::max_element(hl.begin() + g, hl.end()), PK_SRC2, bgo, PK_SRC2,
-                      dst + g, s);
+        if (!launch_decode(din, doff, dlen, g, *std::max_element(hl.begin(), hl.begin() + g), PK_SRC1, rec, PK_SRC1, dst,
+                           s) ||
+            !launch_decode(din, doff + g, dlen + g, g, *std::max_element(hl.begin() + g, hl.end()), PK_SRC2, bgo,
+                           PK_SRC2, dst + g, s)) {
+            rc = FSE_E_CUDA;
+            break;
+        }
         k_unpack_check<<<grid_for((long long)g * PK_CELLS, 256), 256, 0, s>>>(rec, PK_SRC1, g, nmat, dst + 2 * G);
         int first_bad_id = big;
         if (cudaMemcpyAsync(st.data(), dst, 2 * g * sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
@@ -1356,12 +1358,12 @@ int ck_read_section(const CkSection &sec, In &in, CkScratch &sc, cudaStream_t s)
             cudaMemcpyAsync(sc.dlen, len.data(), g * sizeof(int), cudaMemcpyHostToDevice, s) != cudaSuccess)
             return FSE_E_CUDA;
         uint8_t *dst = (uint8_t *)sec.dev + (int64_t)g0 * CK_BLOCK;
-        if (full)
-            launch_decode(sc.din, sc.doff, sc.dlen, full, *std::max_element(len.begin(), len.begin() + full), CK_BLOCK,
-                          dst, CK_BLOCK, sc.status, s);
-        if (tail)
-            launch_decode(sc.din, sc.doff + full, sc.dlen + full, 1, len[full], tail, dst + (size_t)full * CK_BLOCK,
-                          CK_BLOCK, sc.status + full, s);
+        if (full && !launch_decode(sc.din, sc.doff, sc.dlen, full, *std::max_element(len.begin(), len.begin() + full),
+                                   CK_BLOCK, dst, CK_BLOCK, sc.status, s))
+            return FSE_E_CUDA;
+        if (tail && !launch_decode(sc.din, sc.doff + full, sc.dlen + full, 1, len[full], tail,
+                                   dst + (size_t)full * CK_BLOCK, CK_BLOCK, sc.status + full, s))
+            return FSE_E_CUDA;
         count_launches((full ? 1 : 0) + (tail ? 1 : 0));
         if (cudaMemcpyAsync(st.data(), sc.status, g * sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
             cudaStreamSynchronize(s) != cudaSuccess)

@@ -1137,13 +1137,8 @@ cudaError_t launch_particle_tick(WorldDev *d_worlds, int n_worlds, const MatTabl
         const size_t dyn = (size_t)(3 * n_worlds + 2) * sizeof(int);
         // with the kernel's static arrays the table of the largest batches passes the 48 KB
         // that need no opt-in
-        static bool opted_in = false;
-        if (!opted_in) {
-            const cudaError_t e = cudaFuncSetAttribute(k_part_serial, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                       (int)((3 * SERIAL_MAX_WORLDS + 2) * sizeof(int)));
-            if (e != cudaSuccess) return e;
-            opted_in = true;
-        }
+        static SmemOptIn opt_in;
+        if (const cudaError_t e = opt_in(k_part_serial, (3 * SERIAL_MAX_WORLDS + 2) * sizeof(int))) return e;
         static int nsm = 0;
         if (!nsm) {
             int dev = 0;

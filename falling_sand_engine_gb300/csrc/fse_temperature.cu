@@ -322,13 +322,8 @@ int temperature_tiles(int W, int H) { return tiles_x(W) * tiles_y(H); }
 cudaError_t launch_temperature(const WorldDev *d_worlds, int n_worlds, int max_tiles, const MatTable *mt, bool gated,
                                cudaStream_t s) {
     if (n_worlds <= 0 || max_tiles <= 0) return cudaSuccess;
-    static bool attr = false;
-    if (!attr) {
-        cudaError_t e =
-            cudaFuncSetAttribute(k_temp_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(TempSmem));
-        if (e != cudaSuccess) return e;
-        attr = true;
-    }
+    static SmemOptIn opt_in;
+    if (const cudaError_t e = opt_in(k_temp_tiles, sizeof(TempSmem))) return e;
     // 4 CTAs of 256 threads fit an SM (about 56 KB of shared memory each)
     const int gx = std::max(1, std::min(max_tiles, sm_count() * 4));
     k_temp_tiles<<<dim3(gx, n_worlds), TT_THREADS, sizeof(TempSmem), s>>>(d_worlds, mt, gated ? 1 : 0);

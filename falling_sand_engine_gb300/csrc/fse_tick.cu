@@ -2192,15 +2192,10 @@ size_t colour_pass_smem(int C, int halo) {
 template <int HALO, bool TEMP, bool SEQ = false, bool F32 = false, int CC = 0>
 static cudaError_t launch_cc(const WorldDev *worlds, const uint32_t *items, int n_items, int iter, int tk,
                             const MatTable *mt, size_t sm, int grid, cudaStream_t s) {
-    // opt in to the full shared-memory carve-out once per instantiation
-    static size_t set = 0;
-    if (set < sm) {
-        cudaFuncSetAttribute(k_colour_pass<HALO, TEMP, SEQ, F32, false, false, CC>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)sm);
-        set = sm;
-    }
-    k_colour_pass<HALO, TEMP, SEQ, F32, false, false, CC><<<grid, CP_THREADS, sm, s>>>(worlds, items, n_items, iter, tk, mt,
-                                                                     FusedTick{});
+    auto *kernel = k_colour_pass<HALO, TEMP, SEQ, F32, false, false, CC>;
+    static SmemOptIn opt_in;
+    if (const cudaError_t e = opt_in(kernel, sm)) return e;
+    kernel<<<grid, CP_THREADS, sm, s>>>(worlds, items, n_items, iter, tk, mt, FusedTick{});
     return cudaGetLastError();
 }
 
@@ -2218,13 +2213,10 @@ static cudaError_t launch_t(const WorldDev *worlds, const uint32_t *items, int n
 template <int HALO, bool TEMP, bool F32, int CC>
 static cudaError_t launch_fused_cc(const WorldDev *worlds, const FusedTick &ft, const MatTable *mt, size_t sm,
                                   int grid, cudaStream_t s) {
-    static size_t set = 0;
-    if (set < sm) {
-        cudaFuncSetAttribute(k_colour_pass<HALO, TEMP, false, F32, false, true, CC>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        set = sm;
-    }
-    k_colour_pass<HALO, TEMP, false, F32, false, true, CC><<<grid, CP_THREADS, sm, s>>>(worlds, nullptr, 0, 0, 0, mt, ft);
+    auto *kernel = k_colour_pass<HALO, TEMP, false, F32, false, true, CC>;
+    static SmemOptIn opt_in;
+    if (const cudaError_t e = opt_in(kernel, sm)) return e;
+    kernel<<<grid, CP_THREADS, sm, s>>>(worlds, nullptr, 0, 0, 0, mt, ft);
     return cudaGetLastError();
 }
 
@@ -2244,16 +2236,11 @@ static size_t colour_pass_smem_pair(int C, int halo) { return tile_smem<CP_THREA
 template <int HALO, bool TEMP, bool F32, int CC>
 static cudaError_t launch_pair_cc(const WorldDev *worlds, const uint32_t *items, int n_items, int iter, int tk,
                                   const MatTable *mt, size_t sm, int clusters, cudaStream_t s) {
-    static size_t set = 0;
-    if (set < sm) {
-        cudaFuncSetAttribute(k_colour_pass<HALO, TEMP, false, F32, true, false, CC>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sm);
-        // all of the unified L1/shared storage as shared memory, so that two CTAs share an SM
-        // where they fit
-        cudaFuncSetAttribute(k_colour_pass<HALO, TEMP, false, F32, true, false, CC>,
-                             cudaFuncAttributePreferredSharedMemoryCarveout, 100);
-        set = sm;
-    }
+    auto *kernel = k_colour_pass<HALO, TEMP, false, F32, true, false, CC>;
+    // all of the unified L1/shared storage as shared memory, so that two CTAs share an SM
+    // where they fit
+    static SmemOptIn opt_in;
+    if (const cudaError_t e = opt_in(kernel, sm, cudaSharedmemCarveoutMaxShared)) return e;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(2 * clusters);
     cfg.blockDim = dim3(CP_THREADS / 2);
@@ -2266,8 +2253,7 @@ static cudaError_t launch_pair_cc(const WorldDev *worlds, const uint32_t *items,
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    return cudaLaunchKernelEx(&cfg, k_colour_pass<HALO, TEMP, false, F32, true, false, CC>, worlds, items, n_items, iter,
-                              tk, mt, FusedTick{});
+    return cudaLaunchKernelEx(&cfg, kernel, worlds, items, n_items, iter, tk, mt, FusedTick{});
 }
 
 template <int HALO, bool TEMP, bool F32>
