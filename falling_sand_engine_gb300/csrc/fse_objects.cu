@@ -159,7 +159,9 @@ __global__ void __launch_bounds__(256) k_obj_held(const WorldDev *__restrict__ w
     }
 }
 
-// blocks of the two kernels below: contiguous ranges of tiles in order
+// blocks of the two kernels below: contiguous ranges of tiles in order; two a SM, as many as
+// the scan of their counts by one block allows for many times over (a stamp and readback of
+// 2 million tiles took 0.71 ms with 152, 304 and 608 blocks, of 12 million 4.1, 3.9 and 3.8)
 constexpr int OBJ_BLOCKS = 304;
 __device__ __forceinline__ void obj_range(uint32_t total, uint32_t *b0, uint32_t *b1) {
     const uint32_t seg = (total + gridDim.x - 1) / gridDim.x;
