@@ -837,7 +837,7 @@ static void free_world(fse_world *w) {
     WorldDev &h = w->h;
     void *ptrs[] = {h.id, h.col, h.sc, h.fl, h.df, h.tp, h.tnew, h.stage, h.cp_count, h.cp_base, h.p_state, h.p_box0,
                     h.p_box1, h.p_cell, h.p_prev, h.chg, h.scan_tmp, h.ledger, h.airmap, w->ctr, w->d, w->claim,
-                    w->mask_bits, w->obj_list, w->obj_n, w->rec, h.merge_list, h.merge_count, h.merge_claim, h.cdone};
+                    w->mask_bits, w->obj_list, w->obj_n, h.merge_list, h.merge_count, h.merge_claim, h.cdone};
     for (void *q : ptrs)
         if (q) cudaFree(q);
     PartSoA *ps[2] = {&h.p, &h.q};
@@ -1010,14 +1010,14 @@ int fse_world_create(int width, int height, const fse_config *cfg, fse_world **o
     int ncp = h.cell_iter * 4 * h.max_slots * h.cp_rows + 1;
     bool ok = dalloc(w, &h.id, n) && dalloc(w, &h.col, n) && dalloc(w, &h.sc, n) && dalloc(w, &h.fl, n) &&
               dalloc(w, &h.df, n) && dalloc(w, &h.stage, (size_t)h.stage_cap) && dalloc(w, &h.cp_count, ncp) &&
-              dalloc(w, &h.cp_base, ncp) && dalloc(w, &w->ctr, 24) && dalloc(w, &h.ledger, LED_ROWS * MAXMAT) &&
+              dalloc(w, &h.cp_base, ncp) && dalloc(w, &w->ctr, CTR_WORDS + REC_OWN * sizeof(fse_particle) / 4) &&
+              dalloc(w, &h.ledger, LED_ROWS * MAXMAT) &&
               dalloc(w, &h.p_state, (size_t)h.part_cap) && dalloc(w, &h.p_box0, (size_t)h.part_cap) &&
               dalloc(w, &h.p_box1, (size_t)h.part_cap) && dalloc(w, &h.p_cell, (size_t)h.part_cap) &&
               dalloc(w, &h.p_prev, (size_t)h.part_cap) && dalloc(w, &h.scan_tmp, particle_scan_blocks() + 1) &&
               dalloc(w, &h.airmap, (size_t)h.amw * h.amh) && dalloc(w, &h.chg, 2 * (size_t)h.amw * h.amh) &&
               dalloc(w, &h.merge_list, 2 * (size_t)h.part_cap) && dalloc(w, &h.merge_count, 1) &&
-              dalloc(w, &h.cdone, (size_t)h.nCx * h.nCy) && dalloc(w, &w->d, 1) &&
-              dalloc(w, &w->rec, REC_OWN * sizeof(fse_particle) / 4);
+              dalloc(w, &h.cdone, (size_t)h.nCx * h.nCy) && dalloc(w, &w->d, 1);
     PartSoA *ps[2] = {&h.p, &h.q};
     size_t pc = (size_t)h.part_cap;
     for (int k = 0; k < 2 && ok; k++) {
@@ -1059,6 +1059,7 @@ int fse_world_create(int width, int height, const fse_config *cfg, fse_world **o
         free_world(w);
         return FSE_E_NOMEM;
     }
+    w->rec = (uint32_t *)(w->ctr + CTR_WORDS);
     h.stage_count = w->ctr + 0;
     h.part_count = w->ctr + 1;
     h.req_count = w->ctr + 2;  // [3]

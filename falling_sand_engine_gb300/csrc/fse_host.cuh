@@ -53,7 +53,8 @@ struct fse_world {
     uint32_t *obj_list;   // object list scratch
     size_t obj_list_cap;
     int64_t *obj_n;       // object list count
-    uint32_t *rec;        // REC_OWN particle records of fse_particles_read, where no more are to be had
+    // after the counters, REC_OWN particle records for fse_particles_read where no more are to be had
+    uint32_t *rec;
     std::mutex rec_mu;    // held while rec is in use
     std::map<int, cudaGraphExec_t> graphs;  // n_ticks -> step graph
     std::map<int, long long> graph_kernels;  // n_ticks -> kernels one replay launches
@@ -139,6 +140,7 @@ struct CallScratch {
 };
 void scratch_trim();  // frees the idle blocks
 constexpr int REC_OWN = 2048;  // particle records that every world has room for
+constexpr int CTR_WORDS = 64;  // the counters before them (24 in use; the records start 256 bytes on)
 
 // one world::tick() + optionally world::tickCells() for a set of worlds that
 // share a device descriptor table
