@@ -611,9 +611,9 @@ __global__ void __launch_bounds__(SERIAL_THREADS) k_part_serial(const WorldDev *
     // 512, 1024 or 4096 particles measured the same.
     // Every iteration also clears the marks of the worlds that changed, whatever their
     // population, so large worlds take more blocks: with the blocks of the population alone
-    // the update of 100 particles in 8192 x 8192 cells took 0.36 ms, 0.21 with all blocks and
-    // 0.16 with these; 900 particles in 1920 x 1080 cells 0.24, 0.31 and 0.18 (0.20 with
-    // 8,192 marks a block, 0.23 with 16,384).
+    // the update of 100 particles in 8192 x 8192 cells took 0.36 ms, and takes 0.16 so (0.21 in
+    // a build that used all blocks and a slower block map); 900 particles in 1920 x 1080 cells
+    // 0.24 and 0.18 (0.20 with 8,192 marks a block, 0.23 with 16,384; 0.31 in that build).
     const unsigned by_parts = total <= ONE_BLOCK_PARTICLES ? 1u : (unsigned)(total + BLOCK_PARTICLES - 1) / BLOCK_PARTICLES;
     const unsigned nb = min(gridDim.x, max(by_parts, (unsigned)s_marks / BLOCK_MARKS));
     if (blockIdx.x >= nb) return;
