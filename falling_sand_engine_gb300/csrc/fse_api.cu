@@ -318,7 +318,7 @@ int ensure_materials_pushed() {
     if (!g_dirty && g_dev_mt) return FSE_OK;
     build_table(g_host_mt);
     if (!g_dev_mt) {
-        if (cudaMalloc(&g_dev_mt, sizeof(MatTable)) != cudaSuccess) {
+        if (device_alloc(&g_dev_mt, sizeof(MatTable)) != cudaSuccess) {
             g_dev_mt = nullptr;
             return FSE_E_NOMEM;
         }
@@ -412,6 +412,7 @@ bool CallScratch::take(size_t want) {
         }
         cudaGetLastError();  // no memory: nothing is wrong with the device
         p = nullptr;
+        size = want;
         free_idle(*ib, 0);
     }
     return false;
@@ -430,11 +431,21 @@ CallScratch::~CallScratch() {
     ib.list.emplace_back(size, p);
     ib.bytes += size;
 }
-void scratch_trim() {
-    if (IdleBlocks *ib = idle_blocks()) {
-        std::lock_guard<std::mutex> lk(ib->mu);
-        free_idle(*ib, 0);
+bool scratch_trim() {
+    IdleBlocks *ib = idle_blocks();
+    if (!ib) return false;
+    std::lock_guard<std::mutex> lk(ib->mu);
+    const bool any = ib->bytes > 0;
+    free_idle(*ib, 0);
+    return any;
+}
+cudaError_t device_alloc(void **p, size_t bytes) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e == cudaErrorMemoryAllocation && scratch_trim()) {
+        cudaGetLastError();
+        e = cudaMalloc(p, bytes);
     }
+    return e;
 }
 
 static std::atomic<long long> g_launches{0};
@@ -908,7 +919,7 @@ static bool world_tensor_maps(fse_world *w) {
                 strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                 CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
             return true;  // not encodable: cp.async staging
-    if (cudaMalloc(&w->tmaps, sizeof(maps)) != cudaSuccess) {
+    if (device_alloc(&w->tmaps, sizeof(maps)) != cudaSuccess) {
         cudaGetLastError();
         w->tmaps = nullptr;
         return false;
@@ -939,7 +950,7 @@ template <class T>
 static bool dalloc(fse_world *w, T **p, size_t n) {
     size_t b = n * sizeof(T);
     if (b == 0) b = sizeof(T);
-    if (cudaMalloc((void **)p, b) != cudaSuccess) {
+    if (device_alloc((void **)p, b) != cudaSuccess) {
         *p = nullptr;
         cudaGetLastError();
         return false;
@@ -1675,7 +1686,7 @@ int fse_world_census(fse_world *w, int64_t *out) {
     int rc = ensure_materials_pushed();
     if (rc) return rc;
     long long *d = nullptr;
-    FSE_CUDA_TRY(cudaMalloc(&d, 4 * MAXMAT * 8));
+    FSE_CUDA_TRY(device_alloc(&d, 4 * MAXMAT * 8));
     cudaMemsetAsync(d, 0, 4 * MAXMAT * 8, w->stream);
     k_census<<<sm_count() * 2, 512, 0, w->stream>>>(w->d, g_dev_mt, d);
     std::vector<long long> buf(4 * MAXMAT);

@@ -69,13 +69,13 @@ int build_tables(const std::vector<fse_world *> &ws, WorldDev **d_table, uint32_
         }
     }
     if (*d_table) cudaFree(*d_table);
-    if (cudaMalloc(d_table, std::max<size_t>(tab.size(), 1) * sizeof(WorldDev)) != cudaSuccess) return FSE_E_NOMEM;
+    if (device_alloc(d_table, std::max<size_t>(tab.size(), 1) * sizeof(WorldDev)) != cudaSuccess) return FSE_E_NOMEM;
     cudaMemcpyAsync(*d_table, tab.data(), tab.size() * sizeof(WorldDev), cudaMemcpyHostToDevice, s);
     for (int tk = 0; tk < 4; tk++) {
         if (items[tk]) cudaFree(items[tk]);
         items[tk] = nullptr;
         n_items[tk] = (int)it[tk].size();
-        if (cudaMalloc(&items[tk], std::max<size_t>(it[tk].size(), 1) * 4) != cudaSuccess) return FSE_E_NOMEM;
+        if (device_alloc(&items[tk], std::max<size_t>(it[tk].size(), 1) * 4) != cudaSuccess) return FSE_E_NOMEM;
         if (!it[tk].empty()) cudaMemcpyAsync(items[tk], it[tk].data(), it[tk].size() * 4, cudaMemcpyHostToDevice, s);
     }
     if (cudaStreamSynchronize(s) != cudaSuccess) return FSE_E_CUDA;
@@ -207,8 +207,8 @@ int batch_io_prepare(fse_batch *b) {
             at += (nb + 15) & ~(int64_t)15;
         }
     }
-    if (cudaMalloc(&b->io_stage, (size_t)std::max<int64_t>(total, 16)) != cudaSuccess ||
-        cudaMalloc(&b->io_segs, segs.size() * sizeof(IoSeg)) != cudaSuccess) {
+    if (device_alloc(&b->io_stage, (size_t)std::max<int64_t>(total, 16)) != cudaSuccess ||
+        device_alloc(&b->io_segs, segs.size() * sizeof(IoSeg)) != cudaSuccess) {
         cudaGetLastError();
         return FSE_E_NOMEM;
     }
@@ -284,7 +284,7 @@ bool snap_take(fse_world *w, Snapshot &s, cudaStream_t st) {
     for (auto &e : list) {
         if (!e.first) continue;  // planes the world does not keep
         void *d = nullptr;
-        if (cudaMalloc(&d, e.second) != cudaSuccess) return false;
+        if (device_alloc(&d, e.second) != cudaSuccess) return false;
         cudaMemcpyAsync(d, e.first, e.second, cudaMemcpyDeviceToDevice, st);
         s.bufs.push_back(d);
         s.src.push_back(e);

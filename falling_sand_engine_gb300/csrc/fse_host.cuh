@@ -138,7 +138,13 @@ struct CallScratch {
     void *from = nullptr;
     cudaStream_t s;
 };
-void scratch_trim();  // frees the idle blocks
+bool scratch_trim();  // frees the idle blocks; whether there were any
+// cudaMalloc, which the idle blocks make way for
+cudaError_t device_alloc(void **p, size_t bytes);
+template <class T>
+cudaError_t device_alloc(T **p, size_t bytes) {
+    return device_alloc((void **)p, bytes);
+}
 constexpr int REC_OWN = 2048;  // particle records that every world has room for
 constexpr int CTR_WORDS = 64;  // the counters before them (24 in use; the records start 256 bytes on)
 

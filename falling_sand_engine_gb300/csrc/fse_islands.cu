@@ -319,7 +319,7 @@ using namespace fse;
 template <typename T>
 static bool grow(fse_world *w, T **p, size_t n) {
     if (*p) return true;
-    if (cudaMalloc((void **)p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) {
+    if (device_alloc((void **)p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) {
         *p = nullptr;
         cudaGetLastError();
         return false;

@@ -383,7 +383,7 @@ using namespace fse;
 static int obj_prepare(fse_world *w) {
     size_t n = (size_t)w->W * w->H;
     if (!w->claim) {
-        if (cudaMalloc(&w->claim, n * 4) != cudaSuccess) {
+        if (device_alloc(&w->claim, n * 4) != cudaSuccess) {
             w->claim = nullptr;
             return FSE_E_NOMEM;
         }
@@ -464,7 +464,7 @@ static int obj_mask_dev(fse_world *w) {
     size_t n = (size_t)w->W * w->H;
     size_t nwords = (n + 31) / 32;
     if (!w->mask_bits) {
-        if (cudaMalloc(&w->mask_bits, nwords * 4) != cudaSuccess) {
+        if (device_alloc(&w->mask_bits, nwords * 4) != cudaSuccess) {
             w->mask_bits = nullptr;
             return FSE_E_NOMEM;
         }
@@ -494,13 +494,13 @@ int fse_object_list_export(fse_world *w, uint32_t *host_idx, int64_t cap, int64_
     size_t n = (size_t)w->W * w->H, nwords = (n + 31) / 32;
     const int NB = 256;
     if (!w->obj_n) {
-        if (cudaMalloc(&w->obj_n, 8 + (NB + 1) * 4) != cudaSuccess) return FSE_E_NOMEM;
+        if (device_alloc(&w->obj_n, 8 + (NB + 1) * 4) != cudaSuccess) return FSE_E_NOMEM;
     }
     int32_t *blk = (int32_t *)((char *)w->obj_n + 8);
     long long cap_dev = std::max<long long>(cap, 1);
     if (!w->obj_list || w->obj_list_cap < (size_t)cap_dev) {
         if (w->obj_list) cudaFree(w->obj_list);
-        if (cudaMalloc(&w->obj_list, (size_t)cap_dev * 4) != cudaSuccess) {
+        if (device_alloc(&w->obj_list, (size_t)cap_dev * 4) != cudaSuccess) {
             w->obj_list = nullptr;
             w->obj_list_cap = 0;
             return FSE_E_NOMEM;

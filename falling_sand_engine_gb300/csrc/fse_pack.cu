@@ -986,7 +986,7 @@ bool scratch(fse_world *w, int k, T **p, size_t bytes) {
         if (w->pk_scr[k]) cudaFree(w->pk_scr[k]);
         w->pk_scr[k] = nullptr;
         w->pk_scr_bytes[k] = 0;
-        if (cudaMalloc(&w->pk_scr[k], bytes) != cudaSuccess) {
+        if (device_alloc(&w->pk_scr[k], bytes) != cudaSuccess) {
             w->pk_scr[k] = nullptr;
             *p = nullptr;
             return false;
@@ -1241,17 +1241,17 @@ struct CkScratch {
     int *dlen = nullptr;
     bool ok() const { return stage && enc && sizes && anc && sout && status && info && rec && din && doff && dlen; }
     void alloc() {
-        cudaMalloc(&stage, (size_t)CK_GROUP * CK_BLOCK + 16);  // + a zeroed word after the data
-        cudaMalloc(&enc, (size_t)CK_GROUP * CK_SLOT);
-        cudaMalloc(&sizes, (CK_GROUP + 1) * sizeof(int));
-        cudaMalloc(&anc, (size_t)CK_GROUP * CK_SEGS * sizeof(int));
-        cudaMalloc(&sout, (size_t)CK_GROUP * CK_SEGS * sizeof(int));
-        cudaMalloc(&status, (CK_GROUP + 1) * sizeof(int));
-        cudaMalloc(&info, (size_t)CK_GROUP * CK_SEGS * sizeof(SegInfo));
-        cudaMalloc(&rec, (size_t)CK_GROUP * CK_SEGS * ENC_REC * sizeof(uint2));
-        cudaMalloc(&din, (size_t)CK_GROUP * CK_SLOT);
-        cudaMalloc(&doff, (CK_GROUP + 1) * sizeof(long long));
-        cudaMalloc(&dlen, (CK_GROUP + 1) * sizeof(int));
+        device_alloc(&stage, (size_t)CK_GROUP * CK_BLOCK + 16);  // + a zeroed word after the data
+        device_alloc(&enc, (size_t)CK_GROUP * CK_SLOT);
+        device_alloc(&sizes, (CK_GROUP + 1) * sizeof(int));
+        device_alloc(&anc, (size_t)CK_GROUP * CK_SEGS * sizeof(int));
+        device_alloc(&sout, (size_t)CK_GROUP * CK_SEGS * sizeof(int));
+        device_alloc(&status, (CK_GROUP + 1) * sizeof(int));
+        device_alloc(&info, (size_t)CK_GROUP * CK_SEGS * sizeof(SegInfo));
+        device_alloc(&rec, (size_t)CK_GROUP * CK_SEGS * ENC_REC * sizeof(uint2));
+        device_alloc(&din, (size_t)CK_GROUP * CK_SLOT);
+        device_alloc(&doff, (CK_GROUP + 1) * sizeof(long long));
+        device_alloc(&dlen, (CK_GROUP + 1) * sizeof(int));
     }
     void release() {
         void *ps[] = {stage, enc, sizes, anc, sout, status, info, rec, din, doff, dlen};

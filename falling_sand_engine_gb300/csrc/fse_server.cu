@@ -280,7 +280,7 @@ int upload_tables(fse_server *s, const std::vector<int> &want) {
         if (s->arena) cudaFree(s->arena);
         s->arena = nullptr;
         s->arena_cap = 0;
-        if (cudaMalloc(&s->arena, cap) != cudaSuccess) {
+        if (device_alloc(&s->arena, cap) != cudaSuccess) {
             cudaGetLastError();
             return FSE_E_NOMEM;
         }

@@ -342,7 +342,7 @@ int ensure_temperature_scratch(fse_world *w) {
     if (w->h.tnew) return FSE_OK;
     int32_t *p = nullptr;
     const size_t n = temperature_scratch_cells(w->W, w->H);
-    if (cudaMalloc(&p, n * sizeof(int32_t)) != cudaSuccess) return FSE_E_NOMEM;
+    if (device_alloc(&p, n * sizeof(int32_t)) != cudaSuccess) return FSE_E_NOMEM;
     w->h.tnew = p;
     w->bytes += n * sizeof(int32_t);
     if (cudaMemcpyAsync(w->d, &w->h, sizeof(WorldDev), cudaMemcpyHostToDevice, w->stream) != cudaSuccess)
@@ -351,7 +351,7 @@ int ensure_temperature_scratch(fse_world *w) {
 }
 int ensure_temperature_io(fse_world *w) {
     if (w->temp_io) return FSE_OK;
-    if (cudaMalloc(&w->temp_io, (size_t)w->W * w->H * sizeof(int16_t)) != cudaSuccess) {
+    if (device_alloc(&w->temp_io, (size_t)w->W * w->H * sizeof(int16_t)) != cudaSuccess) {
         w->temp_io = nullptr;
         return FSE_E_NOMEM;
     }

@@ -103,7 +103,7 @@ int ensure_tile_stage(fse_world *w, size_t bytes) {
     if (w->tile_stage) cudaFree(w->tile_stage);
     w->tile_stage = nullptr;
     w->tile_stage_bytes = 0;
-    if (cudaMalloc(&w->tile_stage, bytes) != cudaSuccess) {
+    if (device_alloc(&w->tile_stage, bytes) != cudaSuccess) {
         w->tile_stage = nullptr;
         return FSE_E_NOMEM;
     }
